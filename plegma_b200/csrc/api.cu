@@ -409,6 +409,81 @@ p2_status make_plan(p2_ctx* c, const p2_request& r, Plan& pl) {
   return P2_OK;
 }
 
+// Direct FP64 phase sum of a chunk's position buffer and the deterministic
+// reduction, for momentum lists with too many rows for the axis-by-axis sums.
+p2_status project_direct(p2_ctx* c, const Plan& pl, int K, int n, int max_n, const p2::SliceDesc* dsl,
+                         const std::vector<p2::ScatterBlock>& blocks) {
+  const int ptiles = (pl.nmom + 63) / 64;
+  p2::ProjArgs pa{};
+  pa.c = c->cbuf.p;
+  pa.sT = (long long)K * c->V3;
+  pa.sK = c->V3;
+  pa.ntau = n;
+  pa.K = K;
+  pa.V3 = (int)c->V3;
+  pa.nmom = pl.nmom;
+  pa.Lx = c->Ll[0];
+  pa.Ly = c->Ll[1];
+  pa.Lz = c->Ll[2];
+  pa.Lmax = pl.Lmax;
+  pa.tab = (const double*)c->ptab.p;
+  // candidates (component tile, site splits): the least-waste tile at ~2
+  // waves first, then other tiles at 1, 2 and 4 waves
+  std::vector<std::vector<int>> cands;
+  const int tk0 = p2::project_fp64_tk(K, 0);
+  for (int tk : {tk0, 8, 6, 4, 2})
+    for (int waves : {2, 1, 4}) {
+      const int ktiles = (K + 16 * tk - 1) / (16 * tk);
+      int nsplit = (waves * c->nsm + ptiles * ktiles * n - 1) / (ptiles * ktiles * n);
+      nsplit = std::max(1, std::min(nsplit, (int)((c->V3 + 255) / 256)));
+      const int chunk = (int)((((c->V3 + nsplit - 1) / nsplit) + 15) / 16 * 16);
+      std::vector<int> v{tk, (int)((c->V3 + chunk - 1) / chunk), chunk};
+      if (std::find(cands.begin(), cands.end(), v) == cands.end()) cands.push_back(v);
+    }
+  int maxsplit = 0;
+  for (const auto& v : cands) maxsplit = std::max(maxsplit, v[1]);
+  P2_TRY(c, c->part.ensure((size_t)max_n * maxsplit * pl.nmom * K * 16), "partials alloc");
+  pa.part = (double*)c->part.p;
+  char key[160];
+  std::snprintf(key, sizeof(key), "project_fp64 V3=%lld K=%d nmom=%d n=%d", c->V3, K, pl.nmom, n);
+  std::vector<int> pick;
+  P2_TRY(c,
+         tune_choose(c->tuner.get(), key, cands, c->stream, !c->capturing,
+                     [&](const std::vector<int>& v) {
+                       p2::ProjArgs q = pa;
+                       q.tk = v[0];
+                       q.nsplit = v[1];
+                       q.chunk = v[2];
+                       return p2::launch_project_fp64(q, c->stream);
+                     },
+                     pick),
+         "projection tuning");
+  pa.tk = pick[0];
+  pa.nsplit = pick[1];
+  pa.chunk = pick[2];
+  {
+    ProfScope ps(c, "project_fp64");
+    P2_TRY(c, p2::launch_project_fp64(pa, c->stream), "projection kernel");
+  }
+  p2::ScatterArgs sa{};
+  sa.part = (const double*)c->part.p;
+  sa.ntau = n;
+  sa.nsplit = pa.nsplit;
+  sa.nmom = pl.nmom;
+  sa.K = K;
+  if (blocks.size() > (size_t)p2::kMaxBlocks) return c->fail(P2_ERR_INVALID_ARG, "too many result blocks");
+  sa.nblocks = (int)blocks.size();
+  for (size_t b = 0; b < blocks.size(); b++) sa.blk[b] = blocks[b];
+  sa.sl = dsl;
+  sa.moms = (const int*)c->moms.p;
+  for (int d = 0; d < 3; d++) sa.L[d] = c->g.L[d];
+  {
+    ProfScope ps(c, "reduce_scatter");
+    P2_TRY(c, p2::launch_scatter(sa, c->stream), "reduction kernel");
+  }
+  return P2_OK;
+}
+
 }  // namespace p2host
 
 namespace {
@@ -430,7 +505,9 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
   }
   const unsigned what = reqs[idx[0]].contractions;
   p2_status st;
-  if (c->plain_moms_key != pl.moms) {  // phase tables have origin 0: one set per momentum list
+  const AxesPlan* ap = nullptr;  // the axis-by-axis projection, when the list qualifies
+  if ((st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
+  if (!ap && c->plain_moms_key != pl.moms) {  // phase tables have origin 0: one set per momentum list
     c->plain_moms_key.clear();
     std::vector<double> tabh = phase_tables(c, pl.moms.data(), pl.nmom, -1, pl.Lmax);
     if ((st = upload_async(c, c->ptab, tabh.data(), tabh.size() * sizeof(double), "phase table")) != P2_OK) return st;
@@ -445,7 +522,6 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
   Stager sg(c, props, reqs, w);
   if ((st = sg.prepare(outs)) != P2_OK) return st;
 
-  const int ptiles = (pl.nmom + 63) / 64;
   for (int i = 0; i < 2; i++)
     if ((st = sg.issue(i)) != P2_OK) return st;
   for (size_t ci = 0; ci < w.chunks.size(); ci++) {
@@ -467,72 +543,16 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     if ((st = sg.release((int)ci)) != P2_OK) return st;
     if ((st = sg.issue((int)ci + 2)) != P2_OK) return st;
 
-    p2::ProjArgs pa{};
-    pa.c = c->cbuf.p;
-    pa.sT = (long long)pl.K * c->V3;
-    pa.sK = c->V3;
-    pa.ntau = n;
-    pa.K = pl.K;
-    pa.V3 = (int)c->V3;
-    pa.nmom = pl.nmom;
-    pa.Lx = c->Ll[0];
-    pa.Ly = c->Ll[1];
-    pa.Lz = c->Ll[2];
-    pa.Lmax = pl.Lmax;
-    pa.tab = (const double*)c->ptab.p;
-    // candidates (component tile, site splits): the least-waste tile at ~2
-    // waves first, then other tiles at 1, 2 and 4 waves
-    std::vector<std::vector<int>> cands;
-    const int tk0 = p2::project_fp64_tk(pl.K, 0);
-    for (int tk : {tk0, 8, 6, 4, 2})
-      for (int waves : {2, 1, 4}) {
-        const int ktiles = (pl.K + 16 * tk - 1) / (16 * tk);
-        int nsplit = (waves * c->nsm + ptiles * ktiles * n - 1) / (ptiles * ktiles * n);
-        nsplit = std::max(1, std::min(nsplit, (int)((c->V3 + 255) / 256)));
-        const int chunk = (int)((((c->V3 + nsplit - 1) / nsplit) + 15) / 16 * 16);
-        std::vector<int> v{tk, (int)((c->V3 + chunk - 1) / chunk), chunk};
-        if (std::find(cands.begin(), cands.end(), v) == cands.end()) cands.push_back(v);
-      }
-    int maxsplit = 0;
-    for (const auto& v : cands) maxsplit = std::max(maxsplit, v[1]);
-    P2_TRY(c, c->part.ensure((size_t)w.max_n * maxsplit * pl.nmom * pl.K * 16), "partials alloc");
-    pa.part = (double*)c->part.p;
-    char key[160];
-    std::snprintf(key, sizeof(key), "project_fp64 V3=%lld K=%d nmom=%d n=%d", c->V3, pl.K, pl.nmom, n);
-    std::vector<int> pick;
-    P2_TRY(c,
-           tune_choose(c->tuner.get(), key, cands, c->stream, !c->capturing,
-                       [&](const std::vector<int>& v) {
-                         p2::ProjArgs q = pa;
-                         q.tk = v[0];
-                         q.nsplit = v[1];
-                         q.chunk = v[2];
-                         return p2::launch_project_fp64(q, c->stream);
-                       },
-                       pick),
-           "projection tuning");
-    pa.tk = pick[0];
-    pa.nsplit = pick[1];
-    pa.chunk = pick[2];
-    {
-      ProfScope ps(c, "project_fp64");
-      P2_TRY(c, p2::launch_project_fp64(pa, c->stream), "projection kernel");
-    }
-    p2::ScatterArgs sa{};
-    sa.part = (const double*)c->part.p;
-    sa.ntau = n;
-    sa.nsplit = pa.nsplit;
-    sa.nmom = pl.nmom;
-    sa.K = pl.K;
-    if (pl.blocks.size() > (size_t)p2::kMaxBlocks) return c->fail(P2_ERR_INVALID_ARG, "too many result blocks");
-    sa.nblocks = (int)pl.blocks.size();
-    for (size_t b = 0; b < pl.blocks.size(); b++) sa.blk[b] = pl.blocks[b];
-    sa.sl = sg.desc((int)ci);
-    sa.moms = (const int*)c->moms.p;
-    for (int d = 0; d < 3; d++) sa.L[d] = c->g.L[d];
-    {
-      ProfScope ps(c, "reduce_scatter");
-      P2_TRY(c, p2::launch_scatter(sa, c->stream), "reduction kernel");
+    if (ap) {
+      P2_TRY(c, c->axes_s1.ensure((size_t)w.max_n * c->Ll[1] * c->Ll[2] * ap->R1 * pl.K * 16), "projection workspace");
+      if ((st = axes_x(c, *ap, c->cbuf.p, 0, (long long)pl.K * c->V3, c->V3, n, pl.K, c->axes_s1.p)) != P2_OK)
+        return st;
+      AxesOut ao;
+      ao.dsl = sg.desc((int)ci);
+      ao.blocks = &pl.blocks;
+      if ((st = axes_yz(c, *ap, c->axes_s1.p, 0, n, pl.K, ao)) != P2_OK) return st;
+    } else if ((st = project_direct(c, pl, pl.K, n, w.max_n, sg.desc((int)ci), pl.blocks)) != P2_OK) {
+      return st;
     }
     if (p2::g16_raw(what)) {
       // the Gamma sums of the 16 x 16 block on its projected colour products
@@ -550,6 +570,35 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
       ProfScope ps(c, "meson_gamma");
       P2_TRY(c, p2::launch_meson_gamma(mg, c->stream), "meson Gamma sums");
     }
+  }
+  return P2_OK;
+}
+
+// A field's transform axis by axis, in chunks of time slices that keep the
+// partial sums within the workspace budget.
+p2_status ft_axes(p2_ctx* c, const AxesPlan& ap, const double* field, int dof, int nt, double* out, int out_location) {
+  const size_t total = (size_t)nt * dof * ap.nmom;
+  double* dst = out;
+  if (out_location == P2_HOST) {
+    P2_TRY(c, c->res.ensure(total * 16), "result alloc");
+    dst = (double*)c->res.p;
+  }
+  const size_t s1 = (size_t)c->Ll[1] * c->Ll[2] * ap.R1 * dof * 16, per = s1 + (size_t)c->Ll[2] * ap.NP * dof * 16;
+  const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)nt));
+  P2_TRY(c, c->axes_s1.ensure((size_t)tc * s1), "projection workspace");
+  for (int t0 = 0; t0 < nt; t0 += tc) {
+    const int n = std::min(tc, nt - t0);
+    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, c->axes_s1.p);
+    if (st != P2_OK) return st;
+    AxesOut ao;
+    ao.oT = (long long)dof * ap.nmom;
+    ao.oK = ap.nmom;
+    ao.out = dst + 2 * (size_t)t0 * ao.oT;
+    if ((st = axes_yz(c, ap, c->axes_s1.p, 0, n, dof, ao)) != P2_OK) return st;
+  }
+  if (out_location == P2_HOST) {
+    P2_TRY(c, cudaMemcpyAsync(out, dst, total * 16, cudaMemcpyDeviceToHost, c->stream), "result download");
+    P2_TRY(c, cudaStreamSynchronize(c->stream), "result download");
   }
   return P2_OK;
 }
@@ -688,7 +737,9 @@ p2_status p2_ctx_destroy(p2_ctx* c) {
     return P2_OK;
   }
   cudaStreamSynchronize(c->stream);
-  for (DevBuf* b : {&c->cbuf, &c->part, &c->tab, &c->res, &c->moms, &c->sdesc, &c->ptab, &c->ft_kexp}) b->release();
+  for (DevBuf* b : {&c->cbuf, &c->part, &c->tab, &c->res, &c->moms, &c->sdesc, &c->ptab, &c->ft_kexp, &c->axes[0].tab,
+                    &c->axes[0].idx, &c->axes[1].tab, &c->axes[1].idx, &c->axes_s1, &c->axes_s2})
+    b->release();
   if (c->sdesc_host) cudaFreeHost(c->sdesc_host);
   if (c->sdesc_copied) cudaEventDestroy(c->sdesc_copied);
   for (int i = 0; i < 2; i++) {
@@ -1029,6 +1080,10 @@ p2_status p2_ft_apply(p2_ctx* c, const double* field, int dof, int nt, const int
     return c->fail(P2_ERR_INVALID_ARG, "p2_ft_apply: bad arguments");
   if (sign != 1 && sign != -1) return c->fail(P2_ERR_INVALID_ARG, "p2_ft_apply: sign must be +1 or -1");
   if (c->host_only) return c->fail(P2_ERR_UNSUPPORTED, "host-only context");
+  const AxesPlan* ap = nullptr;
+  p2_status st = axes_prepare(c, std::vector<int>(moms, moms + 3 * nmom), sign, &ap);
+  if (st != P2_OK) return st;
+  if (ap) return ft_axes(c, *ap, field, dof, nt, out, out_location);
   const int Lmax = std::max(c->Ll[0], std::max(c->Ll[1], c->Ll[2]));
   std::vector<double> tabh = phase_tables(c, moms, nmom, sign, Lmax);
   P2_TRY(c, c->tab.ensure(tabh.size() * sizeof(double)), "phase table alloc");

@@ -50,6 +50,16 @@ struct DevBuf {
   }
 };
 
+// Tables of the axis-by-axis projection for one momentum list and sign (project_axes.cu).
+struct AxesPlan {
+  std::vector<int> key;  // momentum list the tables were built for
+  bool usable = false;   // the list has few enough rows per axis
+  int R1 = 0, RY = 0, NP = 0, NO = 0, ny = 0, nmom = 0;
+  DevBuf tab, idx;
+  const double *xt = nullptr, *yt = nullptr, *zt = nullptr;
+  const int *first = nullptr, *ylist = nullptr, *orb = nullptr, *omom = nullptr;
+};
+
 struct BlockDef {
   unsigned bit;
   int groups, datasets, comps;
@@ -109,6 +119,9 @@ struct p2_ctx {
   p2host::DevBuf ptab;
   std::vector<int> plain_moms_key;
   p2_udsc_cache* udsc = nullptr;
+  // axis-by-axis projection: tables per transform sign (-1, +1), sums over x and over y
+  p2host::AxesPlan axes[2];
+  p2host::DevBuf axes_s1, axes_s2;
   // launch-shape autotuner (shared with the context's graphs)
   std::shared_ptr<p2host::Tuner> tuner = std::make_shared<p2host::Tuner>();
 
@@ -228,6 +241,23 @@ p2::CompOffsets offsets_of(unsigned what);
 std::vector<double> phase_tables(const p2_ctx* c, const int* moms, int nmom, int sign, int Lmax);
 p2_status make_plan(p2_ctx* c, const p2_request& r, Plan& pl);
 p2_status upload_async(p2_ctx* c, DevBuf& b, const void* src, size_t bytes, const char* what);
+
+// Axis-by-axis projection (project_axes.cu): *out is null when the list keeps the direct projections.
+struct AxesOut {
+  const p2::SliceDesc* dsl = nullptr;
+  const int* exps = nullptr;  // scale exponents per slice, or null
+  const int* kexp = nullptr;
+  const int* kphase = nullptr;
+  const std::vector<p2::ScatterBlock>* blocks = nullptr;  // result blocks of the slices, or null: out, oT, oK
+  double* out = nullptr;
+  long long oT = 0, oK = 0;
+};
+p2_status project_direct(p2_ctx* c, const Plan& pl, int K, int n, int max_n, const p2::SliceDesc* dsl,
+                         const std::vector<p2::ScatterBlock>& blocks);
+p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const AxesPlan** out);
+p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
+                 void* s1);
+p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o);
 
 }  // namespace p2host
 

@@ -187,6 +187,46 @@ cudaError_t launch_meson_gamma(const MesonGammaArgs& a, cudaStream_t s);
 int project_split_smem_bytes(int NT);
 int project_split_max_nt();  // widest N-tile (components) of the tensor-core projection
 
+// ---- projection one axis at a time (project_axes.cu) ------------------------
+constexpr int kAxisMaxRows = 9;  // cos / sin rows per axis
+
+struct AxisXArgs {
+  const void* c;      // complex double or complex float, element (tau, k, x) at c[tau*sT + k*sK + x]
+  long long sT, sK;
+  int ntau, K, rows, Lx, R1;
+  int KL;             // components a warp takes side by side (set by the launcher)
+  const double* xt;   // [Lx][R1] phase rows
+  void* s1;           // [ntau][rows][R1][K] complex, type of c
+};
+struct AxisYArgs {
+  const void* s1;
+  void* s2;           // [ntau][Lz][NP][K] complex double
+  int ntau, K, Ly, Lz, R1, RY, NP;
+  int ny;             // most pairs of one x row
+  const double* yt;   // [Ly][RY]
+  const int* first;   // [R1 + 1] first pair of each x row
+  const int* ylist;   // [NP] y row of each pair
+};
+struct AxisZArgs {
+  const void* s2;
+  int ntau, K, Lz, NP, NO, nmom;
+  const double* zt;   // [z row][Lz]
+  const int* orb;     // [NO][8], see k_axis_z
+  const int* omom;    // [nmom][8]
+  const SliceDesc* sl;
+  int L[3];
+  const int* exps;    // [ntau][2] scale exponents, or null
+  const int* kexp;    // [K][2]
+  const int* kphase;  // [K] or null
+  int nblocks;
+  ScatterBlock blk[kMaxBlocks];
+  long long oT, oK;
+  double* out;
+};
+cudaError_t launch_axis_x(const AxisXArgs& a, int fp32, cudaStream_t s);
+cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s);
+cudaError_t launch_axis_z(const AxisZArgs& a, cudaStream_t s);
+
 cudaError_t launch_contract_plain(const ContractArgs& a, int grid, cudaStream_t s);
 // FP32 site contraction; fp32_in selects complex-float propagators.
 cudaError_t launch_contract_f32(const ContractArgs& a, int fp32_in, int grid, cudaStream_t s);

@@ -1,0 +1,571 @@
+// Momentum projection one axis at a time.
+//
+// C(t, p, k) = sum_x c_k(x, t) exp(sign i p.(x - x0)) over a list of integer
+// momenta (the reference's fourier_transform_3D sums every site with every
+// momentum, lib/kernels/PLEGMA_kernel_utils.cuh:820-860).  The phase is a
+// product of three one-dimensional phases, and a list |n|^2 <= q2 holds few
+// distinct |n_x|, |n_y|, |n_z|, so the sum is taken over x first for each
+// distinct |n_x|, then over y for each distinct (|n_x|, |n_y|), then over z:
+//
+//   S1[t][row = (z, y)][r][k]   = sum_x X_r(x) c_k(x, y, z, t)
+//   S2[t][z][pair = (r, s)][k]  = sum_y Y_s(y) S1[t][z, y][r][k]
+//   C(t, p, k) from sum_z Z_q(z) S2[t][z][pair][k], q in {cos, sin}
+//
+// X_r, Y_s, Z_q are cos(2 pi a x / L) and sin(2 pi a x / L), one or two rows
+// per distinct a = min(n mod L, L - n mod L) (sin is absent for a = 0 and
+// a = L/2), so that the eight momenta (+-a, +-b, +-c) share all their sums
+// ("orbit"; the eight real-phase sums give them with signs and factors i).
+// For the 123 momenta of |n|^2 <= 9 a site and component costs 7 real x
+// complex products over x instead of 123 complex ones, and the later sums run
+// on 7 / Lx of the data.
+//
+// Measured on B200, FP64, against the direct sum of project_fp64.cu (which
+// larger lists keep): the plain form at 24^3 x 48 with 288 components and 123
+// momenta 4.17 ms instead of 14.12 ms (the projection was 10.8 ms of it), the
+// transform of a 32-component field there 0.14 ms instead of 2.18 ms.  Error
+// against 64 bits 1.7e-15 instead of 4.0e-15 (fewer terms per sum).
+//
+// Sums over x: FP64 for FP64 input, FP32 for FP32 input (sequential over one
+// row of Lx sites by one thread, so a row's sum does not depend on the launch
+// shape); sums over y and z: FP64, in a fixed order.
+#include <algorithm>
+#include <cmath>
+#include <cstdio>
+#include <vector>
+
+#include "ctx.h"
+#include "launch_util.h"
+#include "p2_common.cuh"
+
+namespace p2 {
+namespace {
+
+// ---- sums over x of a position buffer ------------------------------------------
+// A "line" is one row of Lx sites of one component; a warp takes 64 lines, two
+// per lane, and streams them in chunks of kBytes = 128 bytes per line through
+// its own shared memory with cp.async (two stages), so the global loads are
+// coalesced 128-byte segments and a lane's reads of its line are free of bank
+// conflicts (odd line stride).  Two lines per lane share each phase.  HBM
+// bound: the buffer is read once and R1 / Lx of it written.
+constexpr int kXWarps = 4;
+constexpr int kLines = 64;
+
+template <typename R>
+struct XChunk {
+  static constexpr int n = 128 / (2 * (int)sizeof(R));  // elements of a 128-byte chunk
+  static constexpr int stride = n + 1;
+  static constexpr int stage = kLines * stride;  // complex elements
+};
+
+template <typename R>
+__device__ __forceinline__ void cp_line(Cx<R>* dst, const Cx<R>* src, bool ok) {
+  if constexpr (sizeof(R) == 8)
+    cp_async16(dst, src, ok ? 16 : 0);
+  else
+    cp_async8(dst, src, ok ? 8 : 0);
+}
+
+template <typename R, int R1>
+__global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
+  using C = XChunk<R>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Cx<R>* st = (Cx<R>*)smem_raw + (threadIdx.x >> 5) * 2 * C::stage;
+  R* ph = (R*)((Cx<R>*)smem_raw + kXWarps * 2 * C::stage);  // [Lx][R1]
+  for (int i = threadIdx.x; i < a.Lx * R1; i += blockDim.x) ph[i] = (R)a.xt[i];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const long long item = (long long)blockIdx.x * kXWarps + (threadIdx.x >> 5);
+  const int kgroups = (a.K + a.KL - 1) / a.KL;
+  const int rows_per = kLines / a.KL;
+  const int rgroups = (a.rows + rows_per - 1) / rows_per;
+  if (item >= (long long)kgroups * rgroups * a.ntau) return;
+  // component groups vary slowest inside a slice, so that neighbouring warps read neighbouring rows
+  const int rg = (int)(item % rgroups), kg = (int)((item / rgroups) % kgroups);
+  const int tau = (int)(item / ((long long)rgroups * kgroups));
+  const int lg = __ffs(a.KL) - 1;
+  const Cx<R>* c = (const Cx<R>*)a.c + (long long)tau * a.sT;
+  const int nchunk = (a.Lx + C::n - 1) / C::n;
+
+  // this lane copies element e of the lines (lane / n) + 32 / n * i
+  constexpr int kPer = 32 / C::n;
+  const int e = lane % C::n, l0 = lane / C::n;
+  auto issue = [&](int ch) {
+    if (ch < nchunk) {
+      Cx<R>* d = st + (ch & 1) * C::stage;
+      const int x = ch * C::n + e;
+#pragma unroll 8
+      for (int i = 0; i < kLines / kPer; i++) {
+        const int ln = l0 + kPer * i;
+        const int k = kg * a.KL + (ln & (a.KL - 1)), row = rg * rows_per + (ln >> lg);
+        const bool ok = x < a.Lx && k < a.K && row < a.rows;
+        cp_line(d + ln * C::stride + e, ok ? c + (long long)k * a.sK + (long long)row * a.Lx + x : c, ok);
+      }
+    }
+    cp_async_commit();
+  };
+  Cx<R> acc[2][R1];
+#pragma unroll
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int r = 0; r < R1; r++) acc[j][r] = czero<R>();
+  issue(0);
+  for (int ch = 0; ch < nchunk; ch++) {
+    issue(ch + 1);
+    cp_async_wait<1>();
+    __syncwarp();
+    const Cx<R>* d = st + (ch & 1) * C::stage + lane * C::stride;
+    const R* p = ph + ch * C::n * R1;
+    const int n = min(C::n, a.Lx - ch * C::n);
+#pragma unroll 4
+    for (int x = 0; x < n; x++) {
+      const Cx<R> v0 = d[x], v1 = d[32 * C::stride + x];
+#pragma unroll
+      for (int r = 0; r < R1; r++) {
+        const R f = p[x * R1 + r];
+        acc[0][r].x = fma(f, v0.x, acc[0][r].x);
+        acc[0][r].y = fma(f, v0.y, acc[0][r].y);
+        acc[1][r].x = fma(f, v1.x, acc[1][r].x);
+        acc[1][r].y = fma(f, v1.y, acc[1][r].y);
+      }
+    }
+    __syncwarp();  // the chunk is read: the stage may be refilled
+  }
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int ln = lane + 32 * j;
+    const int k = kg * a.KL + (ln & (a.KL - 1)), row = rg * rows_per + (ln >> lg);
+    if (k < a.K && row < a.rows) {
+      Cx<R>* o = (Cx<R>*)a.s1 + (((long long)tau * a.rows + row) * R1) * a.K + k;
+#pragma unroll
+      for (int r = 0; r < R1; r++) o[(long long)r * a.K] = acc[j][r];
+    }
+  }
+}
+
+// ---- sums over y ----------------------------------------------------------------
+// Warp r of a block takes x row r of (slice, z) for 32 or 64 components (KPL
+// per lane): every value of S1 is read once and used for all the pairs of r.
+template <typename R, int NY, int KPL>
+__global__ void __launch_bounds__(32 * kAxisMaxRows) k_axis_y(const AxisYArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double* yt = (double*)smem_raw;  // [Ly][RY]
+  for (int i = threadIdx.x; i < a.Ly * a.RY; i += blockDim.x) yt[i] = a.yt[i];
+  __syncthreads();
+  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tau = blockIdx.z, z = blockIdx.y, k0 = blockIdx.x * 32 * KPL + lane;
+  const int first = a.first[r], cnt = a.first[r + 1] - first;
+  if (cnt == 0) return;  // a padding row
+  int ys[NY];
+#pragma unroll
+  for (int j = 0; j < NY; j++) ys[j] = a.ylist[first + min(j, cnt - 1)];
+  Cx<double> acc[NY][KPL];
+#pragma unroll
+  for (int j = 0; j < NY; j++)
+#pragma unroll
+    for (int q = 0; q < KPL; q++) acc[j][q] = czero<double>();
+  const long long rs = (long long)a.R1 * a.K;  // one row of S1
+  const Cx<R>* s = (const Cx<R>*)a.s1 + ((long long)tau * a.Lz + z) * a.Ly * rs + (long long)r * a.K;
+#pragma unroll 4
+  for (int y = 0; y < a.Ly; y++) {
+    Cx<R> v[KPL];
+#pragma unroll
+    for (int q = 0; q < KPL; q++) v[q] = k0 + 32 * q < a.K ? s[y * rs + k0 + 32 * q] : czero<R>();
+#pragma unroll
+    for (int j = 0; j < NY; j++) {
+      const double f = yt[y * a.RY + ys[j]];
+#pragma unroll
+      for (int q = 0; q < KPL; q++) {
+        acc[j][q].x = fma(f, (double)v[q].x, acc[j][q].x);
+        acc[j][q].y = fma(f, (double)v[q].y, acc[j][q].y);
+      }
+    }
+  }
+  Cx<double>* o = (Cx<double>*)a.s2 + (((long long)tau * a.Lz + z) * a.NP + first) * a.K;
+#pragma unroll
+  for (int j = 0; j < NY; j++)
+#pragma unroll
+    for (int q = 0; q < KPL; q++)
+      if (j < cnt && k0 + 32 * q < a.K) o[(long long)j * a.K + k0 + 32 * q] = acc[j][q];
+}
+
+// ---- sums over z and the results --------------------------------------------------
+// One block per (orbit, slice, 128 components): the eight real-phase sums of
+// an orbit, its up to eight momenta, the un-scaling, the source phase and the
+// result layout.
+__global__ void __launch_bounds__(128) k_axis_z(const AxisZArgs a) {
+  const int ob = blockIdx.x, tl = blockIdx.y, k = blockIdx.z * 128 + threadIdx.x;
+  if (k >= a.K) return;
+  const int* od = a.orb + 8 * ob;  // pairs (cos cos, cos sin, sin cos, sin sin) of (x, y), z rows (cos, sin), momenta [m0, m1)
+  int pr[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) pr[i] = od[i];
+  const int zc = od[4], zs = od[5], m0 = od[6], m1 = od[7];
+  Cx<double> A[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; i++) A[i][0] = A[i][1] = czero<double>();
+  const Cx<double>* s = (const Cx<double>*)a.s2 + (long long)tl * a.Lz * a.NP * a.K + k;
+  const long long zstep = (long long)a.NP * a.K;
+#pragma unroll 2
+  for (int z = 0; z < a.Lz; z++) {
+    const double fc = zc >= 0 ? a.zt[zc * a.Lz + z] : 0.0, fs = zs >= 0 ? a.zt[zs * a.Lz + z] : 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (pr[i] >= 0) {
+        const Cx<double> v = s[z * zstep + (long long)pr[i] * a.K];
+        A[i][0].x = fma(fc, v.x, A[i][0].x);
+        A[i][0].y = fma(fc, v.y, A[i][0].y);
+        A[i][1].x = fma(fs, v.x, A[i][1].x);
+        A[i][1].y = fma(fs, v.y, A[i][1].y);
+      }
+  }
+  double f = 1.0;
+  const SliceDesc* sd = a.sl ? a.sl + tl : nullptr;
+  if (a.exps)
+    f = ldexp(1.0, a.kexp[2 * k] * (a.exps[2 * tl] + sd->eh[0]) + a.kexp[2 * k + 1] * (a.exps[2 * tl + 1] + sd->eh[1]));
+  long long base = 0;  // result element of momentum 0, and the step from one momentum to the next
+  int step = 0;
+  if (a.nblocks == 0) {
+    base = (long long)(sd ? sd->tau : tl) * a.oT + (long long)k * a.oK;
+    step = 1;
+  }
+  for (int b = 0; b < a.nblocks; b++) {
+    const ScatterBlock& B = a.blk[b];
+    const int rel = k - B.k0;
+    if (rel >= 0 && rel < B.groups * B.datasets * B.comps) {
+      const int gd = rel / B.comps;
+      base = B.base * sd->totalT * a.nmom + ((long long)gd * sd->totalT + sd->tau) * a.nmom * B.comps + rel % B.comps;
+      step = B.comps;
+    }
+  }
+  Cx<double>* out = (Cx<double>*)(a.nblocks ? sd->out : a.out);
+  const int kq = a.kphase ? a.kphase[k] : 0;
+  for (int m = m0; m < m1; m++) {
+    const int* md = a.omom + 8 * m;  // momentum index, signs of (x, y, z) times the transform's sign, n
+    const double sx = md[1], sy = md[2], sz = md[3];
+    // exp(i s.theta) = (cx + i sx Sx)(cy + i sy Sy)(cz + i sz Sz)
+    Cx<double> v = A[0][0];
+    v.x -= sx * sy * A[3][0].x + sz * (sx * A[2][1].x + sy * A[1][1].x);
+    v.y -= sx * sy * A[3][0].y + sz * (sx * A[2][1].y + sy * A[1][1].y);
+    // terms with one or three sines carry i and -i
+    const double ix = sx * A[2][0].x + sy * A[1][0].x + sz * A[0][1].x - sx * sy * sz * A[3][1].x;
+    const double iy = sx * A[2][0].y + sy * A[1][0].y + sz * A[0][1].y - sx * sy * sz * A[3][1].y;
+    v = cx<double>((v.x - iy) * f, (v.y + ix) * f);
+    if (a.nblocks) v = cmul(v, source_phase(md + 4, sd->x0, a.L));
+    if (kq & 1) v = cx<double>(-v.y, v.x);
+    if (kq & 2) v = cx<double>(-v.x, -v.y);
+    out[base + (long long)md[0] * step] = v;
+  }
+}
+
+template <typename R, int R1>
+cudaError_t launch_x(const AxisXArgs& a, cudaStream_t s) {
+  using C = XChunk<R>;
+  const int smem = kXWarps * 2 * C::stage * 2 * (int)sizeof(R) + a.Lx * R1 * (int)sizeof(R);
+  cudaError_t e = ensure_smem((const void*)k_axis_x<R, R1>, smem);
+  if (e != cudaSuccess) return e;
+  const long long rows_per = kLines / a.KL;
+  const long long items = (a.rows + rows_per - 1) / rows_per * ((a.K + a.KL - 1) / a.KL) * a.ntau;
+  k_axis_x<R, R1><<<(unsigned)((items + kXWarps - 1) / kXWarps), 32 * kXWarps, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t launch_x_t(const AxisXArgs& a, cudaStream_t s) {
+  switch (a.R1) {
+    case 1: return launch_x<R, 1>(a, s);
+    case 3: return launch_x<R, 3>(a, s);
+    case 5: return launch_x<R, 5>(a, s);
+    case 7: return launch_x<R, 7>(a, s);
+    case 9: return launch_x<R, 9>(a, s);
+  }
+  return cudaErrorInvalidValue;
+}
+
+template <typename R, int NY>
+cudaError_t launch_y_n(const AxisYArgs& a, int kpl, cudaStream_t s) {
+  const int smem = a.Ly * a.RY * 8;
+  const dim3 grid((a.K + 32 * kpl - 1) / (32 * kpl), a.Lz, a.ntau);
+  const void* f = kpl == 2 ? (const void*)k_axis_y<R, NY, 2> : (const void*)k_axis_y<R, NY, 1>;
+  if (smem > 48 << 10) {
+    cudaError_t e = ensure_smem(f, smem);
+    if (e != cudaSuccess) return e;
+  }
+  if (kpl == 2)
+    k_axis_y<R, NY, 2><<<grid, 32 * a.R1, smem, s>>>(a);
+  else
+    k_axis_y<R, NY, 1><<<grid, 32 * a.R1, smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+template <typename R>
+cudaError_t launch_y_t(const AxisYArgs& a, int kpl, cudaStream_t s) {
+  if (a.ny <= 1) return launch_y_n<R, 1>(a, kpl, s);
+  if (a.ny <= 3) return launch_y_n<R, 3>(a, kpl, s);
+  if (a.ny <= 5) return launch_y_n<R, 5>(a, kpl, s);
+  if (a.ny <= 7) return launch_y_n<R, 7>(a, kpl, s);
+  if (a.ny <= 9) return launch_y_n<R, 9>(a, kpl, s);
+  return cudaErrorInvalidValue;
+}
+
+// The rows of one axis: for every distinct a its cos row and, unless a = 0 or
+// a = L/2, its sin row.
+struct AxisRows {
+  std::vector<int> a, cos_row, sin_row;  // per distinct a
+  std::vector<int> row_a, row_sin;       // per row
+  int find(int v) const {
+    for (size_t i = 0; i < a.size(); i++)
+      if (a[i] == v) return (int)i;
+    return -1;
+  }
+  int add(int v, int L) {
+    int i = find(v);
+    if (i >= 0) return i;
+    i = (int)a.size();
+    a.push_back(v);
+    cos_row.push_back((int)row_a.size());
+    row_a.push_back(v);
+    row_sin.push_back(0);
+    if (v != 0 && 2 * v != L) {
+      sin_row.push_back((int)row_a.size());
+      row_a.push_back(v);
+      row_sin.push_back(1);
+    } else {
+      sin_row.push_back(-1);
+    }
+    return i;
+  }
+};
+
+}  // namespace
+
+cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
+  if (a0.ntau < 1 || a0.K < 1) return cudaSuccess;
+  AxisXArgs a = a0;
+  a.KL = 1;
+  while (a.KL < 32 && a.KL < a.K) a.KL *= 2;
+  return fp32 ? launch_x_t<float>(a, s) : launch_x_t<double>(a, s);
+}
+
+cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s) {
+  return fp32 ? launch_y_t<float>(a, kpl, s) : launch_y_t<double>(a, kpl, s);
+}
+
+cudaError_t launch_axis_z(const AxisZArgs& a, cudaStream_t s) {
+  k_axis_z<<<dim3(a.NO, a.ntau, (a.K + 127) / 128), 128, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+}  // namespace p2
+
+namespace p2host {
+
+// Whether a momentum list takes the axis-by-axis projection, and its tables
+// on the device (kept per transform sign until the list changes).
+// The list qualifies when no axis has more than kAxisMaxRows rows (|n| <= 4,
+// every list up to |n|^2 <= 24): a row costs the sum over x a register pair
+// per thread, and larger lists keep the direct projections.
+p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const AxesPlan** out) {
+  *out = nullptr;
+  AxesPlan& ap = c->axes[sign > 0 ? 1 : 0];
+  if (ap.key == moms) {
+    if (ap.usable) *out = &ap;
+    return P2_OK;
+  }
+  ap.key.clear();
+  ap.usable = false;
+  const int nmom = (int)moms.size() / 3;
+  p2::AxisRows ax[3];
+  std::vector<int> ia(3 * (size_t)nmom), sg(3 * (size_t)nmom);
+  bool fits = true;
+  for (int p = 0; p < nmom && fits; p++)
+    for (int d = 0; d < 3; d++) {
+      const int L = c->g.L[d];
+      int m = moms[3 * p + d] % L;
+      if (m < 0) m += L;
+      const int a = std::min(m, L - m);
+      ia[3 * p + d] = ax[d].add(a, L);
+      sg[3 * p + d] = m == a ? 1 : -1;
+      fits = fits && (int)ax[d].row_a.size() <= p2::kAxisMaxRows;
+    }
+  if (!fits || c->Ll[0] > 1024 || c->Ll[1] > 2048) {  // the phase tables fit in shared memory (73 and 148 KB)
+    ap.key = moms;
+    return P2_OK;
+  }
+  const int R1 = (int)ax[0].row_a.size() | 1;  // odd: the x sums are instantiated for 1, 3, 5, 7 and 9 rows
+  const int RY = (int)ax[1].row_a.size(), RZ = (int)ax[2].row_a.size();
+  // (x row, y row) pairs, ordered by x row
+  std::vector<std::vector<int>> ylist(R1);
+  auto use = [&](int r, int s) {
+    if (r >= 0 && s >= 0 && std::find(ylist[r].begin(), ylist[r].end(), s) == ylist[r].end()) ylist[r].push_back(s);
+  };
+  for (int p = 0; p < nmom; p++)
+    for (int i = 0; i < 2; i++)
+      for (int j = 0; j < 2; j++)
+        use(i ? ax[0].sin_row[ia[3 * p]] : ax[0].cos_row[ia[3 * p]],
+            j ? ax[1].sin_row[ia[3 * p + 1]] : ax[1].cos_row[ia[3 * p + 1]]);
+  std::vector<int> first(R1 + 1, 0), yl;
+  int ny = 1;
+  for (int r = 0; r < R1; r++) {
+    first[r] = (int)yl.size();
+    yl.insert(yl.end(), ylist[r].begin(), ylist[r].end());
+    ny = std::max(ny, (int)ylist[r].size());
+  }
+  first[R1] = (int)yl.size();
+  auto pair_of = [&](int r, int s) {
+    if (r < 0 || s < 0) return -1;
+    return first[r] + (int)(std::find(ylist[r].begin(), ylist[r].end(), s) - ylist[r].begin());
+  };
+  // orbits and their momenta, in first-occurrence order
+  std::vector<int> orb, omom;
+  std::vector<std::vector<int>> members;
+  std::vector<int> okey;
+  for (int p = 0; p < nmom; p++) {
+    const int key = (ia[3 * p] * 64 + ia[3 * p + 1]) * 64 + ia[3 * p + 2];
+    size_t o = std::find(okey.begin(), okey.end(), key) - okey.begin();
+    if (o == okey.size()) {
+      okey.push_back(key);
+      members.emplace_back();
+    }
+    members[o].push_back(p);
+  }
+  for (const auto& mem : members) {
+    const int p0 = mem[0];
+    const int xc = ax[0].cos_row[ia[3 * p0]], xs = ax[0].sin_row[ia[3 * p0]];
+    const int yc = ax[1].cos_row[ia[3 * p0 + 1]], ysn = ax[1].sin_row[ia[3 * p0 + 1]];
+    for (int v : {pair_of(xc, yc), pair_of(xc, ysn), pair_of(xs, yc), pair_of(xs, ysn),
+                  ax[2].cos_row[ia[3 * p0 + 2]], ax[2].sin_row[ia[3 * p0 + 2]], (int)omom.size() / 8,
+                  (int)(omom.size() / 8 + mem.size())})
+      orb.push_back(v);
+    for (int p : mem) {
+      omom.push_back(p);
+      for (int d = 0; d < 3; d++) omom.push_back(sign * sg[3 * p + d]);
+      for (int d = 0; d < 3; d++) omom.push_back(moms[3 * p + d]);
+      omom.push_back(0);
+    }
+  }
+  // phase tables in global coordinates, a x reduced mod L in integers
+  std::vector<double> tab;
+  auto value = [&](int d, int a, int is_sin, int xl) {
+    const long long L = c->g.L[d], xg = xl + (long long)c->g.coords[d] * c->Ll[d];
+    const double ph = 2.0 * M_PI * (double)((a * xg) % L) / (double)L;
+    return is_sin ? std::sin(ph) : std::cos(ph);
+  };
+  for (int x = 0; x < c->Ll[0]; x++)
+    for (int r = 0; r < R1; r++)
+      tab.push_back(r < (int)ax[0].row_a.size() ? value(0, ax[0].row_a[r], ax[0].row_sin[r], x) : 0.0);
+  const size_t oy = tab.size();
+  for (int y = 0; y < c->Ll[1]; y++)
+    for (int r = 0; r < RY; r++) tab.push_back(value(1, ax[1].row_a[r], ax[1].row_sin[r], y));
+  const size_t oz = tab.size();
+  for (int r = 0; r < RZ; r++)
+    for (int z = 0; z < c->Ll[2]; z++) tab.push_back(value(2, ax[2].row_a[r], ax[2].row_sin[r], z));
+  std::vector<int> idx(first);
+  const size_t ol = idx.size();
+  idx.insert(idx.end(), yl.begin(), yl.end());
+  const size_t oo = idx.size();
+  idx.insert(idx.end(), orb.begin(), orb.end());
+  const size_t om = idx.size();
+  idx.insert(idx.end(), omom.begin(), omom.end());
+  p2_status st;
+  if ((st = upload_async(c, ap.tab, tab.data(), tab.size() * sizeof(double), "axis phases")) != P2_OK) return st;
+  if ((st = upload_async(c, ap.idx, idx.data(), idx.size() * sizeof(int), "axis momenta")) != P2_OK) return st;
+  ap.R1 = R1;
+  ap.RY = RY;
+  ap.NP = (int)yl.size();
+  ap.NO = (int)members.size();
+  ap.ny = ny;
+  ap.nmom = nmom;
+  ap.xt = (const double*)ap.tab.p;
+  ap.yt = ap.xt + oy;
+  ap.zt = ap.xt + oz;
+  ap.first = (const int*)ap.idx.p;
+  ap.ylist = ap.first + ol;
+  ap.orb = ap.first + oo;
+  ap.omom = ap.first + om;
+  ap.usable = true;
+  ap.key = moms;
+  *out = &ap;
+  return P2_OK;
+}
+
+p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
+                 void* s1) {
+  p2::AxisXArgs a{};
+  a.c = field;
+  a.sT = sT;
+  a.sK = sK;
+  a.ntau = n;
+  a.K = K;
+  a.rows = c->Ll[1] * c->Ll[2];
+  a.Lx = c->Ll[0];
+  a.R1 = ap.R1;
+  a.xt = ap.xt;
+  a.s1 = s1;
+  ProfScope ps(c, "project_axis_x");
+  P2_TRY(c, p2::launch_axis_x(a, fp32, c->stream), "projection over x");
+  return P2_OK;
+}
+
+// Sums over y and z of S1 (n slices, K components), then the results: with
+// blocks into the slices' results dsl, otherwise into out[tau * oT + k * oK + p].
+p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o) {
+  const int Lz = c->Ll[2];
+  P2_TRY(c, c->axes_s2.ensure((size_t)n * Lz * ap.NP * K * 16), "projection workspace");
+  p2::AxisYArgs y{};
+  y.s1 = s1;
+  y.s2 = c->axes_s2.p;
+  y.ntau = n;
+  y.K = K;
+  y.Ly = c->Ll[1];
+  y.Lz = Lz;
+  y.R1 = ap.R1;
+  y.RY = ap.RY;
+  y.NP = ap.NP;
+  y.ny = ap.ny;
+  y.yt = ap.yt;
+  y.first = ap.first;
+  y.ylist = ap.ylist;
+  // two components per lane share each phase; one where that leaves too few blocks to fill the SMs
+  std::vector<std::vector<int>> cands{{2}, {1}};
+  if ((long long)n * Lz * ((K + 63) / 64) < 2LL * c->nsm) std::swap(cands[0], cands[1]);
+  char key[160];
+  std::snprintf(key, sizeof(key), "%s axes V3=%lld K=%d nmom=%d n=%d", fp32 ? "project_split" : "project_fp64", c->V3, K,
+                ap.nmom, n);
+  std::vector<int> pick;
+  P2_TRY(c,
+         tune_choose(c->tuner.get(), key, cands, c->stream, !c->capturing,
+                     [&](const std::vector<int>& v) { return p2::launch_axis_y(y, fp32, v[0], c->stream); }, pick),
+         "projection tuning");
+  {
+    ProfScope ps(c, "project_axis_y");
+    P2_TRY(c, p2::launch_axis_y(y, fp32, pick[0], c->stream), "projection over y");
+  }
+  p2::AxisZArgs z{};
+  z.s2 = c->axes_s2.p;
+  z.ntau = n;
+  z.K = K;
+  z.Lz = Lz;
+  z.NP = ap.NP;
+  z.NO = ap.NO;
+  z.nmom = ap.nmom;
+  z.zt = ap.zt;
+  z.orb = ap.orb;
+  z.omom = ap.omom;
+  z.sl = o.dsl;
+  for (int d = 0; d < 3; d++) z.L[d] = c->g.L[d];
+  z.exps = o.exps;
+  z.kexp = o.kexp;
+  z.kphase = o.kphase;
+  const size_t nb = o.blocks ? o.blocks->size() : 0;
+  if (nb > (size_t)p2::kMaxBlocks) return c->fail(P2_ERR_INVALID_ARG, "too many result blocks");
+  z.nblocks = (int)nb;
+  for (size_t b = 0; b < nb; b++) z.blk[b] = (*o.blocks)[b];
+  z.out = o.out;
+  z.oT = o.oT;
+  z.oK = o.oK;
+  ProfScope ps(c, "project_axis_z");
+  P2_TRY(c, p2::launch_axis_z(z, c->stream), "projection over z");
+  return P2_OK;
+}
+
+}  // namespace p2host

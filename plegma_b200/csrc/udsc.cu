@@ -616,8 +616,10 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
       if ((st = upload_async(c, U.kexp, ke.data(), ke.size() * sizeof(int), "udsc exponents")) != P2_OK) return st;
     }
   }
+  const AxesPlan* ap = nullptr;  // the axis-by-axis projection, when the list qualifies
+  if (!split && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
   // phase tables (origin 0; the scatter applies the source phase)
-  if (!split && c->plain_moms_key != pl.moms) {
+  if (!split && !ap && c->plain_moms_key != pl.moms) {
     c->plain_moms_key.clear();
     std::vector<double> tabh = phase_tables(c, pl.moms.data(), pl.nmom, -1, pl.Lmax);
     if ((st = upload_async(c, c->ptab, tabh.data(), tabh.size() * sizeof(double), "phase table")) != P2_OK)
@@ -738,6 +740,29 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
         ProfScope ps(c, "contract_udsc_fp64");
         P2_TRY(c, launch_contract_udsc(a, c->nsm, c->stream), "udsc contraction");
       }
+      std::vector<SliceDesc> desc(n);
+      for (int i = 0; i < n; i++) {
+        std::memset(&desc[i], 0, sizeof(SliceDesc));
+        desc[i].out = dres;
+        desc[i].tau = taus[c0 + i];
+        desc[i].totalT = r->totalT;
+        for (int d = 0; d < 3; d++) desc[i].x0[d] = r->source[d];
+      }
+      P2_TRY(c, U.desc.ensure((size_t)n * sizeof(SliceDesc)), "descriptor alloc");
+      P2_TRY(c,
+             cudaMemcpyAsync(U.desc.p, desc.data(), (size_t)n * sizeof(SliceDesc), cudaMemcpyHostToDevice,
+                             c->stream),
+             "descriptor upload");
+      if (ap) {
+        P2_TRY(c, c->axes_s1.ensure((size_t)n * c->Ll[1] * c->Ll[2] * ap->R1 * nd * 16), "projection workspace");
+        if ((st = axes_x(c, *ap, c->cbuf.p, 0, (long long)nd * c->V3, c->V3, n, nd, c->axes_s1.p)) != P2_OK) return st;
+        const std::vector<ScatterBlock> blocks{ScatterBlock{0, 1, nd, 1, (long long)ds_off}};
+        AxesOut ao;
+        ao.dsl = (const SliceDesc*)U.desc.p;
+        ao.blocks = &blocks;
+        if ((st = axes_yz(c, *ap, c->axes_s1.p, 0, n, nd, ao)) != P2_OK) return st;
+        continue;
+      }
       ProjArgs pa{};
       pa.c = c->cbuf.p;
       pa.sT = (long long)nd * c->V3;
@@ -762,19 +787,6 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
         ProfScope ps(c, "project_fp64");
         P2_TRY(c, launch_project_fp64(pa, c->stream), "projection kernel");
       }
-      std::vector<SliceDesc> desc(n);
-      for (int i = 0; i < n; i++) {
-        std::memset(&desc[i], 0, sizeof(SliceDesc));
-        desc[i].out = dres;
-        desc[i].tau = taus[c0 + i];
-        desc[i].totalT = r->totalT;
-        for (int d = 0; d < 3; d++) desc[i].x0[d] = r->source[d];
-      }
-      P2_TRY(c, U.desc.ensure((size_t)n * sizeof(SliceDesc)), "descriptor alloc");
-      P2_TRY(c,
-             cudaMemcpyAsync(U.desc.p, desc.data(), (size_t)n * sizeof(SliceDesc), cudaMemcpyHostToDevice,
-                             c->stream),
-             "descriptor upload");
       ScatterArgs sa{};
       sa.part = (const double*)c->part.p;
       sa.ntau = n;
