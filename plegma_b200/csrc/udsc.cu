@@ -1,30 +1,34 @@
 // Table-driven baryon two-point functions: the reference's UDSC set
 // (contractBaryonsUDSC, lib/PLEGMA_Correlator.cu:137-189, kernels
-// lib/kernels/PLEGMA_baryons_udsc.cu:85-309), plain FP64 form.
+// lib/kernels/PLEGMA_baryons_udsc.cu:85-309), both forms.
 //
 // A flavour product (e.g. "uud") has up to 16 datasets (interpolator and
 // projector variants); dataset d of a site is
 //   sum_entries w * sum_{eps eps'} P1[s0 s1][a a'] P2[s2 s3][b b'] P3[s4 s5][c c']
-// over the spin tables of plegma_b200/udsc.py (weights in single precision
-// like the reference's).  The colour sums factorise through the diquark
-//   G_{s0 s1, s2 s3}[c][c'] = sum eps_abc eps_a'b'c' P1[a a'] P2[b b']
-// (36 complex products), and an entry costs one 9-term product G . P3.
-// Across a product's datasets only 112-256 distinct (s0 s1 s2 s3) tuples
-// occur, so each G is computed once per site and shared by every entry of
-// every dataset that uses it (the reference evaluates 36 x 3 products per
-// entry).
+// over the spin tables of plegma_b200/udsc.py (real weights in single
+// precision like the reference's; the reference spends 108 complex products
+// per entry).  udsc.site_program turns a product's entries into a program:
+// entries that differ by an exchange of equal flavours are merged, every
+// distinct triple of spin blocks is evaluated once for all datasets, as a
+// diquark of two of its blocks (36 complex products) dotted with the third
+// (9 products), and a greedy cover keeps the diquarks few.  For "uud" that is
+// 133 diquarks and 424 dots for 848 weights, against 240 diquarks and 1100
+// dots of the entries as they stand.
 //
-// Layout: one site per half-warp; the three propagators of 16 sites are
-// staged with cp.async in two stages ([site][3 x 144 + 1] complex double).
-// The host assigns the distinct tuples to the 16 lanes (balanced by work)
-// and encodes one instruction stream per lane:
-//   per tuple: P1 block | P2 block << 8, four words of per-dataset entry
-//   counts (one byte each), then per entry: P3 block, Re w, Im w (float bits).
-// Each lane accumulates all datasets in registers; a half-warp reduce-scatter
-// (lane d ends with dataset d) gives the site's values, written to a
-// [slice][dataset][site] buffer that
-// the FP64 projection (project_fp64.cu) and the deterministic reduction
-// consume.
+// One site per lane: the eight warps of a block take 32 sites of one slice
+// and an eighth of the program each, so the control flow is the same for all
+// lanes (the program is read from constant memory), a block's nine entries
+// are conflict-free loads, and nothing moves between lanes.  The datasets'
+// partial sums of the eight warps meet in shared memory once per product.
+// Products on the same one or two flavours run in one launch on the same
+// staged tile.  The sums go to a [slice][dataset][site] buffer that the
+// projection consumes.
+// Measured on B200 against one instruction stream per lane over the unmerged
+// entries (16 lanes of a site in divergent loops): split form, 32^3 x 16, u and
+// d (28 datasets), 123 momenta 20.6 -> 6.2 ms; plain form, 16^3 x 16, all 200
+// datasets, 33 momenta 33.9 -> 9.4 ms.
+// Bound: the latency of a warp's chain program word -> block -> products, with
+// 16 (split) or 8 (plain) warps per SM; the FMAs alone would take a quarter.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -42,454 +46,373 @@ using namespace p2host;
 namespace p2 {
 namespace {
 
-constexpr int kThreadsU = 256;
-constexpr int kSitesU = 16;
-constexpr int kRowU = 3 * 144 + 1;  // complex per staged site row (P1, P2, P3 + pad)
-constexpr int kStageU = kSitesU * kRowU;
-constexpr int kMaxDs = 16;          // datasets per product (the reference's largest product has 16)
+constexpr int kThreadsU = 32 * kUdscWarps;
+constexpr int kSitesU = 32;  // sites of a tile, one per lane
+constexpr int kMaxDs = 16;   // datasets per product (the reference's largest product has 16)
+constexpr int kMaxProgs = 4; // products on one pair of flavours: aab, abb, aaa, bbb
+
+__constant__ unsigned short c_code[kUdscCodeWords] = P2_INIT_UDSC_CODE;
+__constant__ double c_weight[kUdscWeights] = P2_INIT_UDSC_WEIGHTS;
 
 struct UdscSlice {
-  long long off[3];  // element offset of the slice inside each of the three views
+  long long off[3];  // element offset of the slice inside each of the views
   int xf[3];         // load-time transform of each view on this slice (PropXf)
   int pad;
 };
 
-struct UdscArgs {
-  const Cx<double>* p0;
-  const Cx<double>* p1;
-  const Cx<double>* p2;
-  long long vol0, vol1, vol2;  // component strides of the views
-  const UdscSlice* sl;
-  int ntau, V3, nd;
-  const int* plan;  // [16] lane offsets, then the lane streams
-  Cx<double>* out;  // [ntau][nd][V3]
+// One flavour product of a launch.
+struct UdscProg {
+  int start[kUdscWarps];  // first word of each warp's code
+  int nd, k0;             // datasets and their first component in the output
+  int boff;               // added to the program's blocks (16 x the view of its first flavour)
 };
 
-__device__ __forceinline__ void issue_tile_u(const UdscArgs& a, Cx<double>* st, const TileCursor& t, int ntau) {
-  if (t.tl < ntau) {
-    const int tl = t.tl;
-    const int s = threadIdx.x & (kSitesU - 1);
-    const int x = t.x0() + s;
-    const bool ok = x < a.V3;
-    const UdscSlice* sd = a.sl + tl;
-    // thread i copies component i/16 + 16 r of site i%16: rows r < 9 are P1,
-    // 9 <= r < 18 P2, 18 <= r < 27 P3
+struct UdscArgs {
+  const void* p[3];  // views of the launch's NF flavours
+  long long vol[3];  // component strides
+  const UdscSlice* sl;
+  int ntau, V3, K;   // slices, sites, components of the output
+  int nprog;
+  UdscProg prog[kMaxProgs];
+  int* e3;           // split form: [ntau][3], view v of slice t is staged times 2^-e3[3t+v]
+  int* es;           // split form: [ntau][2], what the components' exponents (kexp) multiply
+  void* out;         // [ntau][K][V3] complex double (plain) or complex float (split)
+  int* cmax;         // split form: [ntau][K] max |Re|, |Im| as float bits, or null
+};
+
+// ---- a tile's propagators in shared memory, the site in the lane -----------
+// FP64: [16 f + block][9 colours][32 sites]; FP32: four pairs of colours as
+// 16-byte units [16 f + block][4][32 sites], then colour 8 [16 f + block][32 sites].
+template <typename R, int NF>
+struct SiteTile;
+template <int NF>
+struct SiteTile<double, NF> {
+  static constexpr int kBytes = NF * 144 * kSitesU * 16;
+  Cx<double>* p;
+  __device__ __forceinline__ SiteTile(unsigned char* sm, int lane) : p((Cx<double>*)sm + lane) {}
+  __device__ __forceinline__ void load9(int blk, Cx<double> (&v)[9]) const {
 #pragma unroll
-    for (int f = 0; f < 3; f++) {
-      const Cx<double>* base = f == 0 ? a.p0 : f == 1 ? a.p1 : a.p2;
-      const long long vol = f == 0 ? a.vol0 : f == 1 ? a.vol1 : a.vol2;
-      const Cx<double>* src = base + sd->off[f] + (ok ? x : 0);
-#pragma unroll 3
-      for (int r = 0; r < 9; r++) {
-        const int comp = (threadIdx.x >> 4) + 16 * r;
-        cp_async16(st + s * kRowU + 144 * f + comp, src + comp * vol, ok ? 16 : 0);
-      }
+    for (int i = 0; i < 9; i++) v[i] = p[(blk * 9 + i) * kSitesU];
+  }
+};
+template <int NF>
+struct SiteTile<float, NF> {
+  static constexpr int kBytes = NF * 144 * kSitesU * 8;
+  float4* q;
+  Cx<float>* last;
+  __device__ __forceinline__ SiteTile(unsigned char* sm, int lane)
+      : q((float4*)sm + lane), last((Cx<float>*)((float4*)sm + NF * 16 * 4 * kSitesU) + lane) {}
+  __device__ __forceinline__ void load9(int blk, Cx<float> (&v)[9]) const {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float4 x = q[(blk * 4 + k) * kSitesU];
+      v[2 * k] = cx<float>(x.x, x.y);
+      v[2 * k + 1] = cx<float>(x.z, x.w);
     }
+    v[8] = last[blk * kSitesU];
+  }
+};
+
+// FP64: the tile by cp.async, the load-time transforms in place.
+template <int NF>
+__device__ __forceinline__ void stage_tile(const UdscArgs& a, const SiteTile<double, NF>& t, int tl, int x, bool ok) {
+  const int warp = threadIdx.x >> 5;
+  const UdscSlice& sd = a.sl[tl];
+#pragma unroll
+  for (int f = 0; f < NF; f++) {
+    const Cx<double>* src = (const Cx<double>*)a.p[f] + sd.off[f] + (ok ? x : 0);
+#pragma unroll 6
+    for (int c = warp; c < 144; c += kUdscWarps)
+      cp_async16(t.p + (144 * f + c) * kSitesU, src + c * a.vol[f], ok ? 16 : 0);
   }
   cp_async_commit();
-}
-
-// Sum of the 16 lanes' dataset accumulators, lane l ending with dataset l:
-// a reduce-scatter (8 + 4 + 2 + 1 exchanged values instead of 16 all-reduces).
-template <typename R>
-__device__ __forceinline__ Cx<R> reduce_scatter16(Cx<R> (&acc)[16], int l, unsigned mask) {
-#pragma unroll
-  for (int h = 8; h >= 1; h >>= 1) {
-    const bool up = (l & h) != 0;
-#pragma unroll
-    for (int j = 0; j < h; j++) {
-      const Cx<R> send = up ? acc[j] : acc[j + h];
-      const Cx<R> keep = up ? acc[j + h] : acc[j];
-      acc[j] = keep + shfl_xor16(send, h, mask);
+  cp_async_wait<0>();
+  if (sd.xf[0] | sd.xf[1] | sd.xf[2]) {  // uniform over the block
+    __syncthreads();
+    for (int q = warp; q < 36 * NF; q += kUdscWarps) {
+      const int f = q / 36;
+      int comp[4];
+      prop_group_comps(q - 36 * f, comp);
+      Cx<double>* r = t.p + 144 * f * kSitesU;
+      prop_group_transform(r[comp[0] * kSitesU], r[comp[1] * kSitesU], r[comp[2] * kSitesU], r[comp[3] * kSitesU],
+                           sd.xf[f]);
     }
   }
-  return acc[0];
 }
 
-__global__ void __launch_bounds__(kThreadsU, 1) k_contract_udsc(const UdscArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<double>* sm = (Cx<double>*)smem_raw;
-  const int tid = threadIdx.x;
-  const int hw = tid >> 4, l = tid & 15;
-  const unsigned mask = halfwarp_mask();
-  const int tiles_per_tau = (a.V3 + kSitesU - 1) / kSitesU;
-  TileCursor cur(blockIdx.x, gridDim.x, tiles_per_tau);
-  TileCursor nx2 = cur.next();
-  const int* stream0 = a.plan + a.plan[l];
-
-  issue_tile_u(a, sm, cur, a.ntau);
-  issue_tile_u(a, sm + kStageU, nx2, a.ntau);
-  for (int it = 0; cur.tl < a.ntau; cur = cur.next(), it++) {
-    Cx<double>* st = sm + (it & 1) * kStageU;
-    cp_async_wait<1>();
-    __syncthreads();
-    const int tl = cur.tl;
-    {
-      // load-time transforms of the staged tile, in place (uniform per tile)
-      const UdscSlice& sd = a.sl[tl];
-      if (sd.xf[0] | sd.xf[1] | sd.xf[2]) {
-        const int s = tid & (kSitesU - 1);
-        for (int q = tid >> 4; q < 108; q += kThreadsU / kSitesU) {
-          const int f = q / 36;
-          int comp[4];
-          prop_group_comps(q - 36 * f, comp);
-          Cx<double>* r = st + s * kRowU + 144 * f;
-          prop_group_transform(r[comp[0]], r[comp[1]], r[comp[2]], r[comp[3]], sd.xf[f]);
+// FP32: loaded, transformed, scaled by 2^-E (in double: exact, no intermediate
+// leaves the range) and converted in registers; two blocks per SM overlap the
+// loads of one with the contraction of the other.
+template <typename Tin, int NF>
+__device__ __forceinline__ void stage_tile(const UdscArgs& a, const SiteTile<float, NF>& t, int tl, int x, bool ok) {
+  const int warp = threadIdx.x >> 5;
+  const UdscSlice& sd = a.sl[tl];
+#pragma unroll
+  for (int f = 0; f < NF; f++) {
+    const Cx<Tin>* src = (const Cx<Tin>*)a.p[f] + sd.off[f] + (ok ? x : 0);
+    const long long vol = a.vol[f];
+    const double sc = ldexp(1.0, -a.e3[3 * tl + f]);
+    const int xf = sd.xf[f];
+    // groups 0..15: (first block b of 0, 1, 4, 5; colours 2k, 2k + 1); 16..19: (b, colour 8)
+#pragma unroll 1
+    for (int g = warp; g < 20; g += kUdscWarps) {
+      const int bq = g & 3, b = (bq >> 1) * 4 + (bq & 1);
+      if (g < 16) {
+        const int k = g >> 2;
+        Cx<Tin> raw[2][4];
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            raw[c][i] = ok ? src[(9 * (b + group_blk(i)) + 2 * k + c) * vol] : czero<Tin>();
+        Cx<double> v[2][4];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+#pragma unroll
+          for (int i = 0; i < 4; i++) v[c][i] = cx<double>((double)raw[c][i].x, (double)raw[c][i].y);
+          prop_group_transform(v[c][0], v[c][1], v[c][2], v[c][3], xf);
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          t.q[((16 * f + b + group_blk(i)) * 4 + k) * kSitesU] =
+              make_float4((float)(v[0][i].x * sc), (float)(v[0][i].y * sc), (float)(v[1][i].x * sc),
+                          (float)(v[1][i].y * sc));
+      } else {
+        Cx<double> v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const Cx<Tin> r = ok ? src[(9 * (b + group_blk(i)) + 8) * vol] : czero<Tin>();
+          v[i] = cx<double>((double)r.x, (double)r.y);
+        }
+        prop_group_transform(v[0], v[1], v[2], v[3], xf);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          t.last[(16 * f + b + group_blk(i)) * kSitesU] = cx<float>((float)(v[i].x * sc), (float)(v[i].y * sc));
       }
     }
-    const int x = cur.x0() + hw;
-    if (x < a.V3) {
-      const RowF64 row{st + hw * kRowU};
-      Cx<double> acc[kMaxDs];
+  }
+}
+
+// G[c][e] = sum eps_abc eps_xye A[a][x] B[b][y]
+__device__ __forceinline__ void site_diquark(const Cx<double> (&a)[9], const Cx<double> (&b)[9], Cx<double> (&g)[9]) {
 #pragma unroll
-      for (int d = 0; d < kMaxDs; d++) acc[d] = czero<double>();
-      const int* q = stream0;
-      const int ntup = *q++;
+  for (int c = 0; c < 3; c++)
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, e1 = (e + 1) % 3, e2 = (e + 2) % 3;
+      Cx<double> r = cmul(a[c1 * 3 + e1], b[c2 * 3 + e2]);
+      cmsub(r, a[c1 * 3 + e2], b[c2 * 3 + e1]);
+      cmsub(r, a[c2 * 3 + e1], b[c1 * 3 + e2]);
+      cmac(r, a[c2 * 3 + e2], b[c1 * 3 + e1]);
+      g[c * 3 + e] = r;
+    }
+}
+__device__ __forceinline__ void site_diquark(const Cx<float> (&a)[9], const Cx<float> (&b)[9], Cx<float> (&g)[9]) {
+  // paired FMAs: (a.x b.x, a.x b.y) and (a.y b.x, a.y b.y) accumulated separately
+  f32x2 bp[9], bn[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) {
+    bp[i] = f2pack(b[i].x, b[i].y);
+    bn[i] = f2pack(-b[i].x, -b[i].y);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, e1 = (e + 1) % 3, e2 = (e + 2) % 3;
+      f32x2 px = f2pack(0.f, 0.f), py = px;
+      auto term = [&](int ia, f32x2 bb) {
+        px = f2fma(f2pack(a[ia].x, a[ia].x), bb, px);
+        py = f2fma(f2pack(a[ia].y, a[ia].y), bb, py);
+      };
+      term(c1 * 3 + e1, bp[c2 * 3 + e2]);
+      term(c1 * 3 + e2, bn[c2 * 3 + e1]);
+      term(c2 * 3 + e1, bn[c1 * 3 + e2]);
+      term(c2 * 3 + e2, bp[c1 * 3 + e1]);
+      float xr, xi, yr, yi;
+      f2unpack(px, xr, xi);
+      f2unpack(py, yr, yi);
+      g[c * 3 + e] = cx<float>(xr - yi, xi + yr);
+    }
+}
+
+// This warp's part of a program on its lanes' sites.
+template <typename R, int NF>
+__device__ __forceinline__ void run_program(const SiteTile<R, NF>& t, int q, int boff, Cx<R> (&acc)[kMaxDs]) {
+  const int na = c_code[q++];
 #pragma unroll 1
-      for (int t = 0; t < ntup; t++) {
-        const int head = q[0];
-        const unsigned cnt[4] = {(unsigned)q[1], (unsigned)q[2], (unsigned)q[3], (unsigned)q[4]};
-        q += 5;
-        Cx<double> g[9];
-#pragma unroll
-        for (int i = 0; i < 9; i++) g[i] = czero<double>();
-        // blocks: P1 at 0..15, P2 at 16..31 of the row (block offset kD), P3 at 32..47
-        diquark_acc(row, head & 255, (head >> 8) & 255, 0, 0, 1.0, 0, 0, g);
-#pragma unroll
-        for (int d = 0; d < kMaxDs; d++) {
-          if (d >= a.nd) break;
-          const int n = (int)((cnt[d >> 2] >> (8 * (d & 3))) & 255u);
+  for (int ia = 0; ia < na; ia++) {
+    Cx<R> A[9];
+    t.load9(c_code[q] + boff, A);
+    const int nb = c_code[q + 1];
+    q += 2;
 #pragma unroll 1
-          for (int e = 0; e < n; e++) {
-            const int blk = q[0];
-            const Cx<double> w = cx<double>((double)__int_as_float(q[1]), (double)__int_as_float(q[2]));
-            q += 3;
-            Cx<double> z[9];
-            row.load9(blk, z);
-            Cx<double> dot = czero<double>();
-#pragma unroll
-            for (int i = 0; i < 9; i++) cmac(dot, g[i], z[i]);
-            cmac(acc[d], w, dot);
+    for (int ib = 0; ib < nb; ib++) {
+      Cx<R> g[9];
+      {
+        Cx<R> B[9];
+        t.load9(c_code[q] + boff, B);
+        site_diquark(A, B, g);
+      }
+      const int ndot = c_code[q + 1];
+      q += 2;
+#pragma unroll 1
+      for (int iz = 0; iz < ndot; iz++) {
+        Cx<R> z[9];
+        t.load9(c_code[q] + boff, z);
+        const int ne = c_code[q + 1];
+        q += 2;
+        const Cx<R> v = cdot9(g, z);
+#pragma unroll 1
+        for (int ie = 0; ie < ne; ie++) {
+          const int w = c_code[q++];
+          const R f = (R)c_weight[w >> 4];
+          switch (w & 15) {
+#define P2_ACC(i)                          \
+  case i:                                  \
+    acc[i].x = fma(f, v.x, acc[i].x);      \
+    acc[i].y = fma(f, v.y, acc[i].y);      \
+    break;
+            P2_ACC(0) P2_ACC(1) P2_ACC(2) P2_ACC(3) P2_ACC(4) P2_ACC(5) P2_ACC(6) P2_ACC(7)
+            P2_ACC(8) P2_ACC(9) P2_ACC(10) P2_ACC(11) P2_ACC(12) P2_ACC(13) P2_ACC(14) P2_ACC(15)
+#undef P2_ACC
           }
         }
       }
-      Cx<double>* o = a.out + (long long)tl * a.nd * a.V3 + x;
-      if (a.nd > 4) {
-        static_assert(kMaxDs == 16, "the reduce-scatter spreads 16 datasets over the 16 lanes");
-        const Cx<double> v = reduce_scatter16(acc, l, mask);
-        if (l < a.nd) o[(long long)l * a.V3] = v;
-      } else {
+    }
+  }
+}
+
+// Shared memory: the tile, then (with more than one program) the warps'
+// partial sums; a single program's go over the tile, which is dead by then
+// (three FP64 flavours fill the shared memory).
+template <typename R, int NF>
+constexpr int udsc_smem(int nprog, int nd) {
+  const int red = kUdscWarps * nd * kSitesU * 2 * (int)sizeof(R);
+  return nprog > 1 ? SiteTile<R, NF>::kBytes + red : SiteTile<R, NF>::kBytes > red ? SiteTile<R, NF>::kBytes : red;
+}
+
+template <typename R, typename Tin, int NF>
+__global__ void __launch_bounds__(kThreadsU, sizeof(R) == 4 ? 2 : 1) k_contract_udsc(const UdscArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const SiteTile<R, NF> tile(smem_raw, lane);
+  Cx<R>* red = (Cx<R>*)(a.nprog > 1 ? smem_raw + SiteTile<R, NF>::kBytes : smem_raw);
+  const int tpt = (a.V3 + kSitesU - 1) / kSitesU;
+  const long long ntile = (long long)tpt * a.ntau;
+  for (long long i = blockIdx.x; i < ntile; i += gridDim.x) {
+    const int tl = (int)(i / tpt), x = (int)(i % tpt) * kSitesU + lane;
+    const bool ok = x < a.V3;
+    if constexpr (sizeof(R) == 8)
+      stage_tile<NF>(a, tile, tl, x, ok);
+    else
+      stage_tile<Tin, NF>(a, tile, tl, x, ok);
+    __syncthreads();
+#pragma unroll 1
+    for (int p = 0; p < a.nprog; p++) {
+      const UdscProg& pg = a.prog[p];
+      Cx<R> acc[kMaxDs];
 #pragma unroll
-        for (int d = 0; d < 4; d++) {
-          if (d >= a.nd) break;
-          Cx<double> v = acc[d];
-          v = v + shfl_xor16(v, 1, mask);
-          v = v + shfl_xor16(v, 2, mask);
-          v = v + shfl_xor16(v, 4, mask);
-          v = v + shfl_xor16(v, 8, mask);
-          if (l == d) o[(long long)d * a.V3] = v;
-        }
+      for (int d = 0; d < kMaxDs; d++) acc[d] = czero<R>();
+      run_program(tile, pg.start[warp], pg.boff, acc);
+      __syncthreads();  // the tile (single program) or the previous program's sums are read
+#pragma unroll
+      for (int d = 0; d < kMaxDs; d++)
+        if (d < pg.nd) red[(warp * pg.nd + d) * kSitesU + lane] = acc[d];
+      __syncthreads();
+      for (int d = warp; d < pg.nd; d += kUdscWarps) {
+        Cx<R> v = czero<R>();
+#pragma unroll
+        for (int w = 0; w < kUdscWarps; w++) v = v + red[(w * pg.nd + d) * kSitesU + lane];
+        const long long row = (long long)tl * a.K + pg.k0 + d;
+        if (ok) ((Cx<R>*)a.out)[row * a.V3 + x] = v;
+        if constexpr (sizeof(R) == 4)
+          if (a.cmax) {
+            const unsigned m = __reduce_max_sync(0xffffffffu, ok ? __float_as_uint(fmaxf(fabsf(v.x), fabsf(v.y))) : 0u);
+            if (lane == 0) atomicMax(a.cmax + row, (int)m);
+          }
       }
     }
-    __syncthreads();
-    nx2 = nx2.next();  // two tiles ahead of the next iteration's
-    issue_tile_u(a, st, nx2, a.ntau);
+    __syncthreads();  // the sums are read and the tile is dead
   }
-  cp_async_wait<0>();
 }
-
-cudaError_t launch_contract_udsc(const UdscArgs& a, int grid, cudaStream_t s) {
-  const int smem = 2 * kStageU * (int)sizeof(Cx<double>);
-  cudaError_t e = ensure_smem((const void*)k_contract_udsc, smem);
-  if (e != cudaSuccess) return e;
-  k_contract_udsc<<<grid, kThreadsU, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-// ---- split form --------------------------------------------------------------
-// The same lane streams in FP32 on the three views scaled by 2^-E (per slice
-// and view, exact), the FP32 tile in the padded row layout of RowF32 with the
-// views at blocks 0-15, 16-31, 32-47; per (slice, dataset) the maximum of
-// |Re|, |Im| for the hi+lo FP16 split of the tensor-core projection.
-constexpr int kRowU32 = 48 * 10 + 2;  // complex per FP32 site row (161 x 3 units: rows start in different bank groups)
-
-struct UdscArgsF32 {
-  const void* p[3];
-  long long vol[3];  // component strides of the views
-  const UdscSlice* sl;
-  int ntau, V3, nd;
-  const int* plan;
-  int* e3;          // [ntau][3]: view v of slice t is staged times 2^-e3[3t+v]
-  int* es;          // [ntau][2]: (sum of the slice's three exponents, 0), the un-scaling of every dataset
-  Cx<float>* out;   // [ntau][nd][V3]
-  int* cmax;        // [ntau][nd] max |Re|, |Im| as float bits
-};
 
 // Per slice and view the binary exponent of the largest of a strided sample
 // (every 7th component, every 97th site), plus one when the view is rotated.
+// One block per (slice, view).
 template <typename Tin>
-__global__ void k_sample_udsc(const UdscArgsF32 a) {
+__global__ void k_sample_udsc(const UdscArgs a, int nf) {
   __shared__ int red[256];
-  const int tl = blockIdx.x;
+  const int tl = blockIdx.x, f = blockIdx.y;
   const UdscSlice& sd = a.sl[tl];
-  int total = 0;
-  for (int f = 0; f < 3; f++) {
-    const Cx<Tin>* p = (const Cx<Tin>*)a.p[f] + sd.off[f];
-    int emax = -100000;
-    for (int i = threadIdx.x; i < 21 * 1024; i += blockDim.x) {
-      const int comp = (i % 21) * 7;
-      const long long x = ((long long)(i / 21) * 97) % a.V3;
-      const Cx<Tin> v = p[comp * a.vol[f] + x];
-      int e;
-      if (v.x != 0) {
-        frexp((double)v.x, &e);
-        emax = max(emax, e);
-      }
-      if (v.y != 0) {
-        frexp((double)v.y, &e);
-        emax = max(emax, e);
-      }
+  const Cx<Tin>* p = (const Cx<Tin>*)a.p[f] + sd.off[f];
+  int emax = -100000;
+  for (int i = threadIdx.x; i < 21 * 1024; i += blockDim.x) {
+    const int comp = (i % 21) * 7;
+    const long long x = ((long long)(i / 21) * 97) % a.V3;
+    const Cx<Tin> v = p[comp * a.vol[f] + x];
+    int e;
+    if (v.x != 0) {
+      frexp((double)v.x, &e);
+      emax = max(emax, e);
     }
-    red[threadIdx.x] = emax;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-      if (threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-      __syncthreads();
+    if (v.y != 0) {
+      frexp((double)v.y, &e);
+      emax = max(emax, e);
     }
-    const int E = (red[0] == -100000 ? 0 : red[0]) + ((sd.xf[f] & 3) ? 1 : 0);
-    total += E;
-    if (threadIdx.x == 0) a.e3[3 * tl + f] = E;
+  }
+  red[threadIdx.x] = emax;
+  __syncthreads();
+  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    if (threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    a.es[2 * tl] = total;
-    a.es[2 * tl + 1] = 0;
-  }
-}
-
-template <typename Tin>
-__device__ __forceinline__ void issue_tile_u32(const UdscArgsF32& a, Cx<Tin>* st, const TileCursor& t, int ntau) {
-  if (t.tl < ntau) {
-    const int tl = t.tl;
-    const int s = threadIdx.x & (kSitesU - 1);
-    const int x = t.x0() + s;
-    const bool ok = x < a.V3;
-    const UdscSlice* sd = a.sl + tl;
-    // component-major staging [view * 144 + component][16 sites]: thread i
-    // copies component i/16 + 16 r of site i%16
-#pragma unroll
-    for (int f = 0; f < 3; f++) {
-      const Cx<Tin>* src = (const Cx<Tin>*)a.p[f] + sd->off[f] + (ok ? x : 0);
-#pragma unroll 3
-      for (int r = 0; r < 9; r++) {
-        const int comp = (threadIdx.x >> 4) + 16 * r;
-        Cx<Tin>* dst = st + (144 * f + comp) * kSitesU + s;
-        if (sizeof(Tin) == 8)
-          cp_async16(dst, src + comp * a.vol[f], ok ? 16 : 0);
-        else
-          cp_async8(dst, src + comp * a.vol[f], ok ? 8 : 0);
-      }
+    const int E = (red[0] == -100000 ? 0 : red[0]) + ((sd.xf[f] & 3) ? 1 : 0);
+    a.e3[3 * tl + f] = E;
+    // one or two flavours: es holds their exponents; three: each component carries all three once
+    if (nf <= 2) {
+      a.es[2 * tl + f] = E;
+      if (nf == 1) a.es[2 * tl + 1] = 0;
+    } else if (f < 2) {
+      a.es[2 * tl + f] = 0;
     }
   }
-  cp_async_commit();
+}
+// three flavours: the sum of the view exponents (after k_sample_udsc)
+__global__ void k_sum_udsc(const UdscArgs a) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < a.ntau) a.es[2 * t] = a.e3[3 * t] + a.e3[3 * t + 1] + a.e3[3 * t + 2];
 }
 
-template <typename Tin>
-__global__ void __launch_bounds__(kThreadsU, 1) k_contract_udsc_f32(const UdscArgsF32 a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Cx<Tin>* st = (Cx<Tin>*)smem_raw;
-  Cx<float>* sf = (Cx<float>*)(smem_raw + 3 * 144 * kSitesU * sizeof(Cx<Tin>));
-  int* smx = (int*)(sf + kSitesU * kRowU32);  // [kMaxDs] maxima of the current slice
-  const int tid = threadIdx.x;
-  const int hw = tid >> 4, l = tid & 15;
-  const unsigned mask = halfwarp_mask();
-  const int tiles_per_tau = (a.V3 + kSitesU - 1) / kSitesU;
-  TileCursor tc(blockIdx.x, gridDim.x, tiles_per_tau);
-  const int* stream0 = a.plan + a.plan[l];
-  if (tid < kMaxDs) smx[tid] = 0;
-
-  issue_tile_u32<Tin>(a, st, tc, a.ntau);
-  int cur = -1;
-  for (; tc.tl < a.ntau; tc = tc.next()) {
-    const int tl = tc.tl;
-    cp_async_wait<0>();
-    __syncthreads();
-    if (tl != cur) {
-      if (cur >= 0 && tid < a.nd) {
-        atomicMax(a.cmax + (long long)cur * a.nd + tid, smx[tid]);
-        smx[tid] = 0;
-      }
-      cur = tl;
-    }
-    // scale, transform and convert: thread (site s, transform groups
-    // q = c0 + 16 j of 108: 36 per view) -> the site's FP32 row
-    {
-      const UdscSlice& sd = a.sl[tl];
-      const int s = tid & (kSitesU - 1), c0 = tid >> 4;
-      Cx<float>* row = sf + s * kRowU32;
-#pragma unroll
-      for (int j = 0; j < 7; j++) {
-        const int q = c0 + 16 * j;
-        if (q < 108) {
-          const int f = q / 36;
-          const double sc = ldexp(1.0, -a.e3[3 * tl + f]);
-          int b, cc;
-          prop_group_base(q - 36 * f, b, cc);
-          const Cx<Tin>* src = st + (144 * f + 9 * b + cc) * kSitesU + s;
-          Cx<double> v[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const Cx<Tin> x = src[9 * group_blk(i) * kSitesU];
-            v[i] = cx<double>((double)x.x, (double)x.y);
-          }
-          prop_group_transform(v[0], v[1], v[2], v[3], sd.xf[f]);
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-            row[2 * row32_unit(16 * f + b + group_blk(i), cc >> 1) + (cc & 1)] =
-                cx<float>((float)(v[i].x * sc), (float)(v[i].y * sc));
-        }
-      }
-    }
-    __syncthreads();
-    issue_tile_u32<Tin>(a, st, tc.next(), a.ntau);
-    const int x = tc.x0() + hw;
-    if (x < a.V3) {
-      const RowF32 row{sf + hw * kRowU32};
-      Cx<float> acc[kMaxDs];
-#pragma unroll
-      for (int d = 0; d < kMaxDs; d++) acc[d] = czero<float>();
-      const int* q = stream0;
-      const int ntup = *q++;
-#pragma unroll 1
-      for (int t = 0; t < ntup; t++) {
-        const int head = q[0];
-        const unsigned cnt[4] = {(unsigned)q[1], (unsigned)q[2], (unsigned)q[3], (unsigned)q[4]};
-        q += 5;
-        Cx<float> g[9];
-#pragma unroll
-        for (int i = 0; i < 9; i++) g[i] = czero<float>();
-        diquark_acc(row, head & 255, (head >> 8) & 255, 0, 0, 1.f, 0, 0, g);
-#pragma unroll
-        for (int d = 0; d < kMaxDs; d++) {
-          if (d >= a.nd) break;
-          const int n = (int)((cnt[d >> 2] >> (8 * (d & 3))) & 255u);
-#pragma unroll 1
-          for (int e = 0; e < n; e++) {
-            const int blk = q[0];
-            const Cx<float> w = cx<float>(__int_as_float(q[1]), __int_as_float(q[2]));
-            q += 3;
-            Cx<float> z[9];
-            row.load9(blk, z);
-            Cx<float> dot = czero<float>();
-#pragma unroll
-            for (int i = 0; i < 9; i++) cmac(dot, g[i], z[i]);
-            cmac(acc[d], w, dot);
-          }
-        }
-      }
-      Cx<float>* o = a.out + (long long)tl * a.nd * a.V3 + x;
-      if (a.nd > 4) {
-        const Cx<float> v = reduce_scatter16(acc, l, mask);
-        if (l < a.nd) {
-          o[(long long)l * a.V3] = v;
-          atomicMax(smx + l, __float_as_int(fmaxf(fabsf(v.x), fabsf(v.y))));
-        }
-      } else {
-#pragma unroll
-        for (int d = 0; d < 4; d++) {
-          if (d >= a.nd) break;
-          Cx<float> v = acc[d];
-          v = v + shfl_xor16(v, 1, mask);
-          v = v + shfl_xor16(v, 2, mask);
-          v = v + shfl_xor16(v, 4, mask);
-          v = v + shfl_xor16(v, 8, mask);
-          if (l == d) {
-            o[(long long)d * a.V3] = v;
-            atomicMax(smx + d, __float_as_int(fmaxf(fabsf(v.x), fabsf(v.y))));
-          }
-        }
-      }
-    }
-  }
-  cp_async_wait<0>();
-  __syncthreads();
-  if (cur >= 0 && tid < a.nd) atomicMax(a.cmax + (long long)cur * a.nd + tid, smx[tid]);
-}
-
-template <typename Tin>
-cudaError_t launch_udsc_split_t(const UdscArgsF32& a, int grid, cudaStream_t s) {
-  k_sample_udsc<Tin><<<a.ntau, 256, 0, s>>>(a);
-  cudaError_t e = cudaGetLastError();
+template <typename R, typename Tin, int NF>
+cudaError_t launch_udsc_t(const UdscArgs& a, int nsm, cudaStream_t s) {
+  int nd = 0;
+  for (int p = 0; p < a.nprog; p++) nd = std::max(nd, a.prog[p].nd);
+  const int smem = udsc_smem<R, NF>(a.nprog, nd);
+  cudaError_t e = ensure_smem((const void*)k_contract_udsc<R, Tin, NF>, smem);
   if (e != cudaSuccess) return e;
-  const int smem = 3 * 144 * kSitesU * (int)sizeof(Cx<Tin>) + kSitesU * kRowU32 * (int)sizeof(Cx<float>) + 64;
-  e = ensure_smem((const void*)k_contract_udsc_f32<Tin>, smem);
-  if (e != cudaSuccess) return e;
-  k_contract_udsc_f32<Tin><<<grid, kThreadsU, smem, s>>>(a);
+  const long long tiles = (long long)((a.V3 + kSitesU - 1) / kSitesU) * a.ntau;
+  const int grid = (int)std::min<long long>(tiles, (long long)nsm * (sizeof(R) == 4 ? 2 : 1));
+  k_contract_udsc<R, Tin, NF><<<grid, kThreadsU, smem, s>>>(a);
   return cudaGetLastError();
 }
 
-// Per-lane instruction streams of one flavour product (see the file comment).
-std::vector<int> build_plan(int prod) {
-  const int d0 = kUdscDsBegin[prod], nd = kUdscDsBegin[prod + 1] - d0;
-  // distinct (P1 block, P2 block) tuples in first-occurrence order, and per
-  // tuple and dataset its entries (P3 block, weight)
-  std::map<int, int> tix;
-  std::vector<int> key;
-  std::vector<std::vector<std::vector<int>>> ent;  // [tuple][dataset] -> (blk, wre bits, wim bits)...
-  for (int d = 0; d < nd; d++)
-    for (int e = kUdscEntBegin[d0 + d]; e < kUdscEntBegin[d0 + d + 1]; e++) {
-      const signed char* m = kUdscIdx[e];
-      const int k = (m[0] * 4 + m[1]) | ((16 + m[2] * 4 + m[3]) << 8);
-      auto it = tix.find(k);
-      int t;
-      if (it == tix.end()) {
-        t = (int)key.size();
-        tix[k] = t;
-        key.push_back(k);
-        ent.emplace_back(nd);
-      } else {
-        t = it->second;
-      }
-      int wb[2];
-      std::memcpy(wb, kUdscVal[e], sizeof(wb));
-      auto& v = ent[t][d];
-      v.push_back(32 + m[4] * 4 + m[5]);
-      v.push_back(wb[0]);
-      v.push_back(wb[1]);
-    }
-  // balance: largest tuples first, each to the least loaded lane (cost in
-  // complex products: 36 for G, 9 per entry)
-  const int nt = (int)key.size();
-  std::vector<int> cost(nt), order(nt);
-  for (int t = 0; t < nt; t++) {
-    int n = 0;
-    for (const auto& v : ent[t]) n += (int)v.size() / 3;
-    cost[t] = 36 + 9 * n;
-  }
-  std::iota(order.begin(), order.end(), 0);
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-  std::vector<std::vector<int>> lane(16);
-  std::vector<int> load(16, 0);
-  for (int t : order) {
-    const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-    lane[l].push_back(t);
-    load[l] += cost[t];
-  }
-  std::vector<int> plan(16, 0);
-  for (int l = 0; l < 16; l++) {
-    plan[l] = (int)plan.size();
-    plan.push_back((int)lane[l].size());
-    for (int t : lane[l]) {
-      plan.push_back(key[t]);
-      unsigned cnt[4] = {0, 0, 0, 0};
-      for (int d = 0; d < nd; d++) cnt[d >> 2] |= (unsigned)(ent[t][d].size() / 3) << (8 * (d & 3));
-      for (int i = 0; i < 4; i++) plan.push_back((int)cnt[i]);
-      for (int d = 0; d < nd; d++) plan.insert(plan.end(), ent[t][d].begin(), ent[t][d].end());
-    }
-  }
-  return plan;
+cudaError_t launch_contract_udsc(const UdscArgs& a, int nf, int nsm, cudaStream_t s) {
+  return nf == 1   ? launch_udsc_t<double, double, 1>(a, nsm, s)
+         : nf == 2 ? launch_udsc_t<double, double, 2>(a, nsm, s)
+                   : launch_udsc_t<double, double, 3>(a, nsm, s);
+}
+
+template <typename Tin>
+cudaError_t launch_udsc_split_t(const UdscArgs& a, int nf, int nsm, cudaStream_t s) {
+  k_sample_udsc<Tin><<<dim3(a.ntau, nf), 256, 0, s>>>(a, nf);
+  if (nf == 3) k_sum_udsc<<<(a.ntau + 255) / 256, 256, 0, s>>>(a);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  return nf == 1   ? launch_udsc_t<float, Tin, 1>(a, nsm, s)
+         : nf == 2 ? launch_udsc_t<float, Tin, 2>(a, nsm, s)
+                   : launch_udsc_t<float, Tin, 3>(a, nsm, s);
 }
 
 // Products a request runs, in the reference's order and with its filters
@@ -516,13 +439,28 @@ int prop_of(const p2_udsc_request& r, char f) {
 }  // namespace
 }  // namespace p2
 
+// Flavour products of a request that run in one launch: same one or two
+// flavours (a product of a single flavour joins a pair with it when both hold
+// the same slices), or one product of three.
+namespace p2 {
+namespace {
+struct UdscGroup {
+  std::string flavours;     // distinct, in the order u d s c
+  std::vector<int> prods;
+  std::vector<int> ds_off;  // first dataset of each product in the result
+  std::vector<int> taus;    // local slices held by all the views
+  std::vector<UdscSlice> sl;
+  int K = 0;                // datasets of the group
+  size_t o_sl = 0, o_desc = 0, o_kexp = 0;  // byte offsets in the call's upload
+};
+}  // namespace
+}  // namespace p2
+
 struct p2_udsc_cache {
-  std::vector<p2host::DevBuf> plan;  // per product, built on first use
-  p2host::DevBuf slices, desc;
-  p2host::DevBuf e3, es, kexp;  // split form: view exponents, un-scaling exponents, component multiplicities
+  p2host::DevBuf args;    // slices, descriptors and component multiplicities of a call's groups
+  p2host::DevBuf e3, es;  // split form: view exponents, un-scaling exponents
   ~p2_udsc_cache() {
-    for (auto& b : plan) b.release();
-    for (p2host::DevBuf* b : {&slices, &desc, &e3, &es, &kexp}) b->release();
+    for (p2host::DevBuf* b : {&args, &e3, &es}) b->release();
   }
 };
 
@@ -593,7 +531,6 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
   if (todo.empty()) return P2_OK;
   if (!c->udsc) c->udsc = new p2_udsc_cache();
   p2_udsc_cache& U = *c->udsc;
-  if (U.plan.empty()) U.plan.resize(kUdscProducts);
 
   double* dres = r->out;
   if (r->out_location == P2_HOST) {
@@ -601,8 +538,11 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
     P2_TRY(c, cudaMemsetAsync(c->res.p, 0, total * 16, c->stream), "result clear");
     dres = (double*)c->res.p;
   }
+  const AxesPlan* ap = nullptr;  // the axis-by-axis projection, when the list qualifies
+  // (an armed p2_debug_wait_timeout asks for the tensor-core projection)
+  if (!(split && c->wait_test) && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
   int nmtile = 0, nkstep = 0;
-  if (split) {
+  if (split && !ap) {
     if (c->project_split_smem_max < project_split_smem_bytes(project_split_max_nt()))
       return c->fail(P2_ERR_UNSUPPORTED, "device shared memory per block too small for the tensor-core projection");
     if (!c->errflag.p) {
@@ -610,14 +550,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
       P2_TRY(c, cudaMemsetAsync(c->errflag.p, 0, 16, c->stream), "error flag clear");
     }
     if ((st = split_prepare_tables(c, pl, 0, nmtile, nkstep)) != P2_OK) return st;
-    if (!U.kexp.p) {  // every dataset carries each of its three views once: (1, 0) against es
-      std::vector<int> ke(2 * kMaxDs, 0);
-      for (int k = 0; k < kMaxDs; k++) ke[2 * k] = 1;
-      if ((st = upload_async(c, U.kexp, ke.data(), ke.size() * sizeof(int), "udsc exponents")) != P2_OK) return st;
-    }
   }
-  const AxesPlan* ap = nullptr;  // the axis-by-axis projection, when the list qualifies
-  if (!split && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
   // phase tables (origin 0; the scatter applies the source phase)
   if (!split && !ap && c->plain_moms_key != pl.moms) {
     c->plain_moms_key.clear();
@@ -628,182 +561,167 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
       return st;
     c->plain_moms_key = pl.moms;
   }
+
+  // groups of products
   const int T = c->T, tl0 = c->g.coords[3] * c->Ll[3];
-  int ds_off = 0;
-  for (int p : todo) {
-    const int nd = kUdscDsBegin[p + 1] - kUdscDsBegin[p];
-    if (!U.plan[p].p) {
-      const std::vector<int> plan = build_plan(p);
-      if ((st = upload_async(c, U.plan[p], plan.data(), plan.size() * sizeof(int), "udsc plan")) != P2_OK) return st;
-    }
-    const p2_prop* v[3];
-    for (int k = 0; k < 3; k++) v[k] = &props[prop_of(*r, kUdscProduct[p][k])];
-    // local slices held by all three views
-    std::vector<int> taus;
-    std::vector<UdscSlice> sl;
+  std::vector<UdscGroup> groups;
+  auto slices_of = [&](const std::string& fl, UdscGroup& g) {
     for (int tau = 0; tau < r->totalT; tau++) {
       const int t = (r->source[3] + tau) % T;
       if (t < tl0 || t >= tl0 + c->Ll[3]) continue;
       UdscSlice s{};
       bool ok = true;
-      for (int k = 0; k < 3; k++) {
-        const int j = ((t - v[k]->t_first) % T + T) % T;
-        ok &= j < v[k]->nt;
+      for (size_t k = 0; k < fl.size(); k++) {
+        const p2_prop& v = props[prop_of(*r, fl[k])];
+        const int j = ((t - v.t_first) % T + T) % T;
+        ok &= j < v.nt;
         s.off[k] = (long long)j * c->V3;
-        s.xf[k] = prop_xf_code(*v[k], t);
+        s.xf[k] = prop_xf_code(v, t);
       }
       if (!ok) continue;
-      taus.push_back(tau);
-      sl.push_back(s);
+      g.taus.push_back(tau);
+      g.sl.push_back(s);
     }
-    const int n_all = (int)taus.size();
-    if (split) {
-      const bool f32 = v[0]->precision == P2_FP32;
-      const size_t per32 = (size_t)nd * c->V3 * 8;
-      const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per32, 1), (size_t)T));
-      for (int c0 = 0; c0 < n_all; c0 += tc) {
-        const int n = std::min(tc, n_all - c0);
-        P2_TRY(c, c->cbuf.ensure((size_t)n * per32), "position buffer alloc");
-        P2_TRY(c, c->cmaxb.ensure((size_t)n * nd * sizeof(int)), "maxima alloc");
-        P2_TRY(c, cudaMemsetAsync(c->cmaxb.p, 0, (size_t)n * nd * sizeof(int), c->stream), "maxima clear");
-        P2_TRY(c, U.e3.ensure((size_t)n * 3 * sizeof(int)), "exponent alloc");
-        P2_TRY(c, U.es.ensure((size_t)n * 2 * sizeof(int)), "exponent alloc");
-        P2_TRY(c, U.slices.ensure((size_t)n * sizeof(UdscSlice)), "slice alloc");
-        P2_TRY(c,
-               cudaMemcpyAsync(U.slices.p, sl.data() + c0, (size_t)n * sizeof(UdscSlice), cudaMemcpyHostToDevice,
-                               c->stream),
-               "slice upload");
-        std::vector<SliceDesc> desc(n);
-        for (int i = 0; i < n; i++) {
-          std::memset(&desc[i], 0, sizeof(SliceDesc));
-          desc[i].out = dres;
-          desc[i].tau = taus[c0 + i];
-          desc[i].totalT = r->totalT;
-          for (int d = 0; d < 3; d++) desc[i].x0[d] = r->source[d];
-        }
-        P2_TRY(c, U.desc.ensure((size_t)n * sizeof(SliceDesc)), "descriptor alloc");
-        P2_TRY(c,
-               cudaMemcpyAsync(U.desc.p, desc.data(), (size_t)n * sizeof(SliceDesc), cudaMemcpyHostToDevice,
-                               c->stream),
-               "descriptor upload");
-        UdscArgsF32 a{};
-        for (int k = 0; k < 3; k++) {
-          a.p[k] = v[k]->data;
-          a.vol[k] = c->V3 * v[k]->nt;
-        }
-        a.sl = (const UdscSlice*)U.slices.p;
-        a.ntau = n;
-        a.V3 = (int)c->V3;
-        a.nd = nd;
-        a.plan = (const int*)U.plan[p].p;
-        a.e3 = (int*)U.e3.p;
-        a.es = (int*)U.es.p;
-        a.out = (Cx<float>*)c->cbuf.p;
-        a.cmax = (int*)c->cmaxb.p;
-        {
-          ProfScope ps(c, "contract_udsc_f32");
-          P2_TRY(c, f32 ? launch_udsc_split_t<float>(a, c->nsm, c->stream) : launch_udsc_split_t<double>(a, c->nsm, c->stream),
-                 "udsc split contraction");
-        }
-        const std::vector<ScatterBlock> blocks{ScatterBlock{0, 1, nd, 1, (long long)ds_off}};
-        if ((st = split_project(c, pl, nd, n, nmtile, nkstep, (const SliceDesc*)U.desc.p, (const int*)U.es.p,
-                                (const int*)U.kexp.p, blocks)) != P2_OK)
-          return st;
+  };
+  int ds_off = 0;
+  std::vector<int> offs;
+  for (int p : todo) {
+    offs.push_back(ds_off);
+    ds_off += kUdscDsBegin[p + 1] - kUdscDsBegin[p];
+  }
+  for (int pass = 0; pass < 2; pass++)  // products of a single flavour join a pair's group, so they come second
+    for (size_t i = 0; i < todo.size(); i++) {
+      const std::string f = kUdscProduct[todo[i]];
+      UdscGroup g;
+      for (char q : std::string("udsc"))
+        if (f.find(q) != std::string::npos) g.flavours += q;
+      if ((g.flavours.size() == 1) != (pass == 1)) continue;
+      slices_of(g.flavours, g);
+      if (g.taus.empty()) continue;
+      UdscGroup* to = nullptr;
+      for (UdscGroup& h : groups)
+        if (!to && (int)h.prods.size() < kMaxProgs && h.taus == g.taus &&
+            (h.flavours == g.flavours ||
+             (pass == 1 && h.flavours.size() == 2 && h.flavours.find(g.flavours) != std::string::npos)))
+          to = &h;
+      if (!to) {
+        groups.push_back(g);
+        to = &groups.back();
       }
-      ds_off += nd;
-      continue;
+      to->prods.push_back(todo[i]);
+      to->ds_off.push_back(offs[i]);
+      to->K += kUdscDsBegin[todo[i] + 1] - kUdscDsBegin[todo[i]];
     }
-    const size_t per = (size_t)nd * c->V3 * 16;
+  // one upload: the groups' slices, descriptors and, per component, how often
+  // it carries each of the launch's first two scales (three flavours: their
+  // summed scale once)
+  std::vector<unsigned char> up;
+  auto reserve = [&](size_t n) {
+    const size_t o = up.size();
+    up.resize(o + (n + 15) / 16 * 16, 0);
+    return o;
+  };
+  for (UdscGroup& g : groups) {
+    const size_t n = g.taus.size();
+    g.o_sl = reserve(n * sizeof(UdscSlice));
+    g.o_desc = reserve(n * sizeof(SliceDesc));
+    g.o_kexp = reserve(2 * (size_t)g.K * sizeof(int));
+    std::memcpy(&up[g.o_sl], g.sl.data(), n * sizeof(UdscSlice));
+    SliceDesc* desc = (SliceDesc*)&up[g.o_desc];
+    for (size_t i = 0; i < n; i++) {
+      desc[i].out = dres;
+      desc[i].tau = g.taus[i];
+      desc[i].totalT = r->totalT;
+      for (int d = 0; d < 3; d++) desc[i].x0[d] = r->source[d];
+    }
+    int* ke = (int*)&up[g.o_kexp];
+    for (int p : g.prods) {
+      const std::string f = kUdscProduct[p];
+      for (int d = kUdscDsBegin[p]; d < kUdscDsBegin[p + 1]; d++, ke += 2) {
+        if (g.flavours.size() == 3)
+          ke[0] = 1;
+        else
+          for (size_t k = 0; k < g.flavours.size(); k++)
+            ke[k] = (int)std::count(f.begin(), f.end(), g.flavours[k]);
+      }
+    }
+  }
+  if (!up.empty() && (st = upload_async(c, U.args, up.data(), up.size(), "udsc arguments")) != P2_OK) return st;
+
+  for (const UdscGroup& g : groups) {
+    const int nf = (int)g.flavours.size(), K = g.K, n_all = (int)g.taus.size();
+    UdscArgs a{};
+    for (int k = 0; k < nf; k++) {
+      const p2_prop& v = props[prop_of(*r, g.flavours[k])];
+      a.p[k] = v.data;
+      a.vol[k] = c->V3 * v.nt;
+    }
+    const bool f32 = props[prop_of(*r, g.flavours[0])].precision == P2_FP32;
+    a.V3 = (int)c->V3;
+    a.K = K;
+    a.nprog = (int)g.prods.size();
+    std::vector<ScatterBlock> blocks;
+    int k0 = 0;
+    for (int i = 0; i < a.nprog; i++) {
+      const int p = g.prods[i], nd = kUdscDsBegin[p + 1] - kUdscDsBegin[p];
+      std::memcpy(a.prog[i].start, kUdscProgramStart[kUdscProgram[p]], sizeof(a.prog[i].start));
+      a.prog[i].nd = nd;
+      a.prog[i].k0 = k0;
+      // a program's blocks count from its own first flavour
+      size_t first = nf;
+      for (char q : std::string(kUdscProduct[p])) first = std::min(first, g.flavours.find(q));
+      a.prog[i].boff = 16 * (int)first;
+      blocks.push_back(ScatterBlock{k0, 1, nd, 1, (long long)g.ds_off[i]});
+      k0 += nd;
+    }
+    const size_t per = (size_t)K * c->V3 * (split ? 8 : 16);
     const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)T));
     for (int c0 = 0; c0 < n_all; c0 += tc) {
       const int n = std::min(tc, n_all - c0);
+      const SliceDesc* dsl = (const SliceDesc*)((const unsigned char*)U.args.p + g.o_desc) + c0;
+      const int* kexp = (const int*)((const unsigned char*)U.args.p + g.o_kexp);
       P2_TRY(c, c->cbuf.ensure((size_t)n * per), "position buffer alloc");
-      P2_TRY(c, U.slices.ensure((size_t)n * sizeof(UdscSlice)), "slice alloc");
-      P2_TRY(c,
-             cudaMemcpyAsync(U.slices.p, sl.data() + c0, (size_t)n * sizeof(UdscSlice), cudaMemcpyHostToDevice,
-                             c->stream),
-             "slice upload");
-      UdscArgs a{};
-      a.p0 = (const Cx<double>*)v[0]->data;
-      a.p1 = (const Cx<double>*)v[1]->data;
-      a.p2 = (const Cx<double>*)v[2]->data;
-      a.vol0 = c->V3 * v[0]->nt;
-      a.vol1 = c->V3 * v[1]->nt;
-      a.vol2 = c->V3 * v[2]->nt;
-      a.sl = (const UdscSlice*)U.slices.p;
+      a.sl = (const UdscSlice*)((const unsigned char*)U.args.p + g.o_sl) + c0;
       a.ntau = n;
-      a.V3 = (int)c->V3;
-      a.nd = nd;
-      a.plan = (const int*)U.plan[p].p;
-      a.out = (Cx<double>*)c->cbuf.p;
-      {
+      a.out = c->cbuf.p;
+      if (split) {
+        P2_TRY(c, U.e3.ensure((size_t)n * 3 * sizeof(int)), "exponent alloc");
+        P2_TRY(c, U.es.ensure((size_t)n * 2 * sizeof(int)), "exponent alloc");
+        a.e3 = (int*)U.e3.p;
+        a.es = (int*)U.es.p;
+        if (!ap) {
+          P2_TRY(c, c->cmaxb.ensure((size_t)n * K * sizeof(int)), "maxima alloc");
+          P2_TRY(c, cudaMemsetAsync(c->cmaxb.p, 0, (size_t)n * K * sizeof(int), c->stream), "maxima clear");
+          a.cmax = (int*)c->cmaxb.p;
+        }
+        ProfScope ps(c, "contract_udsc_f32");
+        P2_TRY(c,
+               f32 ? launch_udsc_split_t<float>(a, nf, c->nsm, c->stream)
+                   : launch_udsc_split_t<double>(a, nf, c->nsm, c->stream),
+               "udsc split contraction");
+      } else {
         ProfScope ps(c, "contract_udsc_fp64");
-        P2_TRY(c, launch_contract_udsc(a, c->nsm, c->stream), "udsc contraction");
+        P2_TRY(c, launch_contract_udsc(a, nf, c->nsm, c->stream), "udsc contraction");
       }
-      std::vector<SliceDesc> desc(n);
-      for (int i = 0; i < n; i++) {
-        std::memset(&desc[i], 0, sizeof(SliceDesc));
-        desc[i].out = dres;
-        desc[i].tau = taus[c0 + i];
-        desc[i].totalT = r->totalT;
-        for (int d = 0; d < 3; d++) desc[i].x0[d] = r->source[d];
-      }
-      P2_TRY(c, U.desc.ensure((size_t)n * sizeof(SliceDesc)), "descriptor alloc");
-      P2_TRY(c,
-             cudaMemcpyAsync(U.desc.p, desc.data(), (size_t)n * sizeof(SliceDesc), cudaMemcpyHostToDevice,
-                             c->stream),
-             "descriptor upload");
       if (ap) {
-        P2_TRY(c, c->axes_s1.ensure((size_t)n * c->Ll[1] * c->Ll[2] * ap->R1 * nd * 16), "projection workspace");
-        if ((st = axes_x(c, *ap, c->cbuf.p, 0, (long long)nd * c->V3, c->V3, n, nd, c->axes_s1.p)) != P2_OK) return st;
-        const std::vector<ScatterBlock> blocks{ScatterBlock{0, 1, nd, 1, (long long)ds_off}};
+        P2_TRY(c, c->axes_s1.ensure((size_t)n * c->Ll[1] * c->Ll[2] * ap->R1 * K * (split ? 8 : 16)),
+               "projection workspace");
+        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, c->axes_s1.p)) != P2_OK)
+          return st;
         AxesOut ao;
-        ao.dsl = (const SliceDesc*)U.desc.p;
+        ao.dsl = dsl;
         ao.blocks = &blocks;
-        if ((st = axes_yz(c, *ap, c->axes_s1.p, 0, n, nd, ao)) != P2_OK) return st;
-        continue;
-      }
-      ProjArgs pa{};
-      pa.c = c->cbuf.p;
-      pa.sT = (long long)nd * c->V3;
-      pa.sK = c->V3;
-      pa.ntau = n;
-      pa.K = nd;
-      pa.V3 = (int)c->V3;
-      pa.nmom = pl.nmom;
-      pa.Lx = c->Ll[0];
-      pa.Ly = c->Ll[1];
-      pa.Lz = c->Ll[2];
-      pa.Lmax = pl.Lmax;
-      pa.tab = (const double*)c->ptab.p;
-      const int ptiles = (pl.nmom + 63) / 64, ktiles = (nd + 31) / 32;
-      int nsplit = (2 * c->nsm + ptiles * ktiles * n - 1) / (ptiles * ktiles * n);
-      nsplit = std::max(1, std::min(nsplit, (int)((c->V3 + 255) / 256)));
-      pa.chunk = (int)((((c->V3 + nsplit - 1) / nsplit) + 15) / 16 * 16);
-      pa.nsplit = (int)((c->V3 + pa.chunk - 1) / pa.chunk);
-      P2_TRY(c, c->part.ensure((size_t)n * pa.nsplit * pl.nmom * nd * 16), "partials alloc");
-      pa.part = (double*)c->part.p;
-      {
-        ProfScope ps(c, "project_fp64");
-        P2_TRY(c, launch_project_fp64(pa, c->stream), "projection kernel");
-      }
-      ScatterArgs sa{};
-      sa.part = (const double*)c->part.p;
-      sa.ntau = n;
-      sa.nsplit = pa.nsplit;
-      sa.nmom = pl.nmom;
-      sa.K = nd;
-      sa.nblocks = 1;
-      sa.blk[0] = ScatterBlock{0, 1, nd, 1, (long long)ds_off};
-      sa.sl = (const SliceDesc*)U.desc.p;
-      sa.moms = (const int*)c->moms.p;
-      for (int d = 0; d < 3; d++) sa.L[d] = c->g.L[d];
-      {
-        ProfScope ps(c, "reduce_scatter");
-        P2_TRY(c, launch_scatter(sa, c->stream), "reduction kernel");
+        if (split) {
+          ao.exps = a.es;
+          ao.kexp = kexp;
+        }
+        if ((st = axes_yz(c, *ap, c->axes_s1.p, split, n, K, ao)) != P2_OK) return st;
+      } else if (split) {
+        if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, a.es, kexp, blocks)) != P2_OK) return st;
+      } else if ((st = project_direct(c, pl, K, n, n, dsl, blocks)) != P2_OK) {
+        return st;
       }
     }
-    ds_off += nd;
   }
   if (r->out_location == P2_HOST) {
     P2_TRY(c, cudaMemcpyAsync(r->out, dres, total * 16, cudaMemcpyDeviceToHost, c->stream), "result download");

@@ -243,6 +243,132 @@ def table_digest(idx, vals) -> str:
     return hashlib.sha256(repr(rows).encode()).hexdigest()[:16]
 
 
+#: Warps that share a site program (udsc.cu)
+PROGRAM_WARPS = 8
+
+
+def site_program(flavours, datasets):
+    """Contraction program of one flavour product, see udsc.cu.
+
+    Every term w eps eps' P1[b1] P2[b2] P3[b3] (b = spin block) is symmetric
+    under exchange of equal flavours together with their blocks, so terms that
+    differ by such an exchange are merged and each distinct triple of
+    (flavour, block) is evaluated once for all datasets.  A triple is a
+    diquark of two of its members dotted with the third; the diquarks are a
+    greedy cover of the triples (each covers as many of those left as any
+    other), so few of them are built.
+
+    Returns (distinct flavours, per-warp lists of
+    (A, [(B, [(Z, [(dataset, weight)])])])): the diquark of blocks A and B, its
+    dots with blocks Z, and what each dot adds to the datasets; block
+    16 slot + b, slot the index among the distinct flavours."""
+    slots = sorted(set(flavours), key="udsc".index)
+    weights: Dict[tuple, Dict[int, float]] = {}
+    for d, (_, tuples, ws) in enumerate(datasets):
+        for t, w in zip(tuples, ws):
+            if abs(np.imag(w)) > 1e-12:
+                raise ValueError("complex table weight")
+            key = tuple(sorted(16 * slots.index(f) + 4 * t[2 * i] + t[2 * i + 1] for i, f in enumerate(flavours)))
+            row = weights.setdefault(key, {})
+            row[d] = row.get(d, 0.0) + float(np.real(w))
+    triples = [k for k, row in weights.items() if any(abs(w) > 1e-9 for w in row.values())]
+    # greedy cover: pairs of each triple, with the triples left to cover
+    def pairs(t):
+        return {(t[0], t[1]), (t[0], t[2]), (t[1], t[2])}
+
+    def third(t, p):
+        rest = list(t)
+        for b in p:
+            rest.remove(b)
+        return rest[0]
+    left: Dict[tuple, set] = {}
+    for t in triples:
+        for p in pairs(t):
+            left.setdefault(p, set()).add(t)
+    cover: Dict[tuple, list] = {}
+    while any(left.values()):
+        best = max(sorted(left), key=lambda p: len(left[p]))
+        cover[best] = sorted(left[best])
+        for t in cover[best]:
+            for p in pairs(t):
+                left[p].discard(t)
+    # pairs that share a block become neighbours, so a warp loads that block once
+    degree: Dict[int, int] = {}
+    for p in cover:
+        for b in set(p):
+            degree[b] = degree.get(b, 0) + 1
+    steps = []
+    for p, ts in cover.items():
+        a, b = p if degree[p[0]] >= degree[p[1]] else (p[1], p[0])
+        dots = [(third(t, p), sorted((d, w) for d, w in weights[t].items() if abs(w) > 1e-9)) for t in ts]
+        steps.append((a, b, dots))
+    steps.sort(key=lambda q: (q[0], q[1]))
+    cost = [36 + sum(9 + 2 * len(e) for _, e in dots) for _, _, dots in steps]
+    # contiguous ranges of equal cost (smallest largest range, by bisection)
+    def ranges(limit):
+        out, acc = [[]], 0
+        for i, c in enumerate(cost):
+            if acc + c > limit and out[-1]:
+                out.append([])
+                acc = 0
+            out[-1].append(i)
+            acc += c
+        return out
+    lo, hi = max(cost), sum(cost)
+    while lo < hi:
+        mid = (lo + hi) // 2
+        if len(ranges(mid)) <= PROGRAM_WARPS:
+            hi = mid
+        else:
+            lo = mid + 1
+    parts = ranges(lo)
+    parts += [[] for _ in range(PROGRAM_WARPS - len(parts))]
+    warps = []
+    for part in parts:
+        groups: List[tuple] = []
+        for i in part:
+            a, b, dots = steps[i]
+            if not groups or groups[-1][0] != a:
+                groups.append((a, []))
+            groups[-1][1].append((b, dots))
+        warps.append(groups)
+    return slots, warps
+
+
+def encode_programs(prods):
+    """(code, weights, program of each product, [(datasets, start of each warp's code)]): the site
+    programs as one stream of 16-bit words, equal programs stored once.  A warp's code is
+    nA, then per A: block, nB, then per B: block, ndots, then per dot: block, entries, then per
+    entry dataset | weight index << 4."""
+    code: List[int] = []
+    values: List[float] = []
+    programs, which, seen = [], [], {}
+    for flavours, datasets in prods:
+        _, warps = site_program(flavours, datasets)
+        ident = repr(warps)
+        if ident not in seen:
+            starts = []
+            for groups in warps:
+                starts.append(len(code))
+                code.append(len(groups))
+                for a, bs in groups:
+                    code += [a, len(bs)]
+                    for b, dots in bs:
+                        code += [b, len(dots)]
+                        for z, entries in dots:
+                            code += [z, len(entries)]
+                            for d, w in entries:
+                                if w not in values:
+                                    values.append(w)
+                                code.append(d | values.index(w) << 4)
+            seen[ident] = len(programs)
+            programs.append((len(datasets), starts))
+        which.append(seen[ident])
+    if len(values) >= 4096 or max(code) >= 65536:
+        raise ValueError("site program does not fit its encoding")
+    return code, values, which, programs
+
+
 def emit_header(path: str) -> bool:
     """C header with the tables (generated at build time); True if the file changed."""
     prods = products()
@@ -272,6 +398,15 @@ def emit_header(path: str) -> bool:
     for i in range(0, len(val), 8):
         L.append("  " + " ".join("{%.9ef,%.9ef}," % v for v in val[i:i + 8]))
     L.append("};")
+    code, values, which, programs = encode_programs(prods)
+    L += ["", f"constexpr int kUdscWarps = {PROGRAM_WARPS};",
+          "static const int kUdscProgram[kUdscProducts] = {" + ", ".join(map(str, which)) + "};",
+          f"static const int kUdscProgramStart[{len(programs)}][kUdscWarps] = {{" +
+          ", ".join("{" + ", ".join(map(str, st)) + "}" for _, st in programs) + "};",
+          f"constexpr int kUdscCodeWords = {len(code)};",
+          "#define P2_INIT_UDSC_CODE {" + ",".join(map(str, code)) + "}",
+          f"constexpr int kUdscWeights = {len(values)};",
+          "#define P2_INIT_UDSC_WEIGHTS {" + ",".join("%.17g" % v for v in values) + "}"]
     text = "\n".join(L) + "\n"
     try:
         with open(path) as f:
