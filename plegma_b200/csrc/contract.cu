@@ -551,68 +551,17 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
     for (int k = tid; k < a.K; k += kThreads) atomicMax(a.cmax + (long long)cur * a.K + k, *smax_slot(sf, k));
 }
 
-// Threads of the sampling kernel: the samples are scattered, so its time is
-// the number of rounds of loads in flight per thread (21504 samples, 8 per
-// thread and round).
-constexpr int kSampleThreads = 512;
-
-// Per-slice exponent E with max(|Re|,|Im|) < 2^E over a strided sample of
-// sites and components (every 7th component, every 97th site), so that the
-// scaled entries are O(1) in FP32.  Only the binary exponents are compared,
-// so FP64 entries far below FP32's range are handled exactly.
-__global__ void k_sample_exponents(const SampleArgs a) {
-  __shared__ int red[kSampleThreads];
+// Per-slice exponent E with max(|Re|,|Im|) < 2^E over a sample (sample_exponent),
+// so that the scaled entries are O(1) in FP32.  One block per (slice, flavour).
+__global__ void __launch_bounds__(kSampleThreads) k_sample_exponents(const SampleArgs a) {
   const int tl = blockIdx.x, f = blockIdx.y;
   const SliceDesc& sd = a.sl[tl];
   const void* p = f ? sd.d : sd.u;
-  const long long vol = f ? sd.vol_d : sd.vol_u;
-  const long long j = f ? sd.off_d : sd.off_u;
-  int emax = -100000;
-  // 8 independent loads in flight per thread (the samples are scattered, so
-  // each is a separate DRAM access)
-  constexpr int kSamples = 21 * 1024, kBatch = 8;
-  for (int i0 = threadIdx.x; i0 < kSamples; i0 += kBatch * blockDim.x) {
-    double re[kBatch], im[kBatch];
-#pragma unroll
-    for (int u = 0; u < kBatch; u++) {
-      const int i = i0 + u * blockDim.x;
-      re[u] = im[u] = 0.0;
-      if (i < kSamples) {
-        const int comp = (i % 21) * 7;
-        const long long x = ((long long)(i / 21) * 97) % a.V3;
-        const long long idx = (long long)comp * vol + j + x;
-        if (a.fp32) {
-          const float2 v = ((const float2*)p)[idx];
-          re[u] = v.x;
-          im[u] = v.y;
-        } else {
-          const double2 v = ((const double2*)p)[idx];
-          re[u] = v.x;
-          im[u] = v.y;
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kBatch; u++) {
-      int e;
-      if (re[u] != 0.0) {
-        frexp(re[u], &e);
-        emax = max(emax, e);
-      }
-      if (im[u] != 0.0) {
-        frexp(im[u], &e);
-        emax = max(emax, e);
-      }
-    }
-  }
-  red[threadIdx.x] = emax;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
+  const long long vol = f ? sd.vol_d : sd.vol_u, j = f ? sd.off_d : sd.off_u;
+  const int E = a.fp32 ? sample_exponent((const Cx<float>*)p + j, vol, a.V3)
+                       : sample_exponent((const Cx<double>*)p + j, vol, a.V3);
   // a rotation can double an entry: one more power of two of headroom
-  if (threadIdx.x == 0) a.exp_out[2 * tl + f] = (red[0] == -100000 ? 0 : red[0]) + ((sd.xf[f] & 3) ? 1 : 0);
+  if (threadIdx.x == 0) a.exp_out[2 * tl + f] = E + ((sd.xf[f] & 3) ? 1 : 0);
 }
 
 }  // namespace

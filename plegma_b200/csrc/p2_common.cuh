@@ -218,6 +218,41 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+// Exponent E with |Re|, |Im| < 2^E over a sample of one slice of a propagator
+// (21 components x 1024 sites: every 7th component, every 97th site), 0 for an
+// all-zero sample; every thread of a block of kSampleThreads gets it.
+// One site per thread with its 21 loads independent of one another, so the
+// time is a few memory latencies; only the exponent bits are compared
+// (infinities and NaNs are passed over).
+constexpr int kSampleThreads = 1024;
+__device__ __forceinline__ int sample_key(double v) {
+  const int b = __double2hiint(v) & 0x7fffffff;
+  return b >= 0x7ff00000 ? 0 : b;
+}
+__device__ __forceinline__ int sample_key(float v) {
+  const int b = __float_as_int(v) & 0x7fffffff;
+  return b >= 0x7f800000 ? 0 : b;
+}
+template <typename T>
+__device__ __forceinline__ int sample_exponent(const Cx<T>* p, long long vol, int V3) {
+  __shared__ int red[kSampleThreads / 32];
+  const Cx<T>* q = p + ((unsigned)threadIdx.x * 97u) % (unsigned)V3;
+  int m = 0;
+#pragma unroll
+  for (int c0 = 0; c0 < 21; c0 += 7) {
+    Cx<T> v[7];
+#pragma unroll
+    for (int c = 0; c < 7; c++) v[c] = q[(c0 + c) * 7 * vol];
+#pragma unroll
+    for (int c = 0; c < 7; c++) m = max(m, max(sample_key(v[c].x), sample_key(v[c].y)));
+  }
+  m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  m = (int)__reduce_max_sync(0xffffffffu, (unsigned)red[threadIdx.x & 31]);
+  return m == 0 ? 0 : sizeof(T) == 8 ? (m >> 20) - 1022 : (m >> 23) - 126;
+}
+
 // exp(i 2 pi sum_d p_d x0_d / L_d): the phase that moves a projection with
 // origin 0 to the source x0; each p_d x0_d is reduced mod L_d in integers.
 __device__ __forceinline__ Cx<double> source_phase(const int* p, const int* x0, const int* L) {

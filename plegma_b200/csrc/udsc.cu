@@ -48,11 +48,21 @@ namespace {
 
 constexpr int kThreadsU = 32 * kUdscWarps;
 constexpr int kSitesU = 32;  // sites of a tile, one per lane
-constexpr int kMaxDs = 16;   // datasets per product (the reference's largest product has 16)
+// datasets of a launch's largest product: 16 with three flavours, 10 with fewer
+template <int NF>
+constexpr int kMaxDs = NF == 3 ? 16 : 10;
 constexpr int kMaxProgs = 4; // products on one pair of flavours: aab, abb, aaa, bbb
 
-__constant__ unsigned short c_code[kUdscCodeWords] = P2_INIT_UDSC_CODE;
+__constant__ unsigned c_code[kUdscCodeWords] = P2_INIT_UDSC_CODE;
 __constant__ double c_weight[kUdscWeights] = P2_INIT_UDSC_WEIGHTS;
+__constant__ float c_weight32[kUdscWeights] = P2_INIT_UDSC_WEIGHTS;
+template <typename R>
+__device__ __forceinline__ R weight(int i) {
+  if constexpr (sizeof(R) == 8)
+    return c_weight[i];
+  else
+    return c_weight32[i];
+}
 
 struct UdscSlice {
   long long off[3];  // element offset of the slice inside each of the views
@@ -62,7 +72,7 @@ struct UdscSlice {
 
 // One flavour product of a launch.
 struct UdscProg {
-  int start[kUdscWarps];  // first word of each warp's code
+  int start[kUdscWarps];  // first record of each warp
   int nd, k0;             // datasets and their first component in the output
   int boff;               // added to the program's blocks (16 x the view of its first flavour)
 };
@@ -194,91 +204,80 @@ __device__ __forceinline__ void stage_tile(const UdscArgs& a, const SiteTile<flo
 }
 
 // G[c][e] = sum eps_abc eps_xye A[a][x] B[b][y]
-__device__ __forceinline__ void site_diquark(const Cx<double> (&a)[9], const Cx<double> (&b)[9], Cx<double> (&g)[9]) {
+template <typename R>
+__device__ __forceinline__ void site_diquark(const Cx<R> (&a)[9], const Cx<R> (&b)[9], Cx<R> (&g)[9]) {
 #pragma unroll
   for (int c = 0; c < 3; c++)
 #pragma unroll
     for (int e = 0; e < 3; e++) {
       const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, e1 = (e + 1) % 3, e2 = (e + 2) % 3;
-      Cx<double> r = cmul(a[c1 * 3 + e1], b[c2 * 3 + e2]);
+      Cx<R> r = cmul(a[c1 * 3 + e1], b[c2 * 3 + e2]);
       cmsub(r, a[c1 * 3 + e2], b[c2 * 3 + e1]);
       cmsub(r, a[c2 * 3 + e1], b[c1 * 3 + e2]);
       cmac(r, a[c2 * 3 + e2], b[c1 * 3 + e1]);
       g[c * 3 + e] = r;
     }
 }
-__device__ __forceinline__ void site_diquark(const Cx<float> (&a)[9], const Cx<float> (&b)[9], Cx<float> (&g)[9]) {
-  // paired FMAs: (a.x b.x, a.x b.y) and (a.y b.x, a.y b.y) accumulated separately
-  f32x2 bp[9], bn[9];
-#pragma unroll
-  for (int i = 0; i < 9; i++) {
-    bp[i] = f2pack(b[i].x, b[i].y);
-    bn[i] = f2pack(-b[i].x, -b[i].y);
-  }
-#pragma unroll
-  for (int c = 0; c < 3; c++)
-#pragma unroll
-    for (int e = 0; e < 3; e++) {
-      const int c1 = (c + 1) % 3, c2 = (c + 2) % 3, e1 = (e + 1) % 3, e2 = (e + 2) % 3;
-      f32x2 px = f2pack(0.f, 0.f), py = px;
-      auto term = [&](int ia, f32x2 bb) {
-        px = f2fma(f2pack(a[ia].x, a[ia].x), bb, px);
-        py = f2fma(f2pack(a[ia].y, a[ia].y), bb, py);
-      };
-      term(c1 * 3 + e1, bp[c2 * 3 + e2]);
-      term(c1 * 3 + e2, bn[c2 * 3 + e1]);
-      term(c2 * 3 + e1, bn[c1 * 3 + e2]);
-      term(c2 * 3 + e2, bp[c1 * 3 + e1]);
-      float xr, xi, yr, yi;
-      f2unpack(px, xr, xi);
-      f2unpack(py, yr, yi);
-      g[c * 3 + e] = cx<float>(xr - yi, xi + yr);
-    }
-}
 
-// This warp's part of a program on its lanes' sites.
+// This warp's part of a program on its lanes' sites, from record q (see
+// udsc.encode_programs) to the ending one.  A record comes from constant
+// memory an iteration before it is used.  A dot's datasets are one case of a
+// generated switch (one uniform branch per dot, the accumulators in
+// registers).
 template <typename R, int NF>
-__device__ __forceinline__ void run_program(const SiteTile<R, NF>& t, int q, int boff, Cx<R> (&acc)[kMaxDs]) {
-  const int na = c_code[q++];
+__device__ __forceinline__ void run_program(const SiteTile<R, NF>& t, int q, int boff, Cx<R> (&acc)[kMaxDs<NF>]) {
+  Cx<R> A[9], g[9];
+#pragma unroll
+  for (int i = 0; i < 9; i++) A[i] = g[i] = czero<R>();
+  unsigned rec = c_code[q], next = c_code[q + 1];
+  q += 2;  // two records follow the last program's end
+  auto advance = [&]() {
+    rec = next;
+    next = c_code[q++];
+  };
+  auto block = [&](unsigned r) { return (int)(r >> 2 & 63) + boff; };
 #pragma unroll 1
-  for (int ia = 0; ia < na; ia++) {
-    Cx<R> A[9];
-    t.load9(c_code[q] + boff, A);
-    const int nb = c_code[q + 1];
-    q += 2;
+  while ((rec & 3) != 3) {
+    if ((rec & 3) == 0) {
+      t.load9(block(rec), A);
+      advance();
+    }
+    {
+      Cx<R> B[9];
+      t.load9(block(rec), B);
+      advance();
+      site_diquark(A, B, g);
+    }
 #pragma unroll 1
-    for (int ib = 0; ib < nb; ib++) {
-      Cx<R> g[9];
-      {
-        Cx<R> B[9];
-        t.load9(c_code[q] + boff, B);
-        site_diquark(A, B, g);
+    while ((rec & 3) == 2) {
+      Cx<R> z[9];
+      t.load9(block(rec), z);
+      const int cs = (int)(rec >> 8 & 255), wi = (int)(rec >> 16);
+      advance();
+      // FP64 three, FP32 two partial sums: chains of dependent FMAs in flight
+      constexpr int NV = sizeof(R) == 8 ? 3 : 2;
+      Cx<R> vs[NV];
+#pragma unroll
+      for (int i = 0; i < 9; i++) {
+        if (i < NV)
+          vs[i] = cmul(g[i], z[i]);
+        else
+          cmac(vs[i % NV], g[i], z[i]);
       }
-      const int ndot = c_code[q + 1];
-      q += 2;
-#pragma unroll 1
-      for (int iz = 0; iz < ndot; iz++) {
-        Cx<R> z[9];
-        t.load9(c_code[q] + boff, z);
-        const int ne = c_code[q + 1];
-        q += 2;
-        const Cx<R> v = cdot9(g, z);
-#pragma unroll 1
-        for (int ie = 0; ie < ne; ie++) {
-          const int w = c_code[q++];
-          const R f = (R)c_weight[w >> 4];
-          switch (w & 15) {
-#define P2_ACC(i)                          \
-  case i:                                  \
-    acc[i].x = fma(f, v.x, acc[i].x);      \
-    acc[i].y = fma(f, v.y, acc[i].y);      \
-    break;
-            P2_ACC(0) P2_ACC(1) P2_ACC(2) P2_ACC(3) P2_ACC(4) P2_ACC(5) P2_ACC(6) P2_ACC(7)
-            P2_ACC(8) P2_ACC(9) P2_ACC(10) P2_ACC(11) P2_ACC(12) P2_ACC(13) P2_ACC(14) P2_ACC(15)
-#undef P2_ACC
-          }
-        }
+      Cx<R> v = vs[0] + vs[1];
+      if constexpr (NV == 3) v = v + vs[2];
+#define P2_ADD(d, i)                                   \
+  {                                                    \
+    const R f = weight<R>(wi + i);                     \
+    acc[d].x = fma(f, v.x, acc[d].x);                  \
+    acc[d].y = fma(f, v.y, acc[d].y);                  \
+  }
+      if constexpr (NF == 3) {
+        switch (cs) { P2_UDSC_CASES_16 }
+      } else {
+        switch (cs) { P2_UDSC_CASES_10 }
       }
+#undef P2_ADD
     }
   }
 }
@@ -311,13 +310,13 @@ __global__ void __launch_bounds__(kThreadsU, sizeof(R) == 4 ? 2 : 1) k_contract_
 #pragma unroll 1
     for (int p = 0; p < a.nprog; p++) {
       const UdscProg& pg = a.prog[p];
-      Cx<R> acc[kMaxDs];
+      Cx<R> acc[kMaxDs<NF>];
 #pragma unroll
-      for (int d = 0; d < kMaxDs; d++) acc[d] = czero<R>();
+      for (int d = 0; d < kMaxDs<NF>; d++) acc[d] = czero<R>();
       run_program(tile, pg.start[warp], pg.boff, acc);
       __syncthreads();  // the tile (single program) or the previous program's sums are read
 #pragma unroll
-      for (int d = 0; d < kMaxDs; d++)
+      for (int d = 0; d < kMaxDs<NF>; d++)
         if (d < pg.nd) red[(warp * pg.nd + d) * kSitesU + lane] = acc[d];
       __syncthreads();
       for (int d = warp; d < pg.nd; d += kUdscWarps) {
@@ -337,38 +336,15 @@ __global__ void __launch_bounds__(kThreadsU, sizeof(R) == 4 ? 2 : 1) k_contract_
   }
 }
 
-// Per slice and view the binary exponent of the largest of a strided sample
-// (every 7th component, every 97th site), plus one when the view is rotated.
-// One block per (slice, view).
+// Per slice and view the exponent of a sample (sample_exponent), plus one when
+// the view is rotated.  One block per (slice, view).
 template <typename Tin>
-__global__ void k_sample_udsc(const UdscArgs a, int nf) {
-  __shared__ int red[256];
+__global__ void __launch_bounds__(kSampleThreads) k_sample_udsc(const UdscArgs a, int nf) {
   const int tl = blockIdx.x, f = blockIdx.y;
   const UdscSlice& sd = a.sl[tl];
-  const Cx<Tin>* p = (const Cx<Tin>*)a.p[f] + sd.off[f];
-  int emax = -100000;
-  for (int i = threadIdx.x; i < 21 * 1024; i += blockDim.x) {
-    const int comp = (i % 21) * 7;
-    const long long x = ((long long)(i / 21) * 97) % a.V3;
-    const Cx<Tin> v = p[comp * a.vol[f] + x];
-    int e;
-    if (v.x != 0) {
-      frexp((double)v.x, &e);
-      emax = max(emax, e);
-    }
-    if (v.y != 0) {
-      frexp((double)v.y, &e);
-      emax = max(emax, e);
-    }
-  }
-  red[threadIdx.x] = emax;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = max(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
-  }
+  const int E0 = sample_exponent((const Cx<Tin>*)a.p[f] + sd.off[f], a.vol[f], a.V3);
   if (threadIdx.x == 0) {
-    const int E = (red[0] == -100000 ? 0 : red[0]) + ((sd.xf[f] & 3) ? 1 : 0);
+    const int E = E0 + ((sd.xf[f] & 3) ? 1 : 0);
     a.e3[3 * tl + f] = E;
     // one or two flavours: es holds their exponents; three: each component carries all three once
     if (nf <= 2) {
@@ -389,6 +365,7 @@ template <typename R, typename Tin, int NF>
 cudaError_t launch_udsc_t(const UdscArgs& a, int nsm, cudaStream_t s) {
   int nd = 0;
   for (int p = 0; p < a.nprog; p++) nd = std::max(nd, a.prog[p].nd);
+  if (nd > kMaxDs<NF>) return cudaErrorInvalidValue;
   const int smem = udsc_smem<R, NF>(a.nprog, nd);
   cudaError_t e = ensure_smem((const void*)k_contract_udsc<R, Tin, NF>, smem);
   if (e != cudaSuccess) return e;
@@ -406,7 +383,7 @@ cudaError_t launch_contract_udsc(const UdscArgs& a, int nf, int nsm, cudaStream_
 
 template <typename Tin>
 cudaError_t launch_udsc_split_t(const UdscArgs& a, int nf, int nsm, cudaStream_t s) {
-  k_sample_udsc<Tin><<<dim3(a.ntau, nf), 256, 0, s>>>(a, nf);
+  k_sample_udsc<Tin><<<dim3(a.ntau, nf), kSampleThreads, 0, s>>>(a, nf);
   if (nf == 3) k_sum_udsc<<<(a.ntau + 255) / 256, 256, 0, s>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;

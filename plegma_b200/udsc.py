@@ -335,38 +335,54 @@ def site_program(flavours, datasets):
     return slots, warps
 
 
+#: Record types of an encoded program
+REC_A, REC_B, REC_DOT, REC_END = range(4)
+
+
 def encode_programs(prods):
-    """(code, weights, program of each product, [(datasets, start of each warp's code)]): the site
-    programs as one stream of 16-bit words, equal programs stored once.  A warp's code is
-    nA, then per A: block, nB, then per B: block, ndots, then per dot: block, entries, then per
-    entry dataset | weight index << 4."""
+    """(records, weights, program of each product, [(datasets, first record of each warp)], cases): the
+    site programs as one stream of 32-bit records, equal programs stored once.  A record is
+    type | block << 2 | case << 8 | weights << 16.  REC_A: the block becomes A; REC_B: it makes the
+    diquark with A; REC_DOT: its dot with the diquark, times weights[weights + i], is added to dataset
+    i of the case.  cases[0] and cases[1] are the lists of datasets (tuples) that the dots of programs
+    of up to ten datasets, and of more, contribute to."""
     code: List[int] = []
+    rows: Dict[tuple, int] = {}
     values: List[float] = []
     programs, which, seen = [], [], {}
+    cases: Tuple[List[tuple], List[tuple]] = ([], [])
+
+    def record(kind, block, case=0, first=0):
+        code.append(kind | block << 2 | case << 8 | first << 16)
     for flavours, datasets in prods:
         _, warps = site_program(flavours, datasets)
         ident = repr(warps)
         if ident not in seen:
             starts = []
+            mine = cases[0 if len(datasets) <= 10 else 1]
             for groups in warps:
                 starts.append(len(code))
-                code.append(len(groups))
                 for a, bs in groups:
-                    code += [a, len(bs)]
+                    record(REC_A, a)
                     for b, dots in bs:
-                        code += [b, len(dots)]
-                        for z, entries in dots:
-                            code += [z, len(entries)]
-                            for d, w in entries:
-                                if w not in values:
-                                    values.append(w)
-                                code.append(d | values.index(w) << 4)
+                        record(REC_B, b)
+                        for block, entries in dots:
+                            support, row = tuple(d for d, _ in entries), tuple(w for _, w in entries)
+                            if support not in mine:
+                                mine.append(support)
+                            if row not in rows:
+                                rows[row] = len(values)
+                                values.extend(row)
+                            record(REC_DOT, block, mine.index(support), rows[row])
+                record(REC_END, 0)
             seen[ident] = len(programs)
             programs.append((len(datasets), starts))
         which.append(seen[ident])
-    if len(values) >= 4096 or max(code) >= 65536:
+    for _ in range(2):  # a warp reads two records ahead
+        record(REC_END, 0)
+    if len(values) >= 1 << 16 or max(len(c) for c in cases) > 256 or max(n for n, _ in programs) > 16:
         raise ValueError("site program does not fit its encoding")
-    return code, values, which, programs
+    return code, values, which, programs, cases
 
 
 def emit_header(path: str) -> bool:
@@ -398,15 +414,20 @@ def emit_header(path: str) -> bool:
     for i in range(0, len(val), 8):
         L.append("  " + " ".join("{%.9ef,%.9ef}," % v for v in val[i:i + 8]))
     L.append("};")
-    code, values, which, programs = encode_programs(prods)
+    code, values, which, programs, cases = encode_programs(prods)
     L += ["", f"constexpr int kUdscWarps = {PROGRAM_WARPS};",
           "static const int kUdscProgram[kUdscProducts] = {" + ", ".join(map(str, which)) + "};",
           f"static const int kUdscProgramStart[{len(programs)}][kUdscWarps] = {{" +
           ", ".join("{" + ", ".join(map(str, st)) + "}" for _, st in programs) + "};",
           f"constexpr int kUdscCodeWords = {len(code)};",
-          "#define P2_INIT_UDSC_CODE {" + ",".join(map(str, code)) + "}",
+          "#define P2_INIT_UDSC_CODE {" + ",".join("%du" % w for w in code) + "}",
           f"constexpr int kUdscWeights = {len(values)};",
           "#define P2_INIT_UDSC_WEIGHTS {" + ",".join("%.17g" % v for v in values) + "}"]
+    # switch bodies: P2_ADD(d, i) adds weight i times the dot to dataset d
+    for name, lists in zip(("10", "16"), cases):
+        L.append(f"#define P2_UDSC_CASES_{name} " + " ".join(
+            f"case {i}: " + " ".join(f"P2_ADD({d}, {k})" for k, d in enumerate(ds)) + " break;"
+            for i, ds in enumerate(lists)))
     text = "\n".join(L) + "\n"
     try:
         with open(path) as f:
