@@ -40,14 +40,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSitesPerTile = 16;
 constexpr int kRow = 289;  // complex per site row (2 * 144 + 1 pad)
-constexpr int kStage = kSitesPerTile * kRow;
 
-// CM = false: site-major [site][kRow] (the plain kernel reads it directly);
-// CM = true: component-major [flavour * 144 + component][16 sites], written
-// without bank conflicts and transposed by the split kernel's conversion.
-// Only the staging rows 144 f + component in [lo, hi) are copied (component-
-// major staging; the site-major one always copies all).
-template <typename Tin, bool CM = false>
+// Component-major [flavour * 144 + component][16 sites], written without bank
+// conflicts and transposed by the split kernel's conversion.  Only the staging
+// rows 144 f + component in [lo, hi) are copied.
+template <typename Tin>
 __device__ __forceinline__ void issue_tile(const ContractArgs& a, Cx<Tin>* st, int tl, int x0, bool valid, int lo = 0,
                                            int hi = 288) {
   if (valid) {
@@ -66,8 +63,8 @@ __device__ __forceinline__ void issue_tile(const ContractArgs& a, Cx<Tin>* st, i
 #pragma unroll 3
       for (int r = 0; r < 9; r++) {
         const int comp = (threadIdx.x >> 4) + 16 * r;
-        Cx<Tin>* dst = CM ? st + (144 * f + comp) * kSitesPerTile + s : st + s * kRow + 144 * f + comp;
-        if (!CM || (144 * f + comp >= lo && 144 * f + comp < hi)) {
+        Cx<Tin>* dst = st + (144 * f + comp) * kSitesPerTile + s;
+        if (144 * f + comp >= lo && 144 * f + comp < hi) {
           if (sizeof(Tin) == 8)
             cp_async16(dst, src, ok ? 16 : 0);
           else
@@ -175,18 +172,13 @@ __device__ __forceinline__ void contract_site(const ContractArgs& a, const Row& 
                        [&](int j, int ds, Cx<R> v) { w.put(base[j] + 16 * ds + l, v); });
   }
   if (DELTA && (a.what & (2u | 4u))) {
-    // group g of each isospin block, datasets (u-rich, d-rich); the iso-1/2
-    // partial sums of G^{ud} wait in a per-thread array (local memory, L1)
-    // until the G^{uu} / G^{dd} terms complete them
-    Cx<R> parked[3][2];
-    delta_site(
-        row, lt, l, mask,
-        [&](int g, int j, Cx<R> v) {
-          // staging rows: iso-1/2 0..95, iso-3/2 96..191
-          if (j < 2 && (a.what & 2u)) w.dput((g * 2 + j) * 16 + l, a.k.diso12 + (g * 2 + j) * 16 + l, v);
-          if (j >= 2 && (a.what & 4u)) w.dput(96 + (g * 2 + j - 2) * 16 + l, a.k.diso32 + (g * 2 + j - 2) * 16 + l, v);
-        },
-        [&](int g, int j, Cx<R> v) { parked[g][j] = v; }, [&](int g, int j) { return parked[g][j]; });
+    // group g of each isospin block, datasets (u-rich, d-rich); the lane holds component (l & 3) 4 + (l >> 2)
+    const int lo = (l & 3) * 4 + (l >> 2);
+    delta_site(row, lt, l, mask, [&](int g, int j, Cx<R> v) {
+      // staging rows: iso-1/2 0..95, iso-3/2 96..191
+      if (j < 2 && (a.what & 2u)) w.dput((g * 2 + j) * 16 + lo, a.k.diso12 + (g * 2 + j) * 16 + lo, v);
+      if (j >= 2 && (a.what & 4u)) w.dput(96 + (g * 2 + j - 2) * 16 + lo, a.k.diso32 + (g * 2 + j - 2) * 16 + lo, v);
+    });
   }
   if (DELTA) return;
   // nucleon outputs: with staged 16 x 16 mesons they wait in registers until
@@ -281,9 +273,56 @@ __device__ __forceinline__ void contract_site(const ContractArgs& a, const Row& 
   }
 }
 
-// Plain FP64 form.
+// Plain FP64 form: tiles of eight sites, 128 threads, two staging buffers per
+// CTA; three CTAs (12 warps, 168 registers) per SM for the nucleon and the
+// mesons, two (255 registers) for the Delta pass, which spills with fewer.
+constexpr int kPS = 8;
+constexpr int kPTh = 16 * kPS;
+constexpr int plain_per_sm(bool delta) { return delta ? 2 : 3; }
+constexpr int kPStage = kPS * kRow;  // [site][kRow]
+
+__device__ __forceinline__ void issue_plain(const ContractArgs& a, Cx<double>* st, int tl, int x0, bool valid) {
+  if (valid) {
+    const int s = threadIdx.x & (kPS - 1), c0 = threadIdx.x / kPS;
+    const bool ok = x0 + s < a.V3;
+    const SliceDesc* sd = a.sl + tl;
+#pragma unroll
+    for (int f = 0; f < 2; f++) {
+      const long long vol = f ? sd->vol_d : sd->vol_u;
+      const Cx<double>* src = (const Cx<double>*)(f ? sd->d : sd->u) + (f ? sd->off_d : sd->off_u) + (ok ? x0 + s : 0) +
+                              c0 * vol;
+#pragma unroll 3
+      for (int r = 0; r < 9; r++) {
+        cp_async16(st + s * kRow + 144 * f + c0 + 16 * r, src, ok ? 16 : 0);
+        src += 16 * vol;
+      }
+    }
+  }
+  cp_async_commit();
+}
+
+// M[al][de] = sum over colour of u[al][x'] conj(d[de][y'])
+__device__ __forceinline__ void colour_products_f64(const RowF64& row, int xp, int yp, Cx<double> (&M)[4][4]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) M[i][j] = czero<double>();
+#pragma unroll 3
+  for (int c = 0; c < 9; c++) {
+    Cx<double> u[4], d[4];
+#pragma unroll
+    for (int b = 0; b < 4; b++) u[b] = row.p[(kU + 4 * b + xp) * 9 + c];
+#pragma unroll
+    for (int z = 0; z < 4; z++) d[z] = row.p[(kD + 4 * z + yp) * 9 + c];
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+      for (int z = 0; z < 4; z++) cmac_conj(M[b][z], u[b], d[z]);
+  }
+}
+
 template <bool DELTA>
-__global__ void __launch_bounds__(kThreads, 1) k_contract_plain(const ContractArgs a) {
+__global__ void __launch_bounds__(kPTh, plain_per_sm(DELTA)) k_contract_plain(const ContractArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Cx<double>* sm = (Cx<double>*)smem_raw;
   const int tid = threadIdx.x;
@@ -291,23 +330,23 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_plain(const ContractAr
   const unsigned mask = halfwarp_mask();
   const LaneTables lt = load_lane_tables(l);
 
-  const int tiles_per_tau = (a.V3 + kSitesPerTile - 1) / kSitesPerTile;
+  const int tiles_per_tau = (a.V3 + kPS - 1) / kPS;
   TileCursor cur(blockIdx.x, gridDim.x, tiles_per_tau);
   TileCursor nx2 = cur.next();
-  issue_tile<double>(a, sm, cur.tl, cur.x0(), cur.tl < a.ntau);
-  issue_tile<double>(a, sm + kStage, nx2.tl, nx2.x0(), nx2.tl < a.ntau);
+  issue_plain(a, sm, cur.tl, cur.rem * kPS, cur.tl < a.ntau);
+  issue_plain(a, sm + kPStage, nx2.tl, nx2.rem * kPS, nx2.tl < a.ntau);
 
   for (int it = 0; cur.tl < a.ntau; cur = cur.next(), it++) {
-    Cx<double>* st = sm + (it & 1) * kStage;
+    Cx<double>* st = sm + (it & 1) * kPStage;
     cp_async_wait<1>();
     __syncthreads();
-    const int tl = cur.tl;
+    const int tl = cur.tl, x0 = cur.rem * kPS;
     {
       // load-time transform of the staged tile, in place (uniform per tile)
       const int xfu = a.sl[tl].xf[0], xfd = a.sl[tl].xf[1];
       if (xfu | xfd) {
-        const int s = tid & (kSitesPerTile - 1);
-        for (int q = tid >> 4; q < 72; q += kThreads / kSitesPerTile) {
+        const int s = tid & (kPS - 1);
+        for (int q = tid / kPS; q < 72; q += kPTh / kPS) {
           const int f = q >= 36;
           int comp[4];
           prop_group_comps(q - 36 * f, comp);
@@ -317,15 +356,48 @@ __global__ void __launch_bounds__(kThreads, 1) k_contract_plain(const ContractAr
         __syncthreads();
       }
     }
-    const int x = cur.x0() + hw;
-    if (x < a.V3) {
+    if (!DELTA && a.g16_raw) {
+      // nucleon and the colour products M_{al de}[x'][y'] of lane (x', y'):
+      // component 16 (4 al + de) + lane.  The outputs take the site's dead row
+      // and leave as 128-byte component rows (direct stores from the lanes
+      // would touch 16 component rows per instruction).
+      const bool nuc = (a.what & 1u) != 0;
+      Cx<double>* const own = st + hw * kRow;
+      if (x0 + hw < a.V3) {
+        const RowF64 row{own};
+        Cx<double> pn[2], M[4][4];
+        if (nuc) nucleon_site(row, lt, l, mask, pn);
+        colour_products_f64(row, l >> 2, l & 3, M);
+        __syncwarp(mask);
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) own[16 * (4 * i + j) + l] = M[i][j];
+        if (nuc) {
+          own[256 + l] = pn[0];
+          own[272 + l] = pn[1];
+        }
+      }
+      __syncthreads();
+      const int s = tid & (kPS - 1), c0 = tid / kPS;
+      if (x0 + s < a.V3) {
+        Cx<double>* o = (Cx<double>*)a.out + (long long)tl * a.K * a.V3 + x0 + s;
+        const Cx<double>* src = st + s * kRow + c0;
+#pragma unroll
+        for (int j = 0; j < 16; j++) o[(long long)(a.k.g16 + c0 + 16 * j) * a.V3] = src[16 * j];
+        if (nuc) {
+          o[(long long)(a.k.nuc + c0) * a.V3] = src[256];
+          o[(long long)(a.k.nuc + 16 + c0) * a.V3] = src[272];
+        }
+      }
+    } else if (x0 + hw < a.V3) {
       const RowF64 row{st + hw * kRow};
-      const Writer<double> w{(Cx<double>*)a.out + (long long)tl * a.K * a.V3 + x, a.V3, nullptr, nullptr, nullptr, 0};
+      const Writer<double> w{(Cx<double>*)a.out + (long long)tl * a.K * a.V3 + x0 + hw, a.V3, nullptr, nullptr, nullptr, 0};
       contract_site<DELTA>(a, row, lt, l, mask, w);
     }
     __syncthreads();
     nx2 = nx2.next();  // two tiles ahead of the next iteration's
-    issue_tile<double>(a, st, nx2.tl, nx2.x0(), nx2.tl < a.ntau);
+    issue_plain(a, st, nx2.tl, nx2.rem * kPS, nx2.tl < a.ntau);
   }
   cp_async_wait<0>();
 }
@@ -373,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
   TileCursor tc(blockIdx.x, gridDim.x, tiles_per_tau);
   for (int k = tid; k < a.K; k += kThreads) *smax_slot(sf, k) = 0;
 
-  issue_tile<Tin, true>(a, st, tc.tl, tc.x0(), tc.tl < a.ntau);
+  issue_tile<Tin>(a, st, tc.tl, tc.x0(), tc.tl < a.ntau);
 
   int cur = -1;  // slice whose maxima the spare slots hold
   // running maxima in registers: nucleon outputs of lane l (slots 0, 1) and
@@ -414,7 +486,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
     cp_async_wait<0>();
     __syncthreads();
     if (tl != cur) {
-      if (cur >= 0)
+      if (cur >= 0 && a.cmax)
         for (int k = tid; k < a.K; k += kThreads) {
           int* slot = smax_slot(sf, k);
           atomicMax(a.cmax + (long long)cur * a.K + k, *slot);
@@ -482,7 +554,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
     // the staged tile has been converted: refill the staging buffer while
     // contracting (with Delta output staging, all but its tail)
     const TileCursor nx = tc.next();
-    issue_tile<Tin, true>(a, st, nx.tl, nx.x0(), nx.tl < a.ntau, 0, dstg ? kLate0 : 288);
+    issue_tile<Tin>(a, st, nx.tl, nx.x0(), nx.tl < a.ntau, 0, dstg ? kLate0 : 288);
     const int x0 = tc.x0();
     if (x0 + hw < a.V3) {
       const RowF32T<kPerm> row{sf + hw * kRow32};
@@ -514,7 +586,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
           if (s == 0) atomicMax(smax_slot(sf, k), __float_as_int(m));
         }
         __syncthreads();  // the staging tail is read: the next tile's last rows may land there
-        issue_tile<Tin, true>(a, st, nx.tl, nx.x0(), nx.tl < a.ntau, kLate0, 288);
+        issue_tile<Tin>(a, st, nx.tl, nx.x0(), nx.tl < a.ntau, kLate0, 288);
       }
     }
     if constexpr (!DELTA) {
@@ -547,7 +619,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_contract_f32(const ContractArgs
   cp_async_wait<0>();
   if (cur >= 0) flush_lane();
   __syncthreads();
-  if (cur >= 0)
+  if (cur >= 0 && a.cmax)
     for (int k = tid; k < a.K; k += kThreads) atomicMax(a.cmax + (long long)cur * a.K + k, *smax_slot(sf, k));
 }
 
@@ -566,14 +638,14 @@ __global__ void __launch_bounds__(kSampleThreads) k_sample_exponents(const Sampl
 
 }  // namespace
 
-int contract_plain_smem_bytes() { return 2 * kStage * (int)sizeof(Cx<double>); }
+int contract_plain_smem_bytes() { return 2 * kPStage * (int)sizeof(Cx<double>); }
 
 template <bool DELTA>
 cudaError_t launch_plain_t(const ContractArgs& a, int grid, cudaStream_t s) {
   const int smem = contract_plain_smem_bytes();
   cudaError_t e = ensure_smem((const void*)k_contract_plain<DELTA>, smem);
   if (e != cudaSuccess) return e;
-  k_contract_plain<DELTA><<<grid, kThreads, smem, s>>>(a);
+  k_contract_plain<DELTA><<<plain_per_sm(DELTA) * grid, kPTh, smem, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -353,12 +353,16 @@ static_assert(typea_lane(kDeltaLane[0]) == 0 && typea_lane(kDeltaLane[1]) == 0 &
 // accumulators, (gx zx, gx zy) and (gy zx, gy zy), so that z enters as the
 // natural (Re, Im) pair of its shared-memory load and only g is broadcast
 // (once per g for all the dot products it takes part in).
+// FP64: three partial sums, so that six chains of DFMAs are in flight (one sum
+// has two chains of eighteen, and few warps to hide their latency).
 template <typename R>
 __device__ __forceinline__ Cx<R> cdot9(const Cx<R> g[9], const Cx<R> z[9]) {
-  Cx<R> r = czero<R>();
+  Cx<R> r[3];
 #pragma unroll
-  for (int i = 0; i < 9; i++) cmac(r, g[i], z[i]);
-  return r;
+  for (int j = 0; j < 3; j++) r[j] = cmul(g[j], z[j]);
+#pragma unroll
+  for (int i = 3; i < 9; i++) cmac(r[i % 3], g[i], z[i]);
+  return r[0] + r[1] + r[2];
 }
 template <>
 __device__ __forceinline__ Cx<float> cdot9<float>(const Cx<float> g[9], const Cx<float> z[9]) {
@@ -415,10 +419,7 @@ __device__ __forceinline__ Cx<typename Row::R> diquark_slots(const Cx<typename R
       for (int m = 0; m < 4; m++) {
         Cx<R> z[9];
         row.load9(Z + m * 4 + dl.z2, z);
-        Cx<R> p2 = czero<R>();
-#pragma unroll
-        for (int i = 0; i < 9; i++) cmac(p2, g[i], z[i]);
-        p2 = cscale(p2, f2);
+        Cx<R> p2 = cscale(cdot9(g, z), f2);
         p2 = p2 + shfl_xor16(p2, 4, mask);
         p2 = p2 + shfl_xor16(p2, 8, mask);
         if (m == mu) r = r + p2;
@@ -431,10 +432,7 @@ __device__ __forceinline__ Cx<typename Row::R> diquark_slots(const Cx<typename R
       for (int m = 0; m < 4; m++) {
         Cx<R> z[9];
         row.load9(Z + m * 4 + dl.z1, z);
-        Cx<R> p1 = czero<R>();
-#pragma unroll
-        for (int i = 0; i < 9; i++) cmac(p1, g[i], z[i]);
-        p1 = cscale(p1, f1);
+        Cx<R> p1 = cscale(cdot9(g, z), f1);
         p1 = p1 + shfl_xor16(p1, 1, mask);
         p1 = p1 + shfl_xor16(p1, 2, mask);
         const Cx<R> v = shfl_idx16(p1, src, mask);
@@ -493,10 +491,7 @@ __device__ __forceinline__ Cx<typename Row::R> diquark_slot1_transposed(const Cx
     for (int m = 0; m < 4; m++) {
       Cx<R> z[9];
       row.load9(Z + m * 4 + dlT.z1, z);
-      Cx<R> p = czero<R>();
-#pragma unroll
-      for (int i = 0; i < 9; i++) cmac(p, g[i], z[i]);
-      p = cscale(p, f1);
+      Cx<R> p = cscale(cdot9(g, z), f1);
       p = p + shfl_xor16(p, 4, mask);
       p = p + shfl_xor16(p, 8, mask);
       if (m == mu) r = r + p;
@@ -721,111 +716,174 @@ __device__ __forceinline__ void meson_site(const Row& row, int A, int B, const L
 //   isospin 1/2, G^{AA}, Z = B: (0, 2, 0, -2, 1, -1)        x 1/3
 //   isospin 1/2, G^{AB}, Z = A: (-4, 0, 2, -2, 4, 0)        x 1/3
 //   isospin 3/2, G^{AA}, Z = A: (-1, 1, 1, -1, 1, -1)
-// Both G^{AA} groups have cN = 1, cL = -1, so they share the type-a sum D.
-//
-// The three sink tables share products: C g_1 and C g_2 use the diagonal
-// pairs (nu, nu) with signs (+ - - +) and (+ + - -), so with
-// A = P00 - P22 and B = P11 - P33, G_1 = A - B and G_2 = A + B; C g_3 uses
-// (0,1), (1,0), (2,3), (3,2) with signs (+ + - -), and for a single flavour
-// P^{XX}_{(lam, nu)}(x', y') = P^{XX}_{(nu, lam)}(y', x'), so
-// G_3^{XX} = Q + Q^T with Q = P01 - P23 (lane transpose).  For G^{uu} and
-// G^{dd} that is 6 products instead of 12 (G^{ud} keeps 12): 24 per site and
-// lane instead of 36.  The tables are pinned in the spin-table tests.
-//
-// For k = g + 1 and lane (mu, mu'), out(g, j, v) receives the final value of
-// j = 0: iso-1/2 Delta+ (u,u,d), 1: iso-1/2 Delta0 (d,d,u), 2: iso-3/2
-// Delta++ (u,u,u), 3: iso-3/2 Delta- (d,d,d); the G^{ud} part of the
-// iso-1/2 values is parked first with part(g, j, v) and read back with
-// part_get(g, j) (registers are the scarce resource here).
-template <typename Row, typename Out, typename Part, typename PartGet>
-__device__ __forceinline__ void delta_site(const Row& row, const LaneTables& lt, int l, unsigned mask, Out&& out,
-                                           Part&& part, PartGet&& part_get) {
+// C g_k is symmetric, so G^{YX} is the lane transpose of G^{XY}, G^{uu} and
+// G^{dd} are symmetric under it, and the source tables have z1 = z(y'),
+// z2 = z(x'), sA1 = sB1 = s(y'), sA2 = sB2 = s(x') and sN = sL (checked
+// below).  The two slots of every group therefore hold the same sum: with
+// Q = G^{uu}, G^{dd} or G^{ud} + G^{du},
+//   T[Q, Z][mu][mu'] = 4 sum_s s(s) Q(mu', s) . Z[mu][z(s)] + 2 (sum_l sN(l) Q(l)) . Z[mu][mu']
+//   Delta+  = (T[G^{ud} + G^{du}, u] + T[G^{uu}, d]) / 3     Delta++ = T[G^{uu}, u]
+//   Delta0  = (T[G^{ud} + G^{du}, d] + T[G^{dd}, u]) / 3     Delta-  = T[G^{dd}, d]
+// so one slot and one type-a sum serve where the Wick terms have two and a
+// lane transpose, and every block of Z is loaded once for three dot products
+// (the loads between shared memory and the registers bound the split form).
+// The diquarks share their products: C g_1 and C g_2 use the diagonal pairs
+// (nu, nu) with signs (+ - - +) and (+ + - -), so with A = P00 - P22 and
+// B = P11 - P33, G_1 = A - B and G_2 = A + B; C g_3 uses (0,1), (1,0), (2,3),
+// (3,2) with signs (+ + - -), and for a single flavour P^{XX}_{(lam, nu)} is
+// the lane transpose of P^{XX}_{(nu, lam)}, so G_3^{XX} = Q + Q^T with
+// Q = P01 - P23: 20 products per site and lane.
+__host__ __device__ constexpr bool delta_lane_symmetric(const int (&t)[16][8]) {
+  for (int l = 0; l < 16; l++) {
+    const int x = l >> 2, y = l & 3;
+    if (t[l][0] != t[y][0] || t[l][3] != t[x][0] || t[l][1] != t[y][1] || t[l][2] != t[y][1] || t[l][4] != t[x][1] ||
+        t[l][5] != t[x][1] || t[l][6] != t[l][7])
+      return false;
+  }
+  return true;
+}
+static_assert(kDeltaLane[0][1][0] == 1 && kDeltaLane[0][2][0] == 2 && kDeltaLane[1][1][0] == 1 && kDeltaLane[1][3][0] == 3,
+              "C g_1 and C g_2 contract equal spins");
+static_assert(delta_lane_symmetric(kDeltaLane[0]) && delta_lane_symmetric(kDeltaLane[1]) &&
+                  delta_lane_symmetric(kDeltaLane[2]),
+              "Delta source tables without the slot symmetry");
+
+// acc += sum_i g[i] z[i]
+template <typename R>
+__device__ __forceinline__ void cdot9_acc(Cx<R>& acc, const Cx<R> g[9], const Cx<R> z[9]) {
+  if constexpr (sizeof(R) == 8) {
+    acc = acc + cdot9(g, z);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 9; i++) cmac(acc, g[i], z[i]);
+  }
+}
+
+// q = P^{XY}_{(a, b)} - P^{XY}_{(a + 2, b + 2)}, plus (both) the same of (b, a)
+template <typename Row>
+__device__ __forceinline__ void delta_products(const Row& row, int X, int Y, int a, int b, bool both, int xp, int yp,
+                                               Cx<typename Row::R> (&q)[9]) {
+  typedef typename Row::R R;
+#pragma unroll
+  for (int i = 0; i < 9; i++) q[i] = czero<R>();
+  // rolled: the Delta's straight-line code does not fit the instruction caches
+#pragma unroll 1
+  for (int t = 0; t < (both ? 4 : 2); t++) {
+    const int n = t < 2 ? a : b, m = t < 2 ? b : a;
+    diquark_acc(row, X, Y, n + 2 * (t & 1), m + 2 * (t & 1), (t & 1) ? R(-1) : R(1), xp, yp, q);
+  }
+}
+
+// For N diquarks g (with the slot's sign) and the line Z, on lane (mu', y'):
+// T[n] = sum_s g[n](mu', s) . Z[mu][z(s)] + (sum_class g[n]) . Z[mu][mu'] / 2,
+// mu = y'.  The dots for mu = 0..3 are reduce-scattered over s (lane bits 1, 0).
+template <int N, typename Row>
+__device__ __forceinline__ void delta_sums(const Row& row, const Cx<typename Row::R> (&g)[N][9],
+                                           const Cx<typename Row::R> (&D)[N][9], int Z, int z, int l, unsigned mask,
+                                           Cx<typename Row::R> (&T)[N]) {
+  typedef typename Row::R R;
+  const bool b1 = (l >> 1) & 1, b0 = l & 1;
+  Cx<R> half[N];
+#pragma unroll
+  for (int h = 0; h < 2; h++) {  // mu = h and mu = h + 2 exchange first
+    Cx<R> P[2][N];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      Cx<R> v[9];
+      row.load9(Z + 4 * (h + 2 * q) + z, v);
+#pragma unroll
+      for (int n = 0; n < N; n++) {
+        P[q][n] = czero<R>();
+        cdot9_acc(P[q][n], g[n], v);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const Cx<R> v = (b1 ? P[1][n] : P[0][n]) + shfl_xor16(b1 ? P[0][n] : P[1][n], 2, mask);
+      if (h == 0)
+        half[n] = v;
+      else
+        T[n] = (b0 ? v : half[n]) + shfl_xor16(b0 ? half[n] : v, 1, mask);
+    }
+  }
+  Cx<R> v[9];
+  row.load9(Z + (l & 3) * 4 + (l >> 2), v);
+#pragma unroll
+  for (int n = 0; n < N; n++) cdot9_acc(T[n], D[n], v);
+}
+
+// For k = g + 1 out(g, j, v) receives the value of j = 0: iso-1/2 Delta+
+// (u,u,d), 1: iso-1/2 Delta0 (d,d,u), 2: iso-3/2 Delta++ (u,u,u), 3: iso-3/2
+// Delta- (d,d,d), of component mu = l & 3, mu' = l >> 2 (the lane that the
+// slot's sum over s leaves it on).  One flavour pair at a time, in a rolled
+// loop: its code fits the instruction caches and its registers 16 warps per
+// SM.  uu feeds Delta++ (Z = u) and Delta+ (Z = d), ud + du Delta+ (u) and
+// Delta0 (d), dd Delta0 (u) and Delta- (d).  C g_1 and C g_2 have z(s) = s, so
+// each load of Z serves both.
+template <typename Row, typename Out>
+__device__ __forceinline__ void delta_site(const Row& row, const LaneTables& lt, int l, unsigned mask, Out&& out) {
   typedef typename Row::R R;
   const int xp = l >> 2, yp = l & 3;
-  const R third = R(1) / R(3);
-  // iso-1/2 partial sums from G^{ud} / G^{du}, completed by the G^{uu} / G^{dd} terms
-  // G^{ud} (A = u) and its lane transpose G^{du} (A = d; C g_k is symmetric)
-  // C g_1 and C g_2 from the shared diagonal products ga = P00 - P22,
-  // gb = P11 - P33 (8 products instead of 12).  FP64: ga and gb formed up
-  // front; FP32 (registers are tighter): C g_3 first, then ga and gb, with
-  // only C g_2's sum ga + gb held over C g_1's evaluation
-  constexpr bool kShare = sizeof(R) == 8;
-  Cx<R> ga[9], gb[9];
-  if (kShare) {
+  auto symmetrise = [&](Cx<R>(&q)[9]) {
+    const int src = ((l & 3) << 2) | (l >> 2);
 #pragma unroll
-    for (int i = 0; i < 9; i++) ga[i] = gb[i] = czero<R>();
-    diquark_acc(row, kU, kD, 0, 0, R(1), xp, yp, ga);
-    diquark_acc(row, kU, kD, 2, 2, R(-1), xp, yp, ga);
-    diquark_acc(row, kU, kD, 1, 1, R(1), xp, yp, gb);
-    diquark_acc(row, kU, kD, 3, 3, R(-1), xp, yp, gb);
-  }
-  Cx<R> q1[9];  // FP32: C g_2's G^{ud}, formed with C g_1's
+    for (int i = 0; i < 9; i++) q[i] = q[i] + shfl_idx16(q[i], src, mask);
+  };
+  Cx<R> part[3][2];  // Delta+ of the pair uu, Delta0 of the pair ud
 #pragma unroll 1
-  for (int it = 0; it < 3; it++) {
-    const int g = kShare ? it : (it == 0 ? 2 : it - 1);
-    Cx<R> q[9], D[9];
-    if (kShare && g < 2) {
-#pragma unroll
-      for (int i = 0; i < 9; i++) q[i] = g == 0 ? ga[i] - gb[i] : ga[i] + gb[i];
-    } else if (!kShare && it == 1) {
-      diquark_pair_ct<0, 0, 1, 2, 2, -1>(row, kU, kD, xp, yp, q);
-      diquark_pair_ct<1, 1, 1, 3, 3, -1>(row, kU, kD, xp, yp, q1);
+  for (int p = 0; p < 3; p++) {
+    const int X = p == 2 ? kD : kU, Y = p == 0 ? kU : kD;
+    auto emit = [&](int g, Cx<R> vu, Cx<R> vd) {
+      vu = cscale(vu, p == 0 ? R(4) : R(4) / R(3));
+      vd = cscale(vd, p == 2 ? R(4) : R(4) / R(3));
+      if (p > 0) vu = vu + part[g][p - 1];
+      out(g, p == 0 ? 2 : p - 1, vu);
+      if (p < 2)
+        part[g][p] = vd;
+      else
+        out(g, 3, vd);
+    };
+    {
+      Cx<R> G[2][9], D[2][9], Tu[2], Td[2];
+      delta_products(row, X, Y, 0, 0, false, xp, yp, G[0]);
+      delta_products(row, X, Y, 1, 1, false, xp, yp, G[1]);
+      const DiquarkLane d1 = unpack_diquark_lane(lt.delta[0]), d2 = unpack_diquark_lane(lt.delta[1]);
+      const R s1 = R(d1.sA1), s2 = R(d2.sA1);
 #pragma unroll
       for (int i = 0; i < 9; i++) {
-        const Cx<R> t = q[i];
-        q[i] = t - q1[i];
-        q1[i] = t + q1[i];
+        const Cx<R> t = G[0][i];
+        G[0][i] = cscale(t - G[1][i], s1);
+        G[1][i] = cscale(t + G[1][i], s2);
       }
-    } else if (!kShare && it == 2) {
+      if (p == 1) {
+        // s(y') G(x', y') + s(y') G(y', x'): the transposed lane's value carries its own sign
+        const R r1 = s1 * R(d1.sA2), r2 = s2 * R(d2.sA2);
+        const int src = ((l & 3) << 2) | (l >> 2);
 #pragma unroll
-      for (int i = 0; i < 9; i++) q[i] = q1[i];
-    } else {
-      diquark_G_ct<3>(row, kU, kD, xp, yp, q);  // g = 2 (C g_3) in both forms
-    }
-    const DiquarkLane dl = unpack_diquark_lane(g == 0 ? lt.delta[0] : g == 1 ? lt.delta[1] : lt.delta[2]);
-    diquark_D(q, R(4 * dl.sN), mask, g == 2 ? 1 : 0, D);  // cN = 4, cL = 0
-    part(g, 0, cscale(diquark_eval<true, true>(q, row, kU, dl, l, mask, -4, 0, 2, -2, D), third));
-    diquark_transpose<R>(q, l, mask, R(1));  // G^{du}; its type-a sum is (+1)(tau = +1) D
-    part(g, 1, cscale(diquark_eval<true, true>(q, row, kD, dl, l, mask, -4, 0, 2, -2, D), third));
-  }
-  // G^{uu} (pair 0: Delta+ and Delta++) and G^{dd} (pair 1: Delta0 and Delta-)
-#pragma unroll 1
-  for (int pair = 0; pair < 2; pair++) {
-    const int X = pair == 0 ? kU : kD;
-    const int O = pair == 0 ? kD : kU;
-    Cx<R> ga[9], gb[9];
-    diquark_pair_ct<0, 0, 1, 2, 2, -1>(row, X, X, xp, yp, ga);
-    diquark_pair_ct<1, 1, 1, 3, 3, -1>(row, X, X, xp, yp, gb);
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-      const Cx<R> t = ga[i];
-      ga[i] = t - gb[i];
-      gb[i] = t + gb[i];
-    }
-#pragma unroll
-    for (int g = 0; g < 3; g++) {
-      Cx<R> q[9];
-      if (g < 2) {
-#pragma unroll
-        for (int i = 0; i < 9; i++) q[i] = g == 0 ? ga[i] : gb[i];
-      } else {
-        diquark_pair_ct<0, 1, 1, 2, 3, -1>(row, X, X, xp, yp, q);
-        Cx<R> t[9];
-#pragma unroll
-        for (int i = 0; i < 9; i++) t[i] = q[i];
-        diquark_transpose<R>(t, l, mask, R(1));
-#pragma unroll
-        for (int i = 0; i < 9; i++) q[i] = q[i] + t[i];
+        for (int i = 0; i < 9; i++) {
+          G[0][i] = G[0][i] + cscale(shfl_idx16(G[0][i], src, mask), r1);
+          G[1][i] = G[1][i] + cscale(shfl_idx16(G[1][i], src, mask), r2);
+        }
       }
-      const DiquarkLane dl = unpack_diquark_lane(g == 0 ? lt.delta[0] : g == 1 ? lt.delta[1] : lt.delta[2]);
-      Cx<R> iso12 = diquark_slots<true, true>(q, row, O, dl, l, mask, 0, 2, 0, -2);
-      Cx<R> iso32 = diquark_slots<true, true>(q, row, X, dl, l, mask, -1, 1, 1, -1);
-      Cx<R> D[9];
-      diquark_D(q, R(dl.sN + dl.sL), mask, g == 2 ? 1 : 0, D);  // cN = 1, cL = -1 for both groups
-      iso12 = iso12 + diquark_typea(D, row, O, l);
-      iso32 = iso32 + diquark_typea(D, row, X, l);
-      out(g, pair, part_get(g, pair) + cscale(iso12, third));
-      out(g, 2 + pair, iso32);
+      diquark_D(G[0], R(d1.sN * d1.sN) * R(0.5), mask, 0, D[0]);
+      diquark_D(G[1], R(d2.sN * d2.sN) * R(0.5), mask, 0, D[1]);
+      delta_sums<2>(row, G, D, kU, yp, l, mask, Tu);
+      delta_sums<2>(row, G, D, kD, yp, l, mask, Td);
+      emit(0, Tu[0], Td[0]);
+      emit(1, Tu[1], Td[1]);
+    }
+    {
+      Cx<R> G[1][9], D[1][9], Tu[1], Td[1];
+      delta_products(row, X, Y, 0, 1, p == 1, xp, yp, G[0]);
+      symmetrise(G[0]);
+      const DiquarkLane d3 = unpack_diquark_lane(lt.delta[2]);
+      const R s3 = R(d3.sA1);
+#pragma unroll
+      for (int i = 0; i < 9; i++) G[0][i] = cscale(G[0][i], s3);
+      diquark_D(G[0], R(d3.sN * d3.sN) * R(0.5), mask, 1, D[0]);
+      delta_sums<1>(row, G, D, kU, d3.z1, l, mask, Tu);
+      delta_sums<1>(row, G, D, kD, d3.z1, l, mask, Td);
+      emit(2, Tu[0], Td[0]);
     }
   }
 }
