@@ -515,10 +515,12 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     c->plain_moms_key = pl.moms;
   }
 
+  const size_t s1_slice = ap ? (size_t)c->Ll[1] * c->Ll[2] * ap->R1 * pl.K * 16 : 0;
   const int tc = chunk_slices(c, pl.K);
   const Work w = make_work(c, props, reqs, idx, nidx, tc);
   if (w.sl.empty()) return P2_OK;
   P2_TRY(c, c->cbuf.ensure((size_t)w.max_n * pl.K * c->V3 * 16), "position buffer alloc");
+  if (ap) P2_TRY(c, c->axes_s1.ensure(std::max(kMinWorkspace, (size_t)w.max_n * s1_slice)), "projection workspace");
   Stager sg(c, props, reqs, w);
   if ((st = sg.prepare(outs)) != P2_OK) return st;
 
@@ -544,9 +546,7 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     if ((st = sg.issue((int)ci + 2)) != P2_OK) return st;
 
     if (ap) {
-      P2_TRY(c, c->axes_s1.ensure((size_t)w.max_n * c->Ll[1] * c->Ll[2] * ap->R1 * pl.K * 16), "projection workspace");
-      if ((st = axes_x(c, *ap, c->cbuf.p, 0, (long long)pl.K * c->V3, c->V3, n, pl.K, c->axes_s1.p)) != P2_OK)
-        return st;
+      if ((st = axes_x_blocks(c, *ap, pl, what, what, c->cbuf.p, 0, n, c->axes_s1.p)) != P2_OK) return st;
       AxesOut ao;
       ao.dsl = sg.desc((int)ci);
       ao.blocks = &pl.blocks;
@@ -588,7 +588,7 @@ p2_status ft_axes(p2_ctx* c, const AxesPlan& ap, const double* field, int dof, i
   P2_TRY(c, c->axes_s1.ensure((size_t)tc * s1), "projection workspace");
   for (int t0 = 0; t0 < nt; t0 += tc) {
     const int n = std::min(tc, nt - t0);
-    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, c->axes_s1.p);
+    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, dof, c->axes_s1.p);
     if (st != P2_OK) return st;
     AxesOut ao;
     ao.oT = (long long)dof * ap.nmom;
@@ -998,6 +998,13 @@ p2_status p2_ft_apply_split(p2_ctx* c, const double* field, int dof, int nt, con
   if (sign != 1 && sign != -1) return c->fail(P2_ERR_INVALID_ARG, "p2_ft_apply_split: sign must be +1 or -1");
   if (out_location != P2_DEVICE && out_location != P2_HOST) return c->fail(P2_ERR_INVALID_ARG, "bad out_location");
   if (c->host_only) return c->fail(P2_ERR_UNSUPPORTED, "host-only context");
+  // a list with few rows per axis is summed axis by axis in FP64 (bound by the
+  // read of the field either way); an armed p2_debug_wait_timeout asks for the
+  // tensor-core projection
+  const AxesPlan* ap = nullptr;
+  p2_status st;
+  if (!c->wait_test && (st = axes_prepare(c, std::vector<int>(moms, moms + 3 * nmom), sign, &ap)) != P2_OK) return st;
+  if (ap) return ft_axes(c, *ap, field, dof, nt, out, out_location);
   if (c->project_split_smem_max < p2::project_split_smem_bytes(p2::project_split_max_nt()))
     return c->fail(P2_ERR_UNSUPPORTED, "device shared memory per block too small for the tensor-core projection");
   // exp(+i p.x) = exp(-i (-p).x): the projection's rows carry exp(-i p.x)
@@ -1014,8 +1021,7 @@ p2_status p2_ft_apply_split(p2_ctx* c, const double* field, int dof, int nt, con
     P2_TRY(c, cudaMemsetAsync(c->errflag.p, 0, 16, c->stream), "error flag clear");
   }
   int nmtile = 0, nkstep = 0;
-  p2_status st = p2::split_prepare_tables(c, pl, 0, nmtile, nkstep);
-  if (st != P2_OK) return st;
+  if ((st = p2::split_prepare_tables(c, pl, 0, nmtile, nkstep)) != P2_OK) return st;
   const size_t total = (size_t)nt * dof * nmom;
   double* dst = out;
   if (out_location == P2_HOST) {

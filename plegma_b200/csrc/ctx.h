@@ -54,10 +54,11 @@ struct DevBuf {
 struct AxesPlan {
   std::vector<int> key;  // momentum list the tables were built for
   bool usable = false;   // the list has few enough rows per axis
-  int R1 = 0, RY = 0, NP = 0, NO = 0, ny = 0, nmom = 0;
+  int R1 = 0, RY = 0, NP = 0, NO = 0, nmom = 0;
   DevBuf tab, idx;
   const double *xt = nullptr, *yt = nullptr, *zt = nullptr;
-  const int *first = nullptr, *ylist = nullptr, *orb = nullptr, *omom = nullptr;
+  std::vector<int> first, ylist;
+  const int *orb = nullptr, *omom = nullptr;
 };
 
 struct BlockDef {
@@ -255,8 +256,15 @@ struct AxesOut {
 p2_status project_direct(p2_ctx* c, const Plan& pl, int K, int n, int max_n, const p2::SliceDesc* dsl,
                          const std::vector<p2::ScatterBlock>& blocks);
 p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const AxesPlan** out);
+// The sums over x of the blocks of `bits` from a position buffer of the whole
+// set `what` (n slices, K components of V3 sites each).
+p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
+                        int fp32, int n, void* s1);
+// The sums over x are small; their buffer starts at this size so that calls of
+// different sizes share one allocation.
+constexpr size_t kMinWorkspace = (size_t)64 << 20;
 p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
-                 void* s1);
+                 int Kst, void* s1);
 p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o);
 
 }  // namespace p2host

@@ -194,18 +194,19 @@ struct AxisXArgs {
   const void* c;      // complex double or complex float, element (tau, k, x) at c[tau*sT + k*sK + x]
   long long sT, sK;
   int ntau, K, rows, Lx, R1;
+  int Kst;            // components of s1 (K of them, from s1's first, are written)
   int KL;             // components a warp takes side by side (set by the launcher)
   const double* xt;   // [Lx][R1] phase rows
-  void* s1;           // [ntau][rows][R1][K] complex, type of c
+  void* s1;           // [ntau][rows][R1][Kst] complex, type of c
 };
 struct AxisYArgs {
   const void* s1;
-  void* s2;           // [ntau][Lz][NP][K] complex double
+  void* s2;           // [ntau][Lz][NP][K] complex, type of s1
   int ntau, K, Ly, Lz, R1, RY, NP;
-  int ny;             // most pairs of one x row
-  const double* yt;   // [Ly][RY]
-  const int* first;   // [R1 + 1] first pair of each x row
-  const int* ylist;   // [NP] y row of each pair
+  int zper;           // z values per block (set by the launcher)
+  const double* yt;   // [RY][Ly]
+  int first[kAxisMaxRows + 1];              // [R1 + 1] first pair of each x row
+  int ylist[kAxisMaxRows * kAxisMaxRows];   // [NP] y row of each pair
 };
 struct AxisZArgs {
   const void* s2;
@@ -225,7 +226,7 @@ struct AxisZArgs {
 };
 cudaError_t launch_axis_x(const AxisXArgs& a, int fp32, cudaStream_t s);
 cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s);
-cudaError_t launch_axis_z(const AxisZArgs& a, cudaStream_t s);
+cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s);
 
 cudaError_t launch_contract_plain(const ContractArgs& a, int grid, cudaStream_t s);
 // FP32 site contraction; fp32_in selects complex-float propagators.

@@ -107,16 +107,39 @@ PhaseRows phase_rows(const std::vector<int>& moms) {
 
 namespace p2 {
 
+// Exponents and phases of a contraction set's components (what = 0: none).
+static p2_status split_component_tables(p2_ctx* c, unsigned what) {
+  p2_status st;
+  if (what && c->split_what_key != what) {
+    // [K][2] scale powers, then [K] unit phases i^q of the 16 x 16 mesons
+    // that the contraction leaves out (g16_phase_deferred; with g16_raw the
+    // components are colour products and the Gamma sums, phases included,
+    // come after the reduction)
+    std::vector<int> ke = component_exponents(what);
+    const int K = (int)ke.size() / 2;
+    ke.resize(3 * (size_t)K, 0);
+    if (g16_phase_deferred(what) && !g16_raw(what)) {
+      const int k0 = offsets_of(what).g16;
+      for (int g1 = 0; g1 < 16; g1++)
+        for (int g2 = 0; g2 < 16; g2++) ke[2 * K + k0 + 16 * g1 + g2] = meson_phase_q(g1, g2);
+    }
+    if ((st = upload_async(c, c->kexp, ke.data(), ke.size() * sizeof(int), "component exponents")) != P2_OK) return st;
+    c->split_what_key = what;
+  }
+  return P2_OK;
+}
+
 // Phase tiles, momentum rows and component exponents, rebuilt only when the
 // momentum list or the contraction set changes (the tiles have origin 0, so
 // every source shares them).  what = 0: tiles and rows only.
 p2_status split_prepare_tables(p2_ctx* c, const Plan& pl, unsigned what, int& nmtile, int& nkstep) {
+  p2_status st = split_component_tables(c, what);
+  if (st != P2_OK) return st;
   PhaseRows pr = phase_rows(pl.moms);
   const int nh = (int)pr.reps.size() / 3;
   const int nrows = (int)pr.row_h.size();
   nmtile = (nrows + 127) / 128;
   nkstep = (int)((c->V3 + 63) / 64);
-  p2_status st;
   if (c->split_moms_key != pl.moms) {
     c->split_moms_key.clear();
     std::vector<double> tabh = phase_tables(c, pr.reps.data(), nh, -1, pl.Lmax);
@@ -161,22 +184,6 @@ p2_status split_prepare_tables(p2_ctx* c, const Plan& pl, unsigned what, int& nm
     c->split_nrep = nh;
     if ((st = upload_async(c, c->momrow, mr.data(), mr.size() * sizeof(int), "momentum rows")) != P2_OK) return st;
     c->split_moms_key = pl.moms;
-  }
-  if (what && c->split_what_key != what) {
-    // [K][2] scale powers, then [K] unit phases i^q of the 16 x 16 mesons
-    // that the contraction leaves out (g16_phase_deferred; with g16_raw the
-    // components are colour products and the Gamma sums, phases included,
-    // come after the reduction)
-    std::vector<int> ke = component_exponents(what);
-    const int K = (int)ke.size() / 2;
-    ke.resize(3 * (size_t)K, 0);
-    if (g16_phase_deferred(what) && !g16_raw(what)) {
-      const int k0 = offsets_of(what).g16;
-      for (int g1 = 0; g1 < 16; g1++)
-        for (int g2 = 0; g2 < 16; g2++) ke[2 * K + k0 + 16 * g1 + g2] = meson_phase_q(g1, g2);
-    }
-    if ((st = upload_async(c, c->kexp, ke.data(), ke.size() * sizeof(int), "component exponents")) != P2_OK) return st;
-    c->split_what_key = what;
   }
   return P2_OK;
 }
@@ -295,12 +302,6 @@ p2_status split_project(p2_ctx* c, const Plan& pl, int K, int n, int nmtile, int
 
 p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request* reqs, const int* idx, int nidx,
                               const Plan& pl, double* const* outs) {
-  if (!c->errflag.p) {
-    P2_TRY(c, c->errflag.ensure(16), "error flag alloc");
-    P2_TRY(c, cudaMemsetAsync(c->errflag.p, 0, 16, c->stream), "error flag clear");
-  }
-  if (c->project_split_smem_max < p2::project_split_smem_bytes(p2::project_split_max_nt()))
-    return c->fail(P2_ERR_UNSUPPORTED, "device shared memory per block too small for the tensor-core projection");
   const p2_request& r0 = reqs[idx[0]];
   const unsigned what = r0.contractions;
   for (int q = 0; q < nidx; q++) {
@@ -318,13 +319,28 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
   }
   const int fp32_in = props[r0.prop_u].precision == P2_FP32;
   const int K = pl.K;
+  // the axis-by-axis projection when the momentum list qualifies, else the
+  // tensor-core one (which an armed p2_debug_wait_timeout asks for)
+  const AxesPlan* ap = nullptr;
+  p2_status st;
+  if (!c->wait_test && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
   int nmtile = 0, nkstep = 0;
-  p2_status st = split_prepare_tables(c, pl, what, nmtile, nkstep);
-  if (st != P2_OK) return st;
+  if (ap) {
+    if ((st = split_component_tables(c, what)) != P2_OK) return st;
+  } else {
+    if (c->project_split_smem_max < p2::project_split_smem_bytes(p2::project_split_max_nt()))
+      return c->fail(P2_ERR_UNSUPPORTED, "device shared memory per block too small for the tensor-core projection");
+    if (!c->errflag.p) {
+      P2_TRY(c, c->errflag.ensure(16), "error flag alloc");
+      P2_TRY(c, cudaMemsetAsync(c->errflag.p, 0, 16, c->stream), "error flag clear");
+    }
+    if ((st = split_prepare_tables(c, pl, what, nmtile, nkstep)) != P2_OK) return st;
+  }
 
   // chunk of slices: FP32 position buffer within the workspace budget; a
   // chunk may hold slices of many requests (a batch of sources), so up to
   // all of the batch's slices go into one chunk
+  const size_t s1_slice = ap ? (size_t)c->Ll[1] * c->Ll[2] * ap->R1 * K * 8 : 0;
   const size_t per_slice = (size_t)K * c->V3 * 8;
   size_t nslices = 0;
   for (int q = 0; q < nidx; q++) nslices += (size_t)std::max(reqs[idx[q]].totalT, 0);
@@ -336,7 +352,10 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
   const int mx = w.max_n;
   P2_TRY(c, c->cbuf.ensure((size_t)mx * per_slice), "position buffer alloc");
   P2_TRY(c, c->expb.ensure((size_t)2 * mx * sizeof(int)), "exponent alloc");
-  P2_TRY(c, c->cmaxb.ensure((size_t)mx * K * sizeof(int)), "maxima alloc");
+  if (ap)
+    P2_TRY(c, c->axes_s1.ensure(std::max(kMinWorkspace, (size_t)mx * s1_slice)), "projection workspace");
+  else
+    P2_TRY(c, c->cmaxb.ensure((size_t)mx * K * sizeof(int)), "maxima alloc");
   Stager sg(c, props, reqs, w);
   sg.cvt32 = all_host64;
   if ((st = sg.prepare(outs)) != P2_OK) return st;
@@ -353,7 +372,7 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
       p2::SampleArgs sa{dsl, chunk_fp32, (int)c->V3, n, (int*)c->expb.p};
       P2_TRY(c, p2::launch_sample_exponents(sa, c->stream), "exponent sample");
     }
-    P2_TRY(c, cudaMemsetAsync(c->cmaxb.p, 0, (size_t)n * K * sizeof(int), c->stream), "maxima clear");
+    if (!ap) P2_TRY(c, cudaMemsetAsync(c->cmaxb.p, 0, (size_t)n * K * sizeof(int), c->stream), "maxima clear");
     p2::ContractArgs a{};
     a.sl = dsl;
     a.V3 = (int)c->V3;
@@ -363,7 +382,7 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     a.k = offsets_of(what);
     a.out = c->cbuf.p;
     a.exps = (const int*)c->expb.p;
-    a.cmax = (int*)c->cmaxb.p;
+    a.cmax = ap ? nullptr : (int*)c->cmaxb.p;  // the scales of the FP16 split
     a.g16_raw = g16_raw(what) ? 1 : 0;
     {
       ProfScope ps(c, "contract_f32");
@@ -372,9 +391,20 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     if ((st = sg.release((int)ci)) != P2_OK) return st;
     if ((st = sg.issue((int)ci + 2)) != P2_OK) return st;
     const int* kexp = (const int*)c->kexp.p;
-    if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, (const int*)c->expb.p, kexp, pl.blocks, nullptr, 0,
-                            0, g16_phase_deferred(what) ? kexp + 2 * K : nullptr)) != P2_OK)
+    const int* kphase = g16_phase_deferred(what) ? kexp + 2 * K : nullptr;
+    if (ap) {
+      if ((st = axes_x_blocks(c, *ap, pl, what, what, c->cbuf.p, 1, n, c->axes_s1.p)) != P2_OK) return st;
+      AxesOut ao;
+      ao.dsl = dsl;
+      ao.exps = (const int*)c->expb.p;
+      ao.kexp = kexp;
+      ao.kphase = kphase;
+      ao.blocks = &pl.blocks;
+      if ((st = axes_yz(c, *ap, c->axes_s1.p, 1, n, K, ao)) != P2_OK) return st;
+    } else if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, (const int*)c->expb.p, kexp, pl.blocks, nullptr,
+                                   0, 0, kphase)) != P2_OK) {
       return st;
+    }
     if (g16_raw(what)) {
       // the Gamma sums of the 16 x 16 block on its projected colour products
       p2::MesonGammaArgs mg{};

@@ -27,7 +27,7 @@
 //
 // Sums over x: FP64 for FP64 input, FP32 for FP32 input (sequential over one
 // row of Lx sites by one thread, so a row's sum does not depend on the launch
-// shape); sums over y and z: FP64, in a fixed order.
+// shape); over y likewise; over z in FP64.  All in a fixed order.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -135,63 +135,100 @@ __global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
     const int ln = lane + 32 * j;
     const int k = kg * a.KL + (ln & (a.KL - 1)), row = rg * rows_per + (ln >> lg);
     if (k < a.K && row < a.rows) {
-      Cx<R>* o = (Cx<R>*)a.s1 + (((long long)tau * a.rows + row) * R1) * a.K + k;
+      Cx<R>* o = (Cx<R>*)a.s1 + (((long long)tau * a.rows + row) * R1) * a.Kst + k;
 #pragma unroll
-      for (int r = 0; r < R1; r++) o[(long long)r * a.K] = acc[j][r];
+      for (int r = 0; r < R1; r++) o[(long long)r * a.Kst] = acc[j][r];
     }
   }
 }
 
 // ---- sums over y ----------------------------------------------------------------
 // Warp r of a block takes x row r of (slice, z) for 32 or 64 components (KPL
-// per lane): every value of S1 is read once and used for all the pairs of r.
-template <typename R, int NY, int KPL>
-__global__ void __launch_bounds__(32 * kAxisMaxRows) k_axis_y(const AxisYArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* yt = (double*)smem_raw;  // [Ly][RY]
-  for (int i = threadIdx.x; i < a.Ly * a.RY; i += blockDim.x) yt[i] = a.yt[i];
-  __syncthreads();
-  const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tau = blockIdx.z, z = blockIdx.y, k0 = blockIdx.x * 32 * KPL + lane;
-  const int first = a.first[r], cnt = a.first[r + 1] - first;
-  if (cnt == 0) return;  // a padding row
-  int ys[NY];
+// per lane): every value of S1 is read once and used for all the pairs of r,
+// U rows y at a time (their loads are in flight together, and vector loads
+// bring the phases of several y), zper values of z one after the other.  The body is instantiated for the number of
+// pairs, so the rows with few of them spend nothing on the others.
+template <typename R, int N, int KPL, int U>
+__device__ __forceinline__ void axis_y_body(const AxisYArgs& a, const R* yt, int LyP, int r, int first) {
+  const int lane = threadIdx.x & 31, tau = blockIdx.z, k0 = blockIdx.x * 32 * KPL + lane;
+  const R* row[N];
 #pragma unroll
-  for (int j = 0; j < NY; j++) ys[j] = a.ylist[first + min(j, cnt - 1)];
-  Cx<double> acc[NY][KPL];
-#pragma unroll
-  for (int j = 0; j < NY; j++)
-#pragma unroll
-    for (int q = 0; q < KPL; q++) acc[j][q] = czero<double>();
+  for (int j = 0; j < N; j++) row[j] = yt + a.ylist[first + j] * LyP;
   const long long rs = (long long)a.R1 * a.K;  // one row of S1
-  const Cx<R>* s = (const Cx<R>*)a.s1 + ((long long)tau * a.Lz + z) * a.Ly * rs + (long long)r * a.K;
-#pragma unroll 4
-  for (int y = 0; y < a.Ly; y++) {
-    Cx<R> v[KPL];
+#pragma unroll 1
+  for (int z = blockIdx.y * a.zper; z < min(a.Lz, (int)(blockIdx.y + 1) * a.zper); z++) {
+    Cx<R> acc[N][KPL];
 #pragma unroll
-    for (int q = 0; q < KPL; q++) v[q] = k0 + 32 * q < a.K ? s[y * rs + k0 + 32 * q] : czero<R>();
+    for (int j = 0; j < N; j++)
 #pragma unroll
-    for (int j = 0; j < NY; j++) {
-      const double f = yt[y * a.RY + ys[j]];
+      for (int q = 0; q < KPL; q++) acc[j][q] = czero<R>();
+    const Cx<R>* s = (const Cx<R>*)a.s1 + ((long long)tau * a.Lz + z) * a.Ly * rs + (long long)r * a.K;
+#pragma unroll 1
+    for (int y0 = 0; y0 < a.Ly; y0 += U) {
+      Cx<R> v[U][KPL];
 #pragma unroll
-      for (int q = 0; q < KPL; q++) {
-        acc[j][q].x = fma(f, (double)v[q].x, acc[j][q].x);
-        acc[j][q].y = fma(f, (double)v[q].y, acc[j][q].y);
+      for (int i = 0; i < U; i++)
+#pragma unroll
+        for (int q = 0; q < KPL; q++)
+          v[i][q] = y0 + i < a.Ly && k0 + 32 * q < a.K ? s[(y0 + i) * rs + k0 + 32 * q] : czero<R>();
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        R f[U];  // zero beyond Ly
+        constexpr int kVec = 16 / (int)sizeof(R);
+#pragma unroll
+        for (int i = 0; i < U; i += kVec)
+          *reinterpret_cast<float4*>(f + i) = *reinterpret_cast<const float4*>(row[j] + y0 + i);
+#pragma unroll
+        for (int i = 0; i < U; i++)
+#pragma unroll
+          for (int q = 0; q < KPL; q++) {
+            acc[j][q].x = fma(f[i], v[i][q].x, acc[j][q].x);
+            acc[j][q].y = fma(f[i], v[i][q].y, acc[j][q].y);
+          }
       }
     }
+    Cx<R>* o = (Cx<R>*)a.s2 + (((long long)tau * a.Lz + z) * a.NP + first) * a.K;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+#pragma unroll
+      for (int q = 0; q < KPL; q++)
+        if (k0 + 32 * q < a.K) o[(long long)j * a.K + k0 + 32 * q] = acc[j][q];
   }
-  Cx<double>* o = (Cx<double>*)a.s2 + (((long long)tau * a.Lz + z) * a.NP + first) * a.K;
-#pragma unroll
-  for (int j = 0; j < NY; j++)
-#pragma unroll
-    for (int q = 0; q < KPL; q++)
-      if (j < cnt && k0 + 32 * q < a.K) o[(long long)j * a.K + k0 + 32 * q] = acc[j][q];
+}
+
+constexpr int kYUnroll = 8;
+
+template <typename R, int KPL>
+__global__ void __launch_bounds__(32 * kAxisMaxRows) k_axis_y(const __grid_constant__ AxisYArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int U = sizeof(R) * KPL == 16 ? kYUnroll / 2 : kYUnroll;
+  R* yt = (R*)smem_raw;  // [RY][Ly rounded up]
+  const int LyP = (a.Ly + kYUnroll - 1) / kYUnroll * kYUnroll;
+  for (int i = threadIdx.x; i < a.RY * LyP; i += blockDim.x) {
+    const int y = i % LyP;
+    yt[i] = y < a.Ly ? (R)a.yt[(i / LyP) * a.Ly + y] : R(0);
+  }
+  __syncthreads();
+  const int r = threadIdx.x >> 5;
+  const int first = a.first[r], cnt = a.first[r + 1] - first;
+  switch (cnt) {  // 0: a padding row
+    case 1: axis_y_body<R, 1, KPL, U>(a, yt, LyP, r, first); break;
+    case 2: axis_y_body<R, 2, KPL, U>(a, yt, LyP, r, first); break;
+    case 3: axis_y_body<R, 3, KPL, U>(a, yt, LyP, r, first); break;
+    case 4: axis_y_body<R, 4, KPL, U>(a, yt, LyP, r, first); break;
+    case 5: axis_y_body<R, 5, KPL, U>(a, yt, LyP, r, first); break;
+    case 6: axis_y_body<R, 6, KPL, U>(a, yt, LyP, r, first); break;
+    case 7: axis_y_body<R, 7, KPL, U>(a, yt, LyP, r, first); break;
+    case 8: axis_y_body<R, 8, KPL, U>(a, yt, LyP, r, first); break;
+    case 9: axis_y_body<R, 9, KPL, U>(a, yt, LyP, r, first); break;
+  }
 }
 
 // ---- sums over z and the results --------------------------------------------------
 // One block per (orbit, slice, 128 components): the eight real-phase sums of
-// an orbit, its up to eight momenta, the un-scaling, the source phase and the
-// result layout.
+// an orbit in FP64, its up to eight momenta, the un-scaling, the source phase
+// and the result layout.
+template <typename R>
 __global__ void __launch_bounds__(128) k_axis_z(const AxisZArgs a) {
   const int ob = blockIdx.x, tl = blockIdx.y, k = blockIdx.z * 128 + threadIdx.x;
   if (k >= a.K) return;
@@ -203,7 +240,7 @@ __global__ void __launch_bounds__(128) k_axis_z(const AxisZArgs a) {
   Cx<double> A[4][2];
 #pragma unroll
   for (int i = 0; i < 4; i++) A[i][0] = A[i][1] = czero<double>();
-  const Cx<double>* s = (const Cx<double>*)a.s2 + (long long)tl * a.Lz * a.NP * a.K + k;
+  const Cx<R>* s = (const Cx<R>*)a.s2 + (long long)tl * a.Lz * a.NP * a.K + k;
   const long long zstep = (long long)a.NP * a.K;
 #pragma unroll 2
   for (int z = 0; z < a.Lz; z++) {
@@ -211,11 +248,11 @@ __global__ void __launch_bounds__(128) k_axis_z(const AxisZArgs a) {
 #pragma unroll
     for (int i = 0; i < 4; i++)
       if (pr[i] >= 0) {
-        const Cx<double> v = s[z * zstep + (long long)pr[i] * a.K];
-        A[i][0].x = fma(fc, v.x, A[i][0].x);
-        A[i][0].y = fma(fc, v.y, A[i][0].y);
-        A[i][1].x = fma(fs, v.x, A[i][1].x);
-        A[i][1].y = fma(fs, v.y, A[i][1].y);
+        const Cx<R> v = s[z * zstep + (long long)pr[i] * a.K];
+        A[i][0].x = fma(fc, (double)v.x, A[i][0].x);
+        A[i][0].y = fma(fc, (double)v.y, A[i][0].y);
+        A[i][1].x = fma(fs, (double)v.x, A[i][1].x);
+        A[i][1].y = fma(fs, (double)v.y, A[i][1].y);
       }
   }
   double f = 1.0;
@@ -281,30 +318,20 @@ cudaError_t launch_x_t(const AxisXArgs& a, cudaStream_t s) {
   return cudaErrorInvalidValue;
 }
 
-template <typename R, int NY>
-cudaError_t launch_y_n(const AxisYArgs& a, int kpl, cudaStream_t s) {
-  const int smem = a.Ly * a.RY * 8;
-  const dim3 grid((a.K + 32 * kpl - 1) / (32 * kpl), a.Lz, a.ntau);
-  const void* f = kpl == 2 ? (const void*)k_axis_y<R, NY, 2> : (const void*)k_axis_y<R, NY, 1>;
+template <typename R, int KPL>
+cudaError_t launch_y(const AxisYArgs& a0, cudaStream_t s) {
+  AxisYArgs a = a0;
+  // as many z per block as leave about eight blocks per SM: a block fills the phase table first
+  const long long per_z = (long long)((a.K + 32 * KPL - 1) / (32 * KPL)) * a.ntau;
+  a.zper = (int)std::max<long long>(1, std::min<long long>(a.Lz, per_z * a.Lz / (8 * 148)));
+  const int smem = a.RY * ((a.Ly + kYUnroll - 1) / kYUnroll * kYUnroll) * (int)sizeof(R);
   if (smem > 48 << 10) {
-    cudaError_t e = ensure_smem(f, smem);
+    cudaError_t e = ensure_smem((const void*)k_axis_y<R, KPL>, smem);
     if (e != cudaSuccess) return e;
   }
-  if (kpl == 2)
-    k_axis_y<R, NY, 2><<<grid, 32 * a.R1, smem, s>>>(a);
-  else
-    k_axis_y<R, NY, 1><<<grid, 32 * a.R1, smem, s>>>(a);
+  const dim3 grid((a.K + 32 * KPL - 1) / (32 * KPL), (a.Lz + a.zper - 1) / a.zper, a.ntau);
+  k_axis_y<R, KPL><<<grid, 32 * a.R1, smem, s>>>(a);
   return cudaGetLastError();
-}
-
-template <typename R>
-cudaError_t launch_y_t(const AxisYArgs& a, int kpl, cudaStream_t s) {
-  if (a.ny <= 1) return launch_y_n<R, 1>(a, kpl, s);
-  if (a.ny <= 3) return launch_y_n<R, 3>(a, kpl, s);
-  if (a.ny <= 5) return launch_y_n<R, 5>(a, kpl, s);
-  if (a.ny <= 7) return launch_y_n<R, 7>(a, kpl, s);
-  if (a.ny <= 9) return launch_y_n<R, 9>(a, kpl, s);
-  return cudaErrorInvalidValue;
 }
 
 // The rows of one axis: for every distinct a its cos row and, unless a = 0 or
@@ -347,11 +374,16 @@ cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
 }
 
 cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s) {
-  return fp32 ? launch_y_t<float>(a, kpl, s) : launch_y_t<double>(a, kpl, s);
+  if (fp32) return kpl == 2 ? launch_y<float, 2>(a, s) : launch_y<float, 1>(a, s);
+  return kpl == 2 ? launch_y<double, 2>(a, s) : launch_y<double, 1>(a, s);
 }
 
-cudaError_t launch_axis_z(const AxisZArgs& a, cudaStream_t s) {
-  k_axis_z<<<dim3(a.NO, a.ntau, (a.K + 127) / 128), 128, 0, s>>>(a);
+cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s) {
+  const dim3 grid(a.NO, a.ntau, (a.K + 127) / 128);
+  if (fp32)
+    k_axis_z<float><<<grid, 128, 0, s>>>(a);
+  else
+    k_axis_z<double><<<grid, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -404,11 +436,9 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
         use(i ? ax[0].sin_row[ia[3 * p]] : ax[0].cos_row[ia[3 * p]],
             j ? ax[1].sin_row[ia[3 * p + 1]] : ax[1].cos_row[ia[3 * p + 1]]);
   std::vector<int> first(R1 + 1, 0), yl;
-  int ny = 1;
   for (int r = 0; r < R1; r++) {
     first[r] = (int)yl.size();
     yl.insert(yl.end(), ylist[r].begin(), ylist[r].end());
-    ny = std::max(ny, (int)ylist[r].size());
   }
   first[R1] = (int)yl.size();
   auto pair_of = [&](int r, int s) {
@@ -454,16 +484,12 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
     for (int r = 0; r < R1; r++)
       tab.push_back(r < (int)ax[0].row_a.size() ? value(0, ax[0].row_a[r], ax[0].row_sin[r], x) : 0.0);
   const size_t oy = tab.size();
-  for (int y = 0; y < c->Ll[1]; y++)
-    for (int r = 0; r < RY; r++) tab.push_back(value(1, ax[1].row_a[r], ax[1].row_sin[r], y));
+  for (int r = 0; r < RY; r++)
+    for (int y = 0; y < c->Ll[1]; y++) tab.push_back(value(1, ax[1].row_a[r], ax[1].row_sin[r], y));
   const size_t oz = tab.size();
   for (int r = 0; r < RZ; r++)
     for (int z = 0; z < c->Ll[2]; z++) tab.push_back(value(2, ax[2].row_a[r], ax[2].row_sin[r], z));
-  std::vector<int> idx(first);
-  const size_t ol = idx.size();
-  idx.insert(idx.end(), yl.begin(), yl.end());
-  const size_t oo = idx.size();
-  idx.insert(idx.end(), orb.begin(), orb.end());
+  std::vector<int> idx(orb);
   const size_t om = idx.size();
   idx.insert(idx.end(), omom.begin(), omom.end());
   p2_status st;
@@ -473,25 +499,27 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
   ap.RY = RY;
   ap.NP = (int)yl.size();
   ap.NO = (int)members.size();
-  ap.ny = ny;
   ap.nmom = nmom;
   ap.xt = (const double*)ap.tab.p;
   ap.yt = ap.xt + oy;
   ap.zt = ap.xt + oz;
-  ap.first = (const int*)ap.idx.p;
-  ap.ylist = ap.first + ol;
-  ap.orb = ap.first + oo;
-  ap.omom = ap.first + om;
+  ap.first = first;
+  ap.ylist = yl;
+  ap.orb = (const int*)ap.idx.p;
+  ap.omom = ap.orb + om;
   ap.usable = true;
   ap.key = moms;
   *out = &ap;
   return P2_OK;
 }
 
+// Sums over x of n slices of K components of a position buffer into the
+// first K of the Kst components of s1.
 p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
-                 void* s1) {
+                 int Kst, void* s1) {
   p2::AxisXArgs a{};
   a.c = field;
+  a.Kst = Kst;
   a.sT = sT;
   a.sK = sK;
   a.ntau = n;
@@ -506,11 +534,34 @@ p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, lon
   return P2_OK;
 }
 
+p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
+                        int fp32, int n, void* s1) {
+  const size_t esz = fp32 ? 8 : 16;
+  // runs of neighbouring blocks; pl.blocks follows kBlocks
+  int k0 = 0, k1 = 0;
+  for (size_t i = 0; i <= sizeof(kBlocks) / sizeof(kBlocks[0]); i++) {
+    const bool end = i == sizeof(kBlocks) / sizeof(kBlocks[0]);
+    if (!end && !(what & kBlocks[i].bit)) continue;
+    const int comps = end ? 0 : kBlocks[i].groups * kBlocks[i].datasets * kBlocks[i].comps;
+    if (!end && (bits & kBlocks[i].bit)) {
+      k1 += comps;
+      continue;
+    }
+    if (k1 > k0) {
+      p2_status st = axes_x(c, ap, (const char*)cbuf + (size_t)k0 * c->V3 * esz, fp32, (long long)pl.K * c->V3, c->V3,
+                            n, k1 - k0, pl.K, (char*)s1 + (size_t)k0 * esz);
+      if (st != P2_OK) return st;
+    }
+    k0 = k1 = k1 + comps;
+  }
+  return P2_OK;
+}
+
 // Sums over y and z of S1 (n slices, K components), then the results: with
 // blocks into the slices' results dsl, otherwise into out[tau * oT + k * oK + p].
 p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o) {
   const int Lz = c->Ll[2];
-  P2_TRY(c, c->axes_s2.ensure((size_t)n * Lz * ap.NP * K * 16), "projection workspace");
+  P2_TRY(c, c->axes_s2.ensure((size_t)n * Lz * ap.NP * K * (fp32 ? 8 : 16)), "projection workspace");
   p2::AxisYArgs y{};
   y.s1 = s1;
   y.s2 = c->axes_s2.p;
@@ -521,13 +572,13 @@ p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n
   y.R1 = ap.R1;
   y.RY = ap.RY;
   y.NP = ap.NP;
-  y.ny = ap.ny;
   y.yt = ap.yt;
-  y.first = ap.first;
-  y.ylist = ap.ylist;
+  std::copy(ap.first.begin(), ap.first.end(), y.first);
+  std::copy(ap.ylist.begin(), ap.ylist.end(), y.ylist);
   // two components per lane share each phase; one where that leaves too few blocks to fill the SMs
-  std::vector<std::vector<int>> cands{{2}, {1}};
-  if ((long long)n * Lz * ((K + 63) / 64) < 2LL * c->nsm) std::swap(cands[0], cands[1]);
+  // (FP64: the registers of two halve the warps in flight)
+  std::vector<std::vector<int>> cands{{1}, {2}};
+  if (fp32 && (long long)n * Lz * ((K + 63) / 64) >= 2LL * c->nsm) std::swap(cands[0], cands[1]);
   char key[160];
   std::snprintf(key, sizeof(key), "%s axes V3=%lld K=%d nmom=%d n=%d", fp32 ? "project_split" : "project_fp64", c->V3, K,
                 ap.nmom, n);
@@ -564,7 +615,7 @@ p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n
   z.oT = o.oT;
   z.oK = o.oK;
   ProfScope ps(c, "project_axis_z");
-  P2_TRY(c, p2::launch_axis_z(z, c->stream), "projection over z");
+  P2_TRY(c, p2::launch_axis_z(z, fp32, c->stream), "projection over z");
   return P2_OK;
 }
 

@@ -683,7 +683,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
       if (ap) {
         P2_TRY(c, c->axes_s1.ensure((size_t)n * c->Ll[1] * c->Ll[2] * ap->R1 * K * (split ? 8 : 16)),
                "projection workspace");
-        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, c->axes_s1.p)) != P2_OK)
+        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, K, c->axes_s1.p)) != P2_OK)
           return st;
         AxesOut ao;
         ao.dsl = dsl;
