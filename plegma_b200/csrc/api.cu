@@ -134,6 +134,14 @@ Work make_work(const p2_ctx* c, const p2_prop* props, const p2_request* reqs, co
   return w;
 }
 
+bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int nidx) {
+  for (int q = 0; q < nidx; q++) {
+    const p2_request& r = reqs[idx[q]];
+    if (props[r.prop_u].location == P2_HOST || props[r.prop_d].location == P2_HOST) return true;
+  }
+  return false;
+}
+
 Stager::Stager(p2_ctx* ctx, const p2_prop* pp, const p2_request* rr, const Work& work)
     : c(ctx), props(pp), reqs(rr), w(work) {
   for (const SliceRef& s : w.sl) {
@@ -515,12 +523,17 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     c->plain_moms_key = pl.moms;
   }
 
-  const size_t s1_slice = ap ? (size_t)c->Ll[1] * c->Ll[2] * ap->R1 * pl.K * 16 : 0;
-  const int tc = chunk_slices(c, pl.K);
+  const unsigned fused = fused_bits(c, ap, what), rest = what & ~fused;
+  const size_t s1_slice = ap ? axes_s1_bytes(c, *ap, 0, 1, pl.K) : 0;
+  // without a position buffer (host propagators keep its chunks: their staging
+  // buffers hold a chunk each, and the copies overlap the chunk before)
+  const bool whole = !rest && !any_host(props, reqs, idx, nidx);
+  const int tc = whole ? (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(s1_slice, 1), (size_t)c->T))
+                       : chunk_slices(c, pl.K);
   const Work w = make_work(c, props, reqs, idx, nidx, tc);
   if (w.sl.empty()) return P2_OK;
-  P2_TRY(c, c->cbuf.ensure((size_t)w.max_n * pl.K * c->V3 * 16), "position buffer alloc");
-  if (ap) P2_TRY(c, c->axes_s1.ensure(std::max(kMinWorkspace, (size_t)w.max_n * s1_slice)), "projection workspace");
+  if (rest) P2_TRY(c, c->cbuf.ensure((size_t)w.max_n * pl.K * c->V3 * 16), "position buffer alloc");
+  if (ap) P2_TRY(c, c->axes_ws.ensure(axes_ws_start(c, *ap, 0, w.max_n, pl.K)), "projection workspace");
   Stager sg(c, props, reqs, w);
   if ((st = sg.prepare(outs)) != P2_OK) return st;
 
@@ -538,7 +551,18 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     a.k = offsets_of(what);
     a.out = c->cbuf.p;
     a.g16_raw = p2::g16_raw(what) ? 1 : 0;  // the projection is followed by k_meson_gamma
-    {
+    if (fused) {
+      p2::ContractArgs r = a;
+      r.out = c->axes_ws.p;
+      r.Lx = c->Ll[0];
+      r.R1 = ap->R1;
+      ProfScope ps(c, "contract_site");
+      if ((r.what = fused & (P2_NUCLEON_CG5 | P2_MESON_G16)))
+        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
+      if ((r.what = fused & (P2_DELTA_ISO12 | P2_DELTA_ISO32)))
+        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
+    }
+    if ((a.what = rest)) {
       ProfScope ps(c, "contract_plain_fp64");
       P2_TRY(c, p2::launch_contract_plain(a, c->nsm, c->stream), "contract kernel");
     }
@@ -546,11 +570,11 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     if ((st = sg.issue((int)ci + 2)) != P2_OK) return st;
 
     if (ap) {
-      if ((st = axes_x_blocks(c, *ap, pl, what, what, c->cbuf.p, 0, n, c->axes_s1.p)) != P2_OK) return st;
+      if (rest && (st = axes_x_blocks(c, *ap, pl, what, rest, c->cbuf.p, 0, n, c->axes_ws.p)) != P2_OK) return st;
       AxesOut ao;
       ao.dsl = sg.desc((int)ci);
       ao.blocks = &pl.blocks;
-      if ((st = axes_yz(c, *ap, c->axes_s1.p, 0, n, pl.K, ao)) != P2_OK) return st;
+      if ((st = axes_yz(c, *ap, c->axes_ws.p, 0, n, pl.K, ao)) != P2_OK) return st;
     } else if ((st = project_direct(c, pl, pl.K, n, w.max_n, sg.desc((int)ci), pl.blocks)) != P2_OK) {
       return st;
     }
@@ -583,18 +607,18 @@ p2_status ft_axes(p2_ctx* c, const AxesPlan& ap, const double* field, int dof, i
     P2_TRY(c, c->res.ensure(total * 16), "result alloc");
     dst = (double*)c->res.p;
   }
-  const size_t s1 = (size_t)c->Ll[1] * c->Ll[2] * ap.R1 * dof * 16, per = s1 + (size_t)c->Ll[2] * ap.NP * dof * 16;
+  const size_t per = axes_ws_bytes(c, ap, 0, 1, dof);
   const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)nt));
-  P2_TRY(c, c->axes_s1.ensure((size_t)tc * s1), "projection workspace");
+  P2_TRY(c, c->axes_ws.ensure(axes_ws_bytes(c, ap, 0, tc, dof)), "projection workspace");
   for (int t0 = 0; t0 < nt; t0 += tc) {
     const int n = std::min(tc, nt - t0);
-    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, dof, c->axes_s1.p);
+    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, dof, c->axes_ws.p);
     if (st != P2_OK) return st;
     AxesOut ao;
     ao.oT = (long long)dof * ap.nmom;
     ao.oK = ap.nmom;
     ao.out = dst + 2 * (size_t)t0 * ao.oT;
-    if ((st = axes_yz(c, ap, c->axes_s1.p, 0, n, dof, ao)) != P2_OK) return st;
+    if ((st = axes_yz(c, ap, c->axes_ws.p, 0, n, dof, ao)) != P2_OK) return st;
   }
   if (out_location == P2_HOST) {
     P2_TRY(c, cudaMemcpyAsync(out, dst, total * 16, cudaMemcpyDeviceToHost, c->stream), "result download");
@@ -738,7 +762,7 @@ p2_status p2_ctx_destroy(p2_ctx* c) {
   }
   cudaStreamSynchronize(c->stream);
   for (DevBuf* b : {&c->cbuf, &c->part, &c->tab, &c->res, &c->moms, &c->sdesc, &c->ptab, &c->ft_kexp, &c->axes[0].tab,
-                    &c->axes[0].idx, &c->axes[1].tab, &c->axes[1].idx, &c->axes_s1, &c->axes_s2})
+                    &c->axes[1].tab, &c->axes_ws})
     b->release();
   if (c->sdesc_host) cudaFreeHost(c->sdesc_host);
   if (c->sdesc_copied) cudaEventDestroy(c->sdesc_copied);

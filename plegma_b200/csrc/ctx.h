@@ -55,7 +55,8 @@ struct AxesPlan {
   std::vector<int> key;  // momentum list the tables were built for
   bool usable = false;   // the list has few enough rows per axis
   int R1 = 0, RY = 0, NP = 0, NO = 0, nmom = 0;
-  DevBuf tab, idx;
+  DevBuf tab;  // phases, then the orbit lists
+  std::vector<double> xth;  // xt on the host, for the fused contraction
   const double *xt = nullptr, *yt = nullptr, *zt = nullptr;
   std::vector<int> first, ylist;
   const int *orb = nullptr, *omom = nullptr;
@@ -122,7 +123,7 @@ struct p2_ctx {
   p2_udsc_cache* udsc = nullptr;
   // axis-by-axis projection: tables per transform sign (-1, +1), sums over x and over y
   p2host::AxesPlan axes[2];
-  p2host::DevBuf axes_s1, axes_s2;
+  p2host::DevBuf axes_ws;  // S1, then S2 (axes_ws_bytes)
   // launch-shape autotuner (shared with the context's graphs)
   std::shared_ptr<p2host::Tuner> tuner = std::make_shared<p2host::Tuner>();
 
@@ -256,13 +257,22 @@ struct AxesOut {
 p2_status project_direct(p2_ctx* c, const Plan& pl, int K, int n, int max_n, const p2::SliceDesc* dsl,
                          const std::vector<p2::ScatterBlock>& blocks);
 p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const AxesPlan** out);
+// Some propagator of the requests is in host memory.
+bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int nidx);
+// Bits of a contraction set that the kernels fused with the sums over x take.
+unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what);
 // The sums over x of the blocks of `bits` from a position buffer of the whole
 // set `what` (n slices, K components of V3 sites each).
 p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
                         int fp32, int n, void* s1);
-// The sums over x are small; their buffer starts at this size so that calls of
-// different sizes share one allocation.
-constexpr size_t kMinWorkspace = (size_t)64 << 20;
+// Bytes of the sums over x of n slices of K components, and of the workspace
+// that holds them and the sums over y (one allocation: each costs about 0.4 ms
+// of a context's first call).
+size_t axes_s1_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
+size_t axes_ws_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
+// The workspace of a contraction: at least 64 MB where a position buffer would
+// have taken that, so that calls of different sizes share one allocation.
+size_t axes_ws_start(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
 p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
                  int Kst, void* s1);
 p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o);

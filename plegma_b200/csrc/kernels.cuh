@@ -65,6 +65,10 @@ struct ContractArgs {
   // 1: the 16 x 16 block's components are the colour products M of g16_raw
   // (its result goes through the projection and then k_meson_gamma)
   int g16_raw;
+  // fused with the sums over x (contract_site.cuh): out is S1 [ntau][V3 / Lx][R1][K] complex
+  int Lx, R1;
+  // set by the launcher: rows per unit, units per slice, and gridDim.x units as slices and units
+  int unit, upt, step_slice, step_unit;
 };
 
 // Per-slice magnitude exponents of the u and d views, from a strided sample.
@@ -231,6 +235,14 @@ cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s);
 cudaError_t launch_contract_plain(const ContractArgs& a, int grid, cudaStream_t s);
 // FP32 site contraction; fp32_in selects complex-float propagators.
 cudaError_t launch_contract_f32(const ContractArgs& a, int fp32_in, int grid, cudaStream_t s);
+// Fused with the sums over x (contract_site.cuh), split or plain form: the
+// nucleon and the colour products of the 16 x 16 mesons; the Delta.  xt
+// [Lx][R1] the phase rows.
+cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                               cudaStream_t s);
+cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                              cudaStream_t s);
+constexpr int kRowsMaxPhases = 960;  // Lx x phase rows (4, 8 or 12) of the fused kernels' parameter block
 cudaError_t launch_sample_exponents(const SampleArgs& a, cudaStream_t s);
 cudaError_t launch_project_fp64(const ProjArgs& a, cudaStream_t s);
 int project_fp64_tk(int K, int tk);  // component tile factor a launch with ProjArgs::tk uses

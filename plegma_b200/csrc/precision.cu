@@ -337,11 +337,17 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     if ((st = split_prepare_tables(c, pl, what, nmtile, nkstep)) != P2_OK) return st;
   }
 
+  const unsigned fused = fused_bits(c, ap, what);
+  const unsigned rest = what & ~fused;
+
   // chunk of slices: FP32 position buffer within the workspace budget; a
   // chunk may hold slices of many requests (a batch of sources), so up to
   // all of the batch's slices go into one chunk
-  const size_t s1_slice = ap ? (size_t)c->Ll[1] * c->Ll[2] * ap->R1 * K * 8 : 0;
-  const size_t per_slice = (size_t)K * c->V3 * 8;
+  const size_t s1_slice = ap ? axes_s1_bytes(c, *ap, 1, 1, K) : 0;
+  const size_t cb_slice = rest ? (size_t)K * c->V3 * 8 : 0;
+  // without a position buffer (host propagators keep its chunks: their staging
+  // buffers hold a chunk each, and the copies overlap the chunk before)
+  const size_t per_slice = !any_host(props, reqs, idx, nidx) ? std::max(cb_slice, s1_slice) : (size_t)K * c->V3 * 8;
   size_t nslices = 0;
   for (int q = 0; q < nidx; q++) nslices += (size_t)std::max(reqs[idx[q]].totalT, 0);
   int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per_slice, 1),
@@ -350,10 +356,10 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
   const Work w = make_work(c, props, reqs, idx, nidx, tc);
   if (w.sl.empty()) return P2_OK;
   const int mx = w.max_n;
-  P2_TRY(c, c->cbuf.ensure((size_t)mx * per_slice), "position buffer alloc");
+  if (rest) P2_TRY(c, c->cbuf.ensure((size_t)mx * cb_slice), "position buffer alloc");
   P2_TRY(c, c->expb.ensure((size_t)2 * mx * sizeof(int)), "exponent alloc");
   if (ap)
-    P2_TRY(c, c->axes_s1.ensure(std::max(kMinWorkspace, (size_t)mx * s1_slice)), "projection workspace");
+    P2_TRY(c, c->axes_ws.ensure(axes_ws_start(c, *ap, 1, mx, K)), "projection workspace");
   else
     P2_TRY(c, c->cmaxb.ensure((size_t)mx * K * sizeof(int)), "maxima alloc");
   Stager sg(c, props, reqs, w);
@@ -377,14 +383,24 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     a.sl = dsl;
     a.V3 = (int)c->V3;
     a.ntau = n;
-    a.what = what;
     a.K = K;
     a.k = offsets_of(what);
     a.out = c->cbuf.p;
     a.exps = (const int*)c->expb.p;
     a.cmax = ap ? nullptr : (int*)c->cmaxb.p;  // the scales of the FP16 split
     a.g16_raw = g16_raw(what) ? 1 : 0;
-    {
+    if (fused) {
+      p2::ContractArgs r = a;
+      r.out = c->axes_ws.p;
+      r.Lx = c->Ll[0];
+      r.R1 = ap->R1;
+      ProfScope ps(c, "contract_site");
+      if ((r.what = fused & (P2_NUCLEON_CG5 | P2_MESON_G16)))
+        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
+      if ((r.what = fused & (P2_DELTA_ISO12 | P2_DELTA_ISO32)))
+        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
+    }
+    if ((a.what = rest)) {
       ProfScope ps(c, "contract_f32");
       P2_TRY(c, p2::launch_contract_f32(a, chunk_fp32, 2 * c->nsm, c->stream), "contract kernel");
     }
@@ -393,14 +409,14 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     const int* kexp = (const int*)c->kexp.p;
     const int* kphase = g16_phase_deferred(what) ? kexp + 2 * K : nullptr;
     if (ap) {
-      if ((st = axes_x_blocks(c, *ap, pl, what, what, c->cbuf.p, 1, n, c->axes_s1.p)) != P2_OK) return st;
+      if (rest && (st = axes_x_blocks(c, *ap, pl, what, rest, c->cbuf.p, 1, n, c->axes_ws.p)) != P2_OK) return st;
       AxesOut ao;
       ao.dsl = dsl;
       ao.exps = (const int*)c->expb.p;
       ao.kexp = kexp;
       ao.kphase = kphase;
       ao.blocks = &pl.blocks;
-      if ((st = axes_yz(c, *ap, c->axes_s1.p, 1, n, K, ao)) != P2_OK) return st;
+      if ((st = axes_yz(c, *ap, c->axes_ws.p, 1, n, K, ao)) != P2_OK) return st;
     } else if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, (const int*)c->expb.p, kexp, pl.blocks, nullptr,
                                    0, 0, kphase)) != P2_OK) {
       return st;

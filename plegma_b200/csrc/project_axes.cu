@@ -24,6 +24,13 @@
 // momenta 4.17 ms instead of 14.12 ms (the projection was 10.8 ms of it), the
 // transform of a 32-component field there 0.14 ms instead of 2.18 ms.  Error
 // against 64 bits 1.7e-15 instead of 4.0e-15 (fewer terms per sum).
+// Split form, against the tensor-core projection (which larger lists keep):
+// 8^3 x 16 with 288 components 96 us instead of 101, 24^3 x 48 light baryons
+// 4.77 ms instead of 5.34, 64^3 x 128 with K = 480 and 123 momenta 22.3 ms
+// instead of 29.4 (with the Delta); error against 64 bits 2e-7 instead of 1e-6
+// (an FP32 sum over one row at a time, no split of the data into FP16 parts).
+// Without the fused contraction (contract_site.cuh) 48^3 slices gain only 2 %:
+// the position buffer's write and read bound both.
 //
 // Sums over x: FP64 for FP64 input, FP32 for FP32 input (sequential over one
 // row of Lx sites by one thread, so a row's sum does not depend on the launch
@@ -31,6 +38,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "ctx.h"
@@ -493,24 +501,38 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
   const size_t om = idx.size();
   idx.insert(idx.end(), omom.begin(), omom.end());
   p2_status st;
-  if ((st = upload_async(c, ap.tab, tab.data(), tab.size() * sizeof(double), "axis phases")) != P2_OK) return st;
-  if ((st = upload_async(c, ap.idx, idx.data(), idx.size() * sizeof(int), "axis momenta")) != P2_OK) return st;
+  std::vector<unsigned char> up(tab.size() * sizeof(double) + idx.size() * sizeof(int));
+  std::memcpy(up.data(), tab.data(), tab.size() * sizeof(double));
+  std::memcpy(up.data() + tab.size() * sizeof(double), idx.data(), idx.size() * sizeof(int));
+  if ((st = upload_async(c, ap.tab, up.data(), up.size(), "axis tables")) != P2_OK) return st;
   ap.R1 = R1;
   ap.RY = RY;
   ap.NP = (int)yl.size();
   ap.NO = (int)members.size();
   ap.nmom = nmom;
+  ap.xth.assign(tab.begin(), tab.begin() + oy);
   ap.xt = (const double*)ap.tab.p;
   ap.yt = ap.xt + oy;
   ap.zt = ap.xt + oz;
   ap.first = first;
   ap.ylist = yl;
-  ap.orb = (const int*)ap.idx.p;
+  ap.orb = (const int*)(ap.xt + tab.size());
   ap.omom = ap.orb + om;
   ap.usable = true;
   ap.key = moms;
   *out = &ap;
   return P2_OK;
+}
+
+size_t axes_s1_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K) {
+  return (n * c->Ll[1] * c->Ll[2] * ap.R1 * K * (fp32 ? 8 : 16) + 255) / 256 * 256;
+}
+size_t axes_ws_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K) {
+  return axes_s1_bytes(c, ap, fp32, n, K) + n * c->Ll[2] * ap.NP * K * (fp32 ? 8 : 16);
+}
+size_t axes_ws_start(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K) {
+  const size_t buf = n * K * (size_t)c->V3 * (fp32 ? 8 : 16);
+  return std::max(std::min(buf, (size_t)64 << 20), axes_ws_bytes(c, ap, fp32, n, K));
 }
 
 // Sums over x of n slices of K components of a position buffer into the
@@ -532,6 +554,20 @@ p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, lon
   ProfScope ps(c, "project_axis_x");
   P2_TRY(c, p2::launch_axis_x(a, fp32, c->stream), "projection over x");
   return P2_OK;
+}
+
+// The Delta (from the second nucleon interpolator too: they share no work),
+// and the nucleon with the 16 x 16 mesons unless other blocks of their pass
+// are requested; the rest goes through a position buffer.  The Delta alone
+// gains from it beside such blocks (24^3 x 48 light baryons 4.77 -> 4.34 ms, odd
+// plain lattice 2.54 -> 2.39 ms), the nucleon would read its propagators a
+// second time.  Lists and lattices whose x phases exceed the parameters keep
+// the position buffer.
+unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what) {
+  constexpr unsigned kDelta = P2_DELTA_ISO12 | P2_DELTA_ISO32, kMes = P2_NUCLEON_CG5 | P2_MESON_G16;
+  constexpr unsigned kPass2 = kDelta | P2_NUCLEON_NTOR | P2_NUCLEON_RTON | P2_NUCLEON_RTOR;
+  if (!ap || c->Ll[0] * (ap->R1 <= 3 ? 4 : ap->R1 <= 7 ? 8 : 12) > p2::kRowsMaxPhases) return 0;
+  return (what & kDelta) | (what & ~(kPass2 | kMes) ? 0u : what & kMes);
 }
 
 p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
@@ -561,10 +597,10 @@ p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned 
 // blocks into the slices' results dsl, otherwise into out[tau * oT + k * oK + p].
 p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o) {
   const int Lz = c->Ll[2];
-  P2_TRY(c, c->axes_s2.ensure((size_t)n * Lz * ap.NP * K * (fp32 ? 8 : 16)), "projection workspace");
+  void* const s2 = (char*)s1 + axes_s1_bytes(c, ap, fp32, n, K);
   p2::AxisYArgs y{};
   y.s1 = s1;
-  y.s2 = c->axes_s2.p;
+  y.s2 = s2;
   y.ntau = n;
   y.K = K;
   y.Ly = c->Ll[1];
@@ -592,7 +628,7 @@ p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n
     P2_TRY(c, p2::launch_axis_y(y, fp32, pick[0], c->stream), "projection over y");
   }
   p2::AxisZArgs z{};
-  z.s2 = c->axes_s2.p;
+  z.s2 = s2;
   z.ntau = n;
   z.K = K;
   z.Lz = Lz;

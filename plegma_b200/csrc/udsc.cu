@@ -625,6 +625,21 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
   }
   if (!up.empty() && (st = upload_async(c, U.args, up.data(), up.size(), "udsc arguments")) != P2_OK) return st;
 
+  // slices of a chunk; the buffers are sized for the largest group at once
+  const size_t esz = split ? 8 : 16;
+  auto chunk_of = [&](const UdscGroup& g) {
+    const size_t fit = c->ws_budget / std::max<size_t>((size_t)g.K * (size_t)c->V3 * esz, 1);
+    return (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)T));
+  };
+  size_t cbytes = 0, wbytes = 0;
+  for (const UdscGroup& g : groups) {
+    const size_t n = std::min((size_t)chunk_of(g), g.taus.size());
+    cbytes = std::max(cbytes, n * (size_t)g.K * (size_t)c->V3 * esz);
+    if (ap) wbytes = std::max(wbytes, axes_ws_bytes(c, *ap, split, n, g.K));
+  }
+  P2_TRY(c, c->cbuf.ensure(cbytes), "position buffer alloc");
+  if (ap) P2_TRY(c, c->axes_ws.ensure(wbytes), "projection workspace");
+
   for (const UdscGroup& g : groups) {
     const int nf = (int)g.flavours.size(), K = g.K, n_all = (int)g.taus.size();
     UdscArgs a{};
@@ -651,13 +666,11 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
       blocks.push_back(ScatterBlock{k0, 1, nd, 1, (long long)g.ds_off[i]});
       k0 += nd;
     }
-    const size_t per = (size_t)K * c->V3 * (split ? 8 : 16);
-    const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)T));
+    const int tc = chunk_of(g);
     for (int c0 = 0; c0 < n_all; c0 += tc) {
       const int n = std::min(tc, n_all - c0);
       const SliceDesc* dsl = (const SliceDesc*)((const unsigned char*)U.args.p + g.o_desc) + c0;
       const int* kexp = (const int*)((const unsigned char*)U.args.p + g.o_kexp);
-      P2_TRY(c, c->cbuf.ensure((size_t)n * per), "position buffer alloc");
       a.sl = (const UdscSlice*)((const unsigned char*)U.args.p + g.o_sl) + c0;
       a.ntau = n;
       a.out = c->cbuf.p;
@@ -681,9 +694,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
         P2_TRY(c, launch_contract_udsc(a, nf, c->nsm, c->stream), "udsc contraction");
       }
       if (ap) {
-        P2_TRY(c, c->axes_s1.ensure((size_t)n * c->Ll[1] * c->Ll[2] * ap->R1 * K * (split ? 8 : 16)),
-               "projection workspace");
-        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, K, c->axes_s1.p)) != P2_OK)
+        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, K, c->axes_ws.p)) != P2_OK)
           return st;
         AxesOut ao;
         ao.dsl = dsl;
@@ -692,7 +703,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
           ao.exps = a.es;
           ao.kexp = kexp;
         }
-        if ((st = axes_yz(c, *ap, c->axes_s1.p, split, n, K, ao)) != P2_OK) return st;
+        if ((st = axes_yz(c, *ap, c->axes_ws.p, split, n, K, ao)) != P2_OK) return st;
       } else if (split) {
         if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, a.es, kexp, blocks)) != P2_OK) return st;
       } else if ((st = project_direct(c, pl, K, n, n, dsl, blocks)) != P2_OK) {
