@@ -49,10 +49,14 @@ typedef enum {
 typedef enum { P2_FP64 = 0, P2_FP32 = 1 } p2_precision;
 
 /* Arithmetic of a request.
- * P2_PLAIN_FP64: FP64 site contraction, FP64 direct phase sum.
+ * P2_PLAIN_FP64: FP64 site contraction, FP64 projection.
  * P2_SPLIT_FP16: FP32 site contraction with power-of-two scaling per time
- *   slice; projection on the tensor cores as hi+lo FP16 products with FP32
- *   accumulation; FP64 cross-block sums and normalisation. */
+ *   slice; FP32 projection sums within a row and a column of sites, FP64
+ *   beyond and normalisation.
+ * The projection runs one axis at a time when the momenta need at most nine
+ * cosine and sine rows per axis (|n_d| <= 4); other lists take a direct FP64
+ * phase sum, or, split form, the tensor cores with hi+lo FP16 products and FP32
+ * accumulation. */
 typedef enum { P2_PLAIN_FP64 = 0, P2_SPLIT_FP16 = 1 } p2_mode;
 
 typedef enum { P2_DEVICE = 0, P2_HOST = 1 } p2_location;
@@ -266,8 +270,8 @@ int p2_local_taus(p2_ctx* ctx, const p2_prop* props, int nprops, const p2_reques
  * products containing s / c.  Result: [dataset][tau][mom] complex double,
  * datasets in the order of p2_udsc_datasets.  Device-resident propagators:
  * mode P2_PLAIN_FP64 (FP64 arithmetic, FP64 propagators) or P2_SPLIT_FP16
- * (FP32 contraction of power-of-two scaled inputs and the hi+lo FP16
- * tensor-core projection, FP64 or FP32 propagators, per-time-slice error
+ * (FP32 contraction of power-of-two scaled inputs and the split form's
+ * projection, FP64 or FP32 propagators, per-time-slice error
  * <= 1e-6 of sum_x |c_d(x,t)|). */
 typedef struct {
   int source[4];
@@ -312,8 +316,9 @@ p2_status p2_graph_destroy(p2_graph* graph);
 
 /* ---- autotuning -------------------------------------------------------- */
 /* With tuning on, the first call with a new shape times the candidate launch
- * shapes of the tunable kernels (tensor-core projection: N-tile width and
- * site splits; FP64 projection: component tile and site splits) and keeps the
+ * shapes of the tunable kernels (axis-by-axis projection: components per lane
+ * of the sums over y; tensor-core projection: N-tile width and site splits;
+ * direct FP64 projection: component tile and site splits) and keeps the
  * fastest.  Choices are cached per (kernel, shape) for the context and its
  * graphs, and, when cache_path is not NULL, in that tab-separated file (read
  * now, rewritten after each new entry; "key<TAB>params<TAB>ms" per line).
@@ -346,7 +351,8 @@ p2_status p2_profile_enable(p2_ctx* ctx, int on);
 int p2_profile_read(p2_ctx* ctx, p2_kernel_time* out, int max, int reset);
 
 /* Test hook for the device-side failure path: the next tensor-core
- * projection launched on this context (split form, p2_ft_apply_split)
+ * projection launched on this context (the next split request or
+ * p2_ft_apply_split takes it, whatever its momenta)
  * withholds its converters' operand-ready signals and gives every mbarrier
  * wait a short limit, so its waits run out; the kernel records the timeout,
  * waits for its own bulk copies, frees its TMEM and returns, and the next
