@@ -202,17 +202,17 @@ def run_reference(args, rank, world):
 
 
 # DRAM bytes (read + write) per site of the dominant kernel, measured with ncu
-# on the 32^3 x 16 case of the same kernel; traffic grows with the sites a
+# on a 32^3 x 4 (split) and a 24^3 x 8 (plain) case of the same kernel; traffic grows with the sites a
 # launch processes, so it scales to the benchmark's launches
-TRAFFIC_PER_SITE = {("contract_f32", "split"): 6864, ("contract_plain_fp64", "plain"): 9129}
+TRAFFIC_PER_SITE = {("contract_site", "split"): 5057, ("contract_site", "plain"): 5779}
 # executed FP64 flop per site of the plain site contraction (2 per DFMA, 1 per
-# DADD / DMUL, from the ncu instruction counters of the 32^3 x 16 case)
-FP64_FLOP_PER_SITE = {"contract_plain_fp64": 50336}
+# DADD / DMUL, the sums over x included, from the ncu instruction counters of a 24^3 x 8 case)
+FP64_FLOP_PER_SITE = {"contract_site": 56624}
 # LSU data-pipe wavefronts per site of the split site contraction (ncu
-# l1tex__data_pipe_lsu_wavefronts.sum / sites, 32^3 x 16 case): its binding
+# l1tex__data_pipe_lsu_wavefronts.sum / sites, 32^3 x 4 case): an
 # on-chip limit, one wavefront (128 bytes between shared memory and the
 # registers) per SM and clock
-LSU_WAVEFRONTS_PER_SITE = {"contract_f32": 394.8}
+LSU_WAVEFRONTS_PER_SITE = {"contract_site": 297.0}
 
 BATCHED = {
     # name: (lattice, sources, window range, |n|^2 max, propagator precision, decay, seed, sources resident at once)
@@ -470,7 +470,7 @@ def main():
         roof = {"kernel": kname, "bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
                 "frac": ach / hbm, "peak_kind": peak_kind,
                 "traffic": tps * per_launch if tps else None,
-                "traffic_note": "DRAM read+write bytes per site from the ncu capture of the 32^3x16 case, "
+                "traffic_note": "DRAM read+write bytes per site from the ncu capture of a small case, "
                                 "times the sites of one launch" if tps else None,
                 "algorithmic_bytes_per_launch": bytes_per_site * per_launch, "sites_per_launch": per_launch}
     # the split contraction against its on-chip bound: the LSU data pipe's one
@@ -483,12 +483,13 @@ def main():
         floor_ms = wf * sites / (nsm * r["clocks"]["sm_mhz"] * 1e6) * 1e3
         ms_k = kms / args.steps
         roof_lsu = {"kernel": ck[0], "bound": "lsu data pipe (1 wavefront / SM / clock)",
-                    "wavefronts_per_site": wf, "wavefronts_source": "ncu, 32^3x16 case",
+                    "wavefronts_per_site": wf, "wavefronts_source": "ncu, 32^3x4 case",
                     "sm_mhz": r["clocks"]["sm_mhz"], "sms": nsm, "floor_ms_per_step": floor_ms,
                     "ms_per_step": ms_k, "frac": floor_ms / ms_k if ms_k > 0 else None}
-    # the projection against the tensor (split) or FP64 (plain) roofline, algorithmic flop = 8 nmom K per site
+    # the projection where it is a sum of its own over momenta: against the tensor (split) or FP64 (plain)
+    # roofline, algorithmic flop = 8 nmom K per site (the axis-by-axis one spends far fewer: its time is in kernels)
     roof_proj = None
-    pk = [k for k in prof if k.startswith("project")]
+    pk = [k for k in prof if k in ("project_split", "project_fp64")]
     if pk:
         n, kms = prof[pk[0]]
         flop = 8.0 * nmom * K * sites * args.steps
@@ -506,7 +507,7 @@ def main():
         pp = results["plain"]["prof"]
         roof64 = {"peak": fp64_tflops, "unit": "TFLOP/s", "peak_kind": "measured (p2_measure_fp64_rate)"}
         for kname, kms in pp.items():
-            if kname.startswith("project"):
+            if kname == "project_fp64":
                 fl = 8.0 * nmom * K
             elif kname.startswith("contract") and FP64_FLOP_PER_SITE.get(kname):
                 fl = FP64_FLOP_PER_SITE[kname]
@@ -517,10 +518,10 @@ def main():
             ach = fl * sites * args.steps / (kms[1] * 1e-3) / 1e12
             roof64[kname] = {"achieved": ach, "frac": ach / fp64_tflops, "flop_per_site": fl,
                              "flop_kind": "algorithmic" if kname.startswith("project") else "executed (ncu)"}
-        if "contract_plain_fp64" in pp:
-            n, kms = pp["contract_plain_fp64"]
+        if "contract_site" in pp:
+            n, kms = pp["contract_site"]
             ach = 2 * 144 * 16 * sites * args.steps / (kms * 1e-3) / 1e9
-            roof64["contract_plain_fp64_hbm"] = {"achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
+            roof64["contract_site_hbm"] = {"achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                                                  "target_frac": 0.7}
 
     # end to end through the C ABI with host buffers (pinned), copies inside the timed region
