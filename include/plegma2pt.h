@@ -205,8 +205,9 @@ p2_status p2_contract_position(p2_ctx* ctx, const p2_prop* props, int nprops, co
 p2_status p2_ft_apply(p2_ctx* ctx, const double* field, int dof, int nt, const int* moms, int nmom, int sign,
                       double* out, int out_location);
 
-/* The same transform on the tensor cores (the split projection of the
- * contractions): each time slice of the field is scaled by 2^-e (e the binary
+/* The same transform; momentum lists that need more than nine phase rows on an
+ * axis run on the tensor cores (the split projection of the contractions), the
+ * others in FP64 one axis at a time.  On the tensor cores each time slice of the field is scaled by 2^-e (e the binary
  * exponent of its largest entry, exact), converted to FP32 and projected with
  * hi+lo FP16 operands and FP32 accumulation; per (t, component, momentum) the
  * error is <= 1e-6 of sum_x |field(x, t)| of that component. */

@@ -1,5 +1,8 @@
-// Split-FP16 form: orchestration of the FP32 site contraction and the
-// tensor-core projection (project_split.cu) for one or more requests.
+// Split form: orchestration of the FP32 site contraction and the projection
+// for one or more requests.  Momentum lists with few phase rows are projected
+// one axis at a time (project_axes.cu), the sums over x inside the contraction
+// for the blocks of fused_bits; the others on the tensor cores
+// (project_split.cu), which is steps 2 to 4 below.
 //
 // Per chunk of time slices (from one or many requests):
 //   1. per-slice exponents E_u, E_d from a strided sample of each propagator;
