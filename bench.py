@@ -212,7 +212,7 @@ FP64_FLOP_PER_SITE = {"contract_site": 56624}
 # l1tex__data_pipe_lsu_wavefronts.sum / sites, 32^3 x 4 case): an
 # on-chip limit, one wavefront (128 bytes between shared memory and the
 # registers) per SM and clock
-LSU_WAVEFRONTS_PER_SITE = {"contract_site": 297.0}
+LSU_WAVEFRONTS_PER_SITE = {"contract_site": 296.0}
 
 BATCHED = {
     # name: (lattice, sources, window range, |n|^2 max, propagator precision, decay, seed, sources resident at once)

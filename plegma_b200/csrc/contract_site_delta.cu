@@ -19,8 +19,8 @@
 // and after the three pairs the outputs to the output tile and, X, the sums
 // over x.
 // Bound: FMA issue and, in A, the shared-memory loads (18 wavefronts of a
-// block against 36 issue slots of the dots it feeds): split form 1765 clk/site
-// with 3886 warp instructions and 1024 wavefronts; plain form 3326 clk/site,
+// block against 36 issue slots of the dots it feeds): split form 1780 clk/site
+// with 3874 warp instructions and 1024 wavefronts; plain form 3361 clk/site,
 // FP64 pipe 47 %.
 #include "contract_site.cuh"
 

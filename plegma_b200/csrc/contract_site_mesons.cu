@@ -15,10 +15,10 @@
 // of the class itself: z(s) = r in T[m][r] exactly for the class role (r,
 // r ^ 1), so that role adds s D to its Q before its slot terms.  The four
 // roles of the class form D among themselves, the others do not wait.
-// Bound, split form: issue with four warps per scheduler, 674 clk/site (53 %
-// of the slots, 1429 warp instructions, 297 shared-memory wavefronts); half of
-// it is A.  Plain form: FP64 latency at 8 warps per SM, 1205 clk/site (FP64
-// pipe 40 %).  The HBM floor is 196 clk/site.
+// Bound, split form: issue with four warps per scheduler, 662 clk/site (52 %
+// of the slots, 1383 warp instructions, 296 shared-memory wavefronts); half of
+// it is A.  Plain form: FP64 latency at 8 warps per SM, 1176 clk/site (FP64
+// pipe 41 %).  The HBM floor is 196 clk/site.
 #include "contract_site.cuh"
 
 namespace p2 {
