@@ -558,9 +558,9 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
       r.R1 = ap->R1;
       ProfScope ps(c, "contract_site");
       if ((r.what = fused & (P2_NUCLEON_CG5 | P2_MESON_G16)))
-        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), ap->rows, 1, 0, c->nsm, c->stream), "contract kernel");
       if ((r.what = fused & (P2_DELTA_ISO12 | P2_DELTA_ISO32)))
-        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), ap->rows, 1, 0, c->nsm, c->stream), "contract kernel");
     }
     if ((a.what = rest)) {
       ProfScope ps(c, "contract_plain_fp64");

@@ -16,7 +16,8 @@
 // prefetched into L2 during a tile's contraction; its u half is loaded into
 // registers before the last phase of the contraction, its d half before the
 // sums over x, so that both latencies are covered.  A row's sites are added
-// in order by one thread, so a row's sum does not depend on the launch shape.
+// in order by one thread, in the split form by groups that depend on Lx alone
+// (RowGroups), so a row's sum does not depend on the launch shape.
 // The x phases are kernel parameters: they come through the constant bank and
 // cost no shared-memory wavefronts (copied to shared memory the plain form was
 // 14 % slower).
@@ -50,24 +51,31 @@ struct Cfg {
 };
 
 // ---- sums over x -----------------------------------------------------------------
-// [Lx][phase_stride(RT)]
+// t: [Lx][phase_stride(RT)]; g: the groups of a row (split form)
 template <typename R>
 struct __align__(16) XPhases {
   R t[kRowsMaxPhases];
+  RowGroups g;
 };
 __host__ __device__ constexpr int phase_stride(int RT) { return (RT + 3) / 4 * 4; }
 
 // Sums of one output position for N units of phase rows: FP32 a unit is a
-// packed pair of rows (one paired FMA for both), FP64 one row.
+// packed pair of rows (one paired FMA for both), FP64 one row.  FP32 sums run
+// over a group of sites (RowGroups) and fold() adds the group to the row's.
 template <typename R, int N>
 struct RowSums;
 template <int N>
 struct RowSums<float, N> {
   static constexpr int kRows = 2;  // rows per unit
-  f32x2 re[N], im[N];
+  f32x2 re[N], im[N];    // the row's groups
+  f32x2 gre[N], gim[N];  // the group
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < N; i++) re[i] = im[i] = f2pack(0.f, 0.f);
+  }
+  __device__ __forceinline__ void begin() {
+#pragma unroll
+    for (int i = 0; i < N; i++) gre[i] = gim[i] = f2pack(0.f, 0.f);
   }
   __device__ __forceinline__ void add(const float* f, Cx<float> v) {
     const f32x2 vx = f2pack(v.x, v.x), vy = f2pack(v.y, v.y);
@@ -75,9 +83,17 @@ struct RowSums<float, N> {
 #pragma unroll
     for (int i = 0; i < N; i++) {
       const unsigned long long p = q[i];
-      re[i] = f2fma(p, vx, re[i]);
-      im[i] = f2fma(p, vy, im[i]);
+      gre[i] = f2fma(p, vx, gre[i]);
+      gim[i] = f2fma(p, vy, gim[i]);
     }
+  }
+  __device__ __forceinline__ void fold() {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      re[i] = f2add(re[i], gre[i]);
+      im[i] = f2add(im[i], gim[i]);
+    }
+    begin();
   }
   __device__ __forceinline__ void write(Cx<float>* o, int row, int R1, long long K) {
 #pragma unroll
@@ -107,6 +123,8 @@ struct RowSums<double, N> {
       s[i].y = fma(f[i], v.y, s[i].y);
     }
   }
+  __device__ __forceinline__ void begin() {}
+  __device__ __forceinline__ void fold() {}
   __device__ __forceinline__ void write(Cx<double>* o, int row, int R1, long long K) {
 #pragma unroll
     for (int i = 0; i < N; i++)
@@ -121,30 +139,51 @@ constexpr int row_units(int RT, int share) {
 }
 
 // A CTA's walk over units of a.unit whole rows (the last unit of a slice
-// fewer), each in tiles of kS consecutive sites.  The units of all slices are
-// numbered through and a CTA takes every gridDim.x-th.
-template <int kS>
+// fewer), each in tiles of up to kS consecutive sites; in the split form a tile
+// ends with a group, so that no group's sum is carried from one tile to the
+// next (both sums live through the contraction made the kernels 4 to 12 %
+// slower by spills, a place for them in shared memory as much by a smaller L1).
+// The units of all slices are numbered through and a CTA takes every
+// gridDim.x-th.
+template <typename R>
 struct Cursor {
+  static constexpr int kS = Cfg<R>::kS;
   int tl, unit, x0, n;  // slice, unit, first site of the tile in the slice, sites of the tile
   int row, x;           // of the first site
-  __device__ __forceinline__ void place(const ContractArgs& a) {
+  int nrow, nx;         // split form: of the site after the last
+  __device__ __forceinline__ int end(const ContractArgs& a) const { return min(a.V3, (unit + 1) * a.unit * a.Lx); }
+  __device__ __forceinline__ void fit(const ContractArgs& a, const RowGroups& g) {
+    n = min(kS, end(a) - x0);
+    if constexpr (sizeof(R) == 4) {
+      nrow = row;
+      for (nx = x + n; nx >= a.Lx; nx -= a.Lx) nrow++;
+      const int b = g.begin[nx];
+      n -= nx - b;
+      nx = b;
+    }
+  }
+  __device__ __forceinline__ void place(const ContractArgs& a, const RowGroups& g) {
     row = unit * a.unit;
     x = 0;
     x0 = row * a.Lx;
-    n = min(kS, min(a.V3, x0 + a.unit * a.Lx) - x0);
+    fit(a, g);
   }
-  __device__ __forceinline__ void first(const ContractArgs& a) {
+  __device__ __forceinline__ void first(const ContractArgs& a, const RowGroups& g) {
     tl = (int)(blockIdx.x / (unsigned)a.upt);
     unit = (int)(blockIdx.x % (unsigned)a.upt);
-    place(a);
+    place(a, g);
   }
   __device__ __forceinline__ bool valid(const ContractArgs& a) const { return tl < a.ntau; }
-  __device__ __forceinline__ void next(const ContractArgs& a) {
-    const int end = min(a.V3, (unit + 1) * a.unit * a.Lx);
-    x0 += kS;
-    if (x0 < end) {
-      n = min(kS, end - x0);
-      for (x += kS; x >= a.Lx; x -= a.Lx) row++;
+  __device__ __forceinline__ void next(const ContractArgs& a, const RowGroups& g) {
+    x0 += n;
+    if (x0 < end(a)) {
+      if constexpr (sizeof(R) == 4) {
+        row = nrow;
+        x = nx;
+      } else {
+        for (x += kS; x >= a.Lx; x -= a.Lx) row++;
+      }
+      fit(a, g);
     } else {  // gridDim.x units further, without a division
       tl += a.step_slice;
       unit += a.step_unit;
@@ -152,22 +191,24 @@ struct Cursor {
         unit -= a.upt;
         tl++;
       }
-      place(a);
+      place(a, g);
     }
   }
 };
 
 // Adds the tile's values of one output position (val(s), sites 0..n-1) into
 // its sums for the phase rows from `first` on, writing every x row that ends.
-template <typename R, int RT, int N, int kS, typename Val>
-__device__ __forceinline__ void add_x(const ContractArgs& a, const R* ph, RowSums<R, N>& acc, int first,
-                                      const Cursor<kS>& c, int k, Val&& val) {
+template <typename R, int RT, int N, typename Val>
+__device__ __forceinline__ void add_x(const ContractArgs& a, const XPhases<R>& ph, RowSums<R, N>& acc, int first,
+                                      const Cursor<R>& c, int k, Val&& val) {
   constexpr int kStride = phase_stride(RT);
   const int rows = a.V3 / a.Lx;
   int row = c.row, x = c.x, s = 0;
+  acc.begin();
   while (s < c.n) {
-    const int end = min(c.n, s + a.Lx - x);  // the sites of this row
-    const R* f = ph + x * kStride + first;
+    // the sites of this group (split form) or row
+    const int end = sizeof(R) == 4 ? s + ph.g.end[x] - x : min(c.n, s + a.Lx - x);
+    const R* f = ph.t + x * kStride + first;
     x += end - s;
 #pragma unroll 1
     for (; s + 4 <= end; s += 4, f += 4 * kStride) {
@@ -179,6 +220,7 @@ __device__ __forceinline__ void add_x(const ContractArgs& a, const R* ph, RowSum
     }
 #pragma unroll 1
     for (; s < end; s++, f += kStride) acc.add(f, val(s));
+    acc.fold();
     if (x == a.Lx) {
       acc.write((Cx<R>*)a.out + ((long long)c.tl * rows + row) * a.R1 * a.K + k, first, a.R1, a.K);
       x = 0;
@@ -265,7 +307,7 @@ struct Loader {
     }
   }
   // sites past the tile's last one read the first (their sums are not used)
-  __device__ __forceinline__ void load(const ContractArgs& a, const Cursor<kS>& c, int flavour, int role, int site) {
+  __device__ __forceinline__ void load(const ContractArgs& a, const Cursor<R>& c, int flavour, int role, int site) {
     if (!c.valid(a)) return;
     const SliceDesc* sd = a.sl + c.tl;
     f = flavour;
@@ -282,7 +324,7 @@ struct Loader {
     }
   }
   // split form: scaled by 2^-E (in double: exact, no intermediate leaves the range)
-  __device__ __forceinline__ void store(const ContractArgs& a, const Cursor<kS>& c, const Tile<R>& t, int role) {
+  __device__ __forceinline__ void store(const ContractArgs& a, const Cursor<R>& c, const Tile<R>& t, int role) {
     if (!c.valid(a)) return;
     double sc = 1.0;
     if (sizeof(R) == 4) {
@@ -308,7 +350,7 @@ struct Loader {
 
 // The tile's 288 rows of kS sites into L2; a role takes its block of both flavours.
 template <typename R, typename Tin>
-__device__ __forceinline__ void prefetch(const ContractArgs& a, const Cursor<Cfg<R>::kS>& c, int role, int site) {
+__device__ __forceinline__ void prefetch(const ContractArgs& a, const Cursor<R>& c, int role, int site) {
   if (!c.valid(a)) return;
   constexpr int kS = Cfg<R>::kS, kLine = 128 / (int)sizeof(Cx<Tin>), kLines = kS / kLine;  // sites per line, lines per row
   const SliceDesc* sd = a.sl + c.tl;
@@ -379,13 +421,14 @@ __device__ __forceinline__ void diquark_add(const Cx<R> (&x)[9], const Cx<R> (&y
 
 // xt: [Lx][R1] phase rows; one CTA per SM (its shared memory and registers fill it)
 template <typename R, typename K>
-cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, int RT, int smem, int nsm,
-                         cudaStream_t s) {
+cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, const RowPlan& rp, int RT, int smem,
+                         int nsm, cudaStream_t s) {
   constexpr int kS = Cfg<R>::kS;
   ContractArgs a = a0;
   const int stride = phase_stride(RT);
   if (a.Lx * stride > kRowsMaxPhases || a.R1 > RT) return cudaErrorInvalidValue;
   XPhases<R> ph;
+  ph.g = rp.g;
   for (int i = 0; i < a.Lx; i++)
     for (int r = 0; r < stride; r++) ph.t[i * stride + r] = r < a.R1 ? (R)xt[i * a.R1 + r] : R(0);
   // rows per unit: the fewest tiles per CTA, the smaller unit on a tie (a unit
@@ -394,7 +437,7 @@ cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, int
   long long best = -1;
   for (int m = 1; m <= kS && m <= rows; m++) {
     const long long units = (long long)((rows + m - 1) / m) * a.ntau;
-    const long long cost = (units + nsm - 1) / nsm * ((m * a.Lx + kS - 1) / kS);
+    const long long cost = (units + nsm - 1) / nsm * (kS == 32 ? rp.tiles[m] : (m * a.Lx + kS - 1) / kS);
     if (best < 0 || cost < best) {
       best = cost;
       a.unit = m;

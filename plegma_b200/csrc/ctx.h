@@ -57,6 +57,7 @@ struct AxesPlan {
   int R1 = 0, RY = 0, NP = 0, NO = 0, nmom = 0;
   DevBuf tab;  // phases, then the orbit lists
   std::vector<double> xth;  // xt on the host, for the fused contraction
+  p2::RowPlan rows;         // the same
   const double *xt = nullptr, *yt = nullptr, *zt = nullptr;
   std::vector<int> first, ylist;
   const int *orb = nullptr, *omom = nullptr;

@@ -32,9 +32,11 @@
 // Without the fused contraction (contract_site.cuh) 48^3 slices gain only 2 %:
 // the position buffer's write and read bound both.
 //
-// Sums over x: FP64 for FP64 input, FP32 for FP32 input (sequential over one
-// row of Lx sites by one thread, so a row's sum does not depend on the launch
-// shape); over y likewise; over z in FP64.  All in a fixed order.
+// Sums over x: FP64 for FP64 input; FP32 input in FP32 over groups of at most
+// kSumGroup sites and in FP64 over these, one row of Lx sites by one thread, so
+// a row's sum does not depend on the launch shape; over y in FP32 by groups of
+// groups (a conversion to FP64 per group doubled its time: 402 us instead of 197
+// at 48^3 x 24 slices with K = 288); over z in FP64.  All in a fixed order.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -111,11 +113,29 @@ __global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
     }
     cp_async_commit();
   };
+  // FP32: acc the current group of kSumGroup sites, tot the groups before it
+  constexpr bool kGroups = sizeof(R) == 4;
+  static_assert(!kGroups || C::n % kSumGroup == 0, "a chunk holds whole groups");
   Cx<R> acc[2][R1];
+  Cx<double> tot[2][kGroups ? R1 : 1];
 #pragma unroll
-  for (int j = 0; j < 2; j++)
+  for (int j = 0; j < 2; j++) {
 #pragma unroll
     for (int r = 0; r < R1; r++) acc[j][r] = czero<R>();
+#pragma unroll
+    for (int r = 0; r < (kGroups ? R1 : 1); r++) tot[j][r] = czero<double>();
+  }
+  auto add = [&](const Cx<R>* d, const R* p, int x) {
+    const Cx<R> v0 = d[x], v1 = d[32 * C::stride + x];
+#pragma unroll
+    for (int r = 0; r < R1; r++) {
+      const R f = p[x * R1 + r];
+      acc[0][r].x = fma(f, v0.x, acc[0][r].x);
+      acc[0][r].y = fma(f, v0.y, acc[0][r].y);
+      acc[1][r].x = fma(f, v1.x, acc[1][r].x);
+      acc[1][r].y = fma(f, v1.y, acc[1][r].y);
+    }
+  };
   issue(0);
   for (int ch = 0; ch < nchunk; ch++) {
     issue(ch + 1);
@@ -124,17 +144,24 @@ __global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
     const Cx<R>* d = st + (ch & 1) * C::stage + lane * C::stride;
     const R* p = ph + ch * C::n * R1;
     const int n = min(C::n, a.Lx - ch * C::n);
+    if constexpr (kGroups) {
+#pragma unroll 1
+      for (int x0 = 0; x0 < n; x0 += kSumGroup) {
+        const int x1 = min(n, x0 + kSumGroup);
 #pragma unroll 4
-    for (int x = 0; x < n; x++) {
-      const Cx<R> v0 = d[x], v1 = d[32 * C::stride + x];
+        for (int x = x0; x < x1; x++) add(d, p, x);
 #pragma unroll
-      for (int r = 0; r < R1; r++) {
-        const R f = p[x * R1 + r];
-        acc[0][r].x = fma(f, v0.x, acc[0][r].x);
-        acc[0][r].y = fma(f, v0.y, acc[0][r].y);
-        acc[1][r].x = fma(f, v1.x, acc[1][r].x);
-        acc[1][r].y = fma(f, v1.y, acc[1][r].y);
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int r = 0; r < R1; r++) {
+            tot[j][r].x += (double)acc[j][r].x;
+            tot[j][r].y += (double)acc[j][r].y;
+            acc[j][r] = czero<R>();
+          }
       }
+    } else {
+#pragma unroll 4
+      for (int x = 0; x < n; x++) add(d, p, x);
     }
     __syncwarp();  // the chunk is read: the stage may be refilled
   }
@@ -145,7 +172,8 @@ __global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
     if (k < a.K && row < a.rows) {
       Cx<R>* o = (Cx<R>*)a.s1 + (((long long)tau * a.rows + row) * R1) * a.Kst + k;
 #pragma unroll
-      for (int r = 0; r < R1; r++) o[(long long)r * a.Kst] = acc[j][r];
+      for (int r = 0; r < R1; r++)
+        o[(long long)r * a.Kst] = kGroups ? cx<R>((R)tot[j][kGroups ? r : 0].x, (R)tot[j][kGroups ? r : 0].y) : acc[j][r];
     }
   }
 }
@@ -154,10 +182,12 @@ __global__ void __launch_bounds__(32 * kXWarps, 3) k_axis_x(const AxisXArgs a) {
 // Warp r of a block takes x row r of (slice, z) for 32 or 64 components (KPL
 // per lane): every value of S1 is read once and used for all the pairs of r,
 // U rows y at a time (their loads are in flight together, and vector loads
-// bring the phases of several y), zper values of z one after the other.  The body is instantiated for the number of
-// pairs, so the rows with few of them spend nothing on the others.
-template <typename R, int N, int KPL, int U>
-__device__ __forceinline__ void axis_y_body(const AxisYArgs& a, const R* yt, int LyP, int r, int first) {
+// bring the phases of several y), zper values of z one after the other.  The
+// body is instantiated for the number of pairs, so the rows with few of them
+// spend nothing on the others.
+template <int N, int KPL, int U>
+__device__ __forceinline__ void axis_y_body(const AxisYArgs& a, const double* yt, int LyP, int r, int first) {
+  typedef double R;
   const int lane = threadIdx.x & 31, tau = blockIdx.z, k0 = blockIdx.x * 32 * KPL + lane;
   const R* row[N];
 #pragma unroll
@@ -204,10 +234,73 @@ __device__ __forceinline__ void axis_y_body(const AxisYArgs& a, const R* yt, int
   }
 }
 
+// FP32: a step's sums are added up over kSumGroups steps, and these in the result.
+template <int N, int KPL, int U>
+__device__ __forceinline__ void axis_y_body(const AxisYArgs& a, const float* yt, int LyP, int r, int first) {
+  static_assert(U <= kSumGroup, "a running sum's steps");
+  const int lane = threadIdx.x & 31, tau = blockIdx.z, k0 = blockIdx.x * 32 * KPL + lane;
+  const float* row[N];
+#pragma unroll
+  for (int j = 0; j < N; j++) row[j] = yt + a.ylist[first + j] * LyP;
+  const long long rs = (long long)a.R1 * a.K;  // one row of S1
+#pragma unroll 1
+  for (int z = blockIdx.y * a.zper; z < min(a.Lz, (int)(blockIdx.y + 1) * a.zper); z++) {
+    const Cx<float>* s = (const Cx<float>*)a.s1 + ((long long)tau * a.Lz + z) * a.Ly * rs + (long long)r * a.K;
+#pragma unroll 1
+    for (int ys = 0; ys < a.Ly; ys += kSumGroups * U) {
+      Cx<float> acc[N][KPL];
+#pragma unroll
+      for (int j = 0; j < N; j++)
+#pragma unroll
+        for (int q = 0; q < KPL; q++) acc[j][q] = czero<float>();
+      const int ye = min(a.Ly, ys + kSumGroups * U);
+#pragma unroll 1
+      for (int y0 = ys; y0 < ye; y0 += U) {
+        Cx<float> v[U][KPL];
+#pragma unroll
+        for (int i = 0; i < U; i++)
+#pragma unroll
+          for (int q = 0; q < KPL; q++)
+            v[i][q] = y0 + i < a.Ly && k0 + 32 * q < a.K ? s[(y0 + i) * rs + k0 + 32 * q] : czero<float>();
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+          asm volatile("" ::: "memory");  // keeps the phases of later pairs from being moved up (registers)
+          float f[U];                     // zero beyond Ly
+#pragma unroll
+          for (int i = 0; i < U; i += 4)
+            *reinterpret_cast<float4*>(f + i) = *reinterpret_cast<const float4*>(row[j] + y0 + i);
+#pragma unroll
+          for (int q = 0; q < KPL; q++) {
+            Cx<float> g = czero<float>();
+#pragma unroll
+            for (int i = 0; i < U; i++) {
+              g.x = fma(f[i], v[i][q].x, g.x);
+              g.y = fma(f[i], v[i][q].y, g.y);
+            }
+            acc[j][q] = acc[j][q] + g;
+          }
+        }
+      }
+      Cx<float>* o = (Cx<float>*)a.s2 + (((long long)tau * a.Lz + z) * a.NP + first) * a.K;
+#pragma unroll
+      for (int j = 0; j < N; j++)
+#pragma unroll
+        for (int q = 0; q < KPL; q++)
+          if (k0 + 32 * q < a.K) {
+            Cx<float>& d = o[(long long)j * a.K + k0 + 32 * q];
+            d = ys ? d + acc[j][q] : acc[j][q];
+          }
+    }
+  }
+}
+
 constexpr int kYUnroll = 8;
 
-template <typename R, int KPL>
-__global__ void __launch_bounds__(32 * kAxisMaxRows) k_axis_y(const __grid_constant__ AxisYArgs a) {
+// W: most rows.  FP32: two blocks per SM; up to seven rows then have 128
+// registers, which hold the sums (bounded for nine rows they spill: 207 us
+// instead of 197 at 48^3 x 24 slices, K = 288).
+template <typename R, int KPL, int W>
+__global__ void __launch_bounds__(32 * W, sizeof(R) == 4 ? 2 : 0) k_axis_y(const __grid_constant__ AxisYArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int U = sizeof(R) * KPL == 16 ? kYUnroll / 2 : kYUnroll;
   R* yt = (R*)smem_raw;  // [RY][Ly rounded up]
@@ -220,15 +313,15 @@ __global__ void __launch_bounds__(32 * kAxisMaxRows) k_axis_y(const __grid_const
   const int r = threadIdx.x >> 5;
   const int first = a.first[r], cnt = a.first[r + 1] - first;
   switch (cnt) {  // 0: a padding row
-    case 1: axis_y_body<R, 1, KPL, U>(a, yt, LyP, r, first); break;
-    case 2: axis_y_body<R, 2, KPL, U>(a, yt, LyP, r, first); break;
-    case 3: axis_y_body<R, 3, KPL, U>(a, yt, LyP, r, first); break;
-    case 4: axis_y_body<R, 4, KPL, U>(a, yt, LyP, r, first); break;
-    case 5: axis_y_body<R, 5, KPL, U>(a, yt, LyP, r, first); break;
-    case 6: axis_y_body<R, 6, KPL, U>(a, yt, LyP, r, first); break;
-    case 7: axis_y_body<R, 7, KPL, U>(a, yt, LyP, r, first); break;
-    case 8: axis_y_body<R, 8, KPL, U>(a, yt, LyP, r, first); break;
-    case 9: axis_y_body<R, 9, KPL, U>(a, yt, LyP, r, first); break;
+    case 1: axis_y_body<1, KPL, U>(a, yt, LyP, r, first); break;
+    case 2: axis_y_body<2, KPL, U>(a, yt, LyP, r, first); break;
+    case 3: axis_y_body<3, KPL, U>(a, yt, LyP, r, first); break;
+    case 4: axis_y_body<4, KPL, U>(a, yt, LyP, r, first); break;
+    case 5: axis_y_body<5, KPL, U>(a, yt, LyP, r, first); break;
+    case 6: axis_y_body<6, KPL, U>(a, yt, LyP, r, first); break;
+    case 7: axis_y_body<7, KPL, U>(a, yt, LyP, r, first); break;
+    case 8: axis_y_body<8, KPL, U>(a, yt, LyP, r, first); break;
+    case 9: axis_y_body<9, KPL, U>(a, yt, LyP, r, first); break;
   }
 }
 
@@ -326,7 +419,7 @@ cudaError_t launch_x_t(const AxisXArgs& a, cudaStream_t s) {
   return cudaErrorInvalidValue;
 }
 
-template <typename R, int KPL>
+template <typename R, int KPL, int W>
 cudaError_t launch_y(const AxisYArgs& a0, cudaStream_t s) {
   AxisYArgs a = a0;
   // as many z per block as leave about eight blocks per SM: a block fills the phase table first
@@ -334,11 +427,11 @@ cudaError_t launch_y(const AxisYArgs& a0, cudaStream_t s) {
   a.zper = (int)std::max<long long>(1, std::min<long long>(a.Lz, per_z * a.Lz / (8 * 148)));
   const int smem = a.RY * ((a.Ly + kYUnroll - 1) / kYUnroll * kYUnroll) * (int)sizeof(R);
   if (smem > 48 << 10) {
-    cudaError_t e = ensure_smem((const void*)k_axis_y<R, KPL>, smem);
+    cudaError_t e = ensure_smem((const void*)k_axis_y<R, KPL, W>, smem);
     if (e != cudaSuccess) return e;
   }
   const dim3 grid((a.K + 32 * KPL - 1) / (32 * KPL), (a.Lz + a.zper - 1) / a.zper, a.ntau);
-  k_axis_y<R, KPL><<<grid, 32 * a.R1, smem, s>>>(a);
+  k_axis_y<R, KPL, W><<<grid, 32 * a.R1, smem, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -373,6 +466,45 @@ struct AxisRows {
 
 }  // namespace
 
+// A row of Lx sites in equal groups.  Their number is that with the best filled
+// tiles of 32 sites: small groups leave less of a tile empty (a row of 21: two
+// groups, 30.5 sites of a tile on average; one in ten of all Lx loses more than
+// 10 %), each costs an addition per sum and a turn of the loop (0.8 % of a tile
+// per group, measured with two and four of them in a tile at Lx = 48).  It
+// depends on Lx alone, so that a row's sum does not depend on the launch.
+RowPlan row_plan(int Lx) {
+  RowPlan best{};
+  double least = 0;
+  const int n0 = (Lx + kSumGroup - 1) / kSumGroup;
+  for (int n = n0; n <= std::max(n0, std::min(24, Lx / 4)); n++) {
+    RowPlan p{};
+    auto start = [&](int i) { return i * Lx / n; };
+    for (int i = 0; i < n; i++)
+      for (int x = start(i); x < start(i + 1); x++) {
+        p.g.begin[x] = (unsigned char)start(i);
+        p.g.end[x] = (unsigned char)start(i + 1);
+      }
+    int left = 0;
+    for (int m = 1; m <= 32; m++) {
+      p.tiles[m] = p.tiles[m - 1];
+      for (int i = 0; i < n; i++) {
+        const int len = start(i + 1) - start(i);
+        if (left < len) {
+          p.tiles[m]++;
+          left = 32;
+        }
+        left -= len;
+      }
+    }
+    const double cost = p.tiles[32] + 0.008 * 32 * n;
+    if (n == n0 || cost < least) {
+      least = cost;
+      best = p;
+    }
+  }
+  return best;
+}
+
 cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
   if (a0.ntau < 1 || a0.K < 1) return cudaSuccess;
   AxisXArgs a = a0;
@@ -382,8 +514,10 @@ cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
 }
 
 cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s) {
-  if (fp32) return kpl == 2 ? launch_y<float, 2>(a, s) : launch_y<float, 1>(a, s);
-  return kpl == 2 ? launch_y<double, 2>(a, s) : launch_y<double, 1>(a, s);
+  constexpr int W = kAxisMaxRows;
+  if (!fp32) return kpl == 2 ? launch_y<double, 2, W>(a, s) : launch_y<double, 1, W>(a, s);
+  if (a.R1 <= 7) return kpl == 2 ? launch_y<float, 2, 7>(a, s) : launch_y<float, 1, 7>(a, s);
+  return kpl == 2 ? launch_y<float, 2, W>(a, s) : launch_y<float, 1, W>(a, s);
 }
 
 cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s) {
@@ -511,6 +645,7 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
   ap.NO = (int)members.size();
   ap.nmom = nmom;
   ap.xth.assign(tab.begin(), tab.begin() + oy);
+  if (c->Ll[0] <= p2::kRowsMaxLx) ap.rows = p2::row_plan(c->Ll[0]);
   ap.xt = (const double*)ap.tab.p;
   ap.yt = ap.xt + oy;
   ap.zt = ap.xt + oz;

@@ -7,6 +7,7 @@ units of several rows, FP32 propagators.  Tolerance, relative to sum_x
 sites for the per-site rounding to average, plain 1e-13 (test_gpu_axes.py)."""
 import numpy as np
 import pytest
+import torch
 
 from plegma_b200 import lib as p2
 
@@ -66,4 +67,57 @@ def test_rows_do_not_depend_on_the_batch(mode):
     a, b = p2.result_blocks(what, 5, len(moms), ref), p2.result_blocks(what, 1, len(moms), one)
     for bit in a:
         assert np.array_equal(a[bit][:, :, :1], b[bit])
+    ctx.close()
+
+
+def _constant_props(ctx, baryons, seed):
+    """u and d without a dependence on the site (a free field from a wall
+    source at p = 0) whose contractions are exact in FP32: one spin block each,
+    integers of 7 bits on the colour diagonal (three-quark sums of at most 24
+    bits) or of 12 bits in one colour entry (products of 24 bits)."""
+    T = ctx.Ll[3]
+    g = torch.Generator().manual_seed(seed)
+    bufs = []
+    for block in (0, 5):
+        p = torch.zeros((144, T, ctx.V3), dtype=torch.complex128, device="cuda")
+        for c in ((0, 4, 8) if baryons else (0,)):
+            v = torch.randint(65, 128, (T,), generator=g) if baryons else torch.randint(2049, 4096, (T,), generator=g)
+            p[9 * block + c] = v.cuda()[:, None]
+        bufs.append(p)
+    return bufs
+
+
+@pytest.mark.parametrize("what,baryons", [
+    (G16, False), (p2.MESON_ALL34 | p2.MESON_NEW10, False),         # sums over x in the contraction; from the position buffer
+    (NUC | D, True), (NUC | p2.MESON_ALL34, True),
+    ("udsc", True),
+])
+@pytest.mark.parametrize("L", [(64, 64, 1, 16), (128, 128, 1, 4), (236, 230, 1, 2)])
+def test_sums_of_equal_values(what, baryons, L):
+    """Adding one value again and again rounds the same way at every step, so
+    the FP32 sums of the split form lose the most here (one running sum over x,
+    then one over y: 1.7e-6 at 64 x 64, 7e-6 at 240 x 240).  Bound of the form:
+    1e-6 of sum_x |c_k(x)|, which is |C(p = 0)| for equal values."""
+    ctx = p2.Context(L)
+    bufs = _constant_props(ctx, baryons, 64)
+    T, moms = L[3], p2.mom_list(1)
+    got = []
+    for mode in (p2.P2_PLAIN_FP64, SPLIT):
+        if what == "udsc":
+            n = len(p2.udsc_datasets(ctx.udsc_request((0, 0, 0, 0), T, None, moms=moms, prop_u=0, prop_d=1)))
+            out = torch.zeros(n * T * len(moms), dtype=torch.complex128, device="cuda")
+            req = ctx.udsc_request((0, 0, 0, 0), T, out.data_ptr(), moms=moms, mode=mode, prop_u=0, prop_d=1)
+            ctx.contract_udsc([ctx.prop(b.data_ptr()) for b in bufs], req)
+            ctx.sync()
+            got.append([out.cpu().numpy().reshape(n, T, len(moms))])
+        else:
+            out, _ = run(ctx, bufs, (0, 0, 0, 0), T, what, moms=moms, mode=mode)
+            got.append([b for b in p2.result_blocks(what, T, len(moms), out).values()])
+    for ref, res in zip(*got):
+        ax = 2 if what == "udsc" else 3
+        scale = np.abs(np.take(ref, [0], axis=ax))  # momentum 0 is p = 0
+        held = scale > 1e-3 * scale.max()
+        assert held.any()
+        err = np.abs(res - ref) / np.where(held, scale, np.inf)
+        assert err.max() < 1e-6, err.max()
     ctx.close()
