@@ -164,10 +164,13 @@ const char* p2_last_error(const p2_ctx* ctx);
 p2_status p2_sync(p2_ctx* ctx);
 /* Work is issued on `stream` (a cudaStream_t; NULL = the context's own). */
 p2_status p2_set_stream(p2_ctx* ctx, void* stream);
-/* Upper bound on the context's per-chunk position-space buffer (time slices
- * are contracted and projected in chunks that fit it; default min(8 GiB,
- * free/4)).  Smaller values cut memory and make more, shorter launches; the
- * result does not depend on it beyond rounding.  No counterpart in the
+/* Upper bound on the context's per-chunk scratch: the position-space buffer
+ * and the projection's partial sums over x and over y (time slices are
+ * contracted and projected in chunks that fit it, one slice at least; default
+ * min(8 GiB, free/4)).  The tables, the staging of host propagators and, for
+ * momentum lists that are projected directly, the partial sums of that
+ * projection come on top.  Smaller values cut memory and make more, shorter
+ * launches; the result does not depend on it beyond rounding.  No counterpart in the
  * reference (it allocates per call, lib/kernels/PLEGMA_baryons.cuh:122). */
 p2_status p2_set_workspace(p2_ctx* ctx, size_t bytes);
 

@@ -142,6 +142,28 @@ bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int 
   return false;
 }
 
+int chunk_slices(const p2_ctx* c, size_t per, long long slices) {
+  const size_t most = (size_t)std::max(1LL, std::min(slices, 65535LL));
+  return (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), most));
+}
+
+size_t sums_offset(const p2_ctx* c, int fp32, size_t n, size_t Kr) {
+  return (n * Kr * c->V3 * (fp32 ? 8 : 16) + 255) / 256 * 256;
+}
+
+size_t scratch_bytes(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t n, size_t K, size_t Kr) {
+  return sums_offset(c, fp32, n, Kr) + (ap ? axes_ws_bytes(c, *ap, fp32, n, K) : 0);
+}
+
+size_t scratch_start(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t n, size_t K, size_t Kr) {
+  const size_t all = n * K * (size_t)c->V3 * (fp32 ? 8 : 16);
+  return std::max(std::min({all, c->ws_budget, (size_t)64 << 20}), scratch_bytes(c, ap, fp32, n, K, Kr));
+}
+
+size_t slice_bytes(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t K, size_t Kr, bool host) {
+  return std::max(scratch_bytes(c, ap, fp32, 1, K, Kr), host ? K * (size_t)c->V3 * (fp32 ? 8 : 16) : 0);
+}
+
 Stager::Stager(p2_ctx* ctx, const p2_prop* pp, const p2_request* rr, const Work& work)
     : c(ctx), props(pp), reqs(rr), w(work) {
   for (const SliceRef& s : w.sl) {
@@ -496,12 +518,6 @@ p2_status project_direct(p2_ctx* c, const Plan& pl, int K, int n, int max_n, con
 
 namespace {
 
-int chunk_slices(p2_ctx* c, int K) {
-  const size_t per = (size_t)K * c->V3 * 16;
-  size_t n = c->ws_budget / std::max<size_t>(per, 1);
-  return (int)std::max<size_t>(1, std::min<size_t>(n, (size_t)c->T));
-}
-
 // Plain FP64 form for requests reqs[idx[..]] that share contractions and
 // momenta: FP64 site contraction, FP64 projection, deterministic reduction.
 p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, const int* idx, int nidx,
@@ -524,16 +540,12 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
   }
 
   const unsigned fused = fused_bits(c, ap, what), rest = what & ~fused;
-  const size_t s1_slice = ap ? axes_s1_bytes(c, *ap, 0, 1, pl.K) : 0;
-  // without a position buffer (host propagators keep its chunks: their staging
-  // buffers hold a chunk each, and the copies overlap the chunk before)
-  const bool whole = !rest && !any_host(props, reqs, idx, nidx);
-  const int tc = whole ? (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(s1_slice, 1), (size_t)c->T))
-                       : chunk_slices(c, pl.K);
-  const Work w = make_work(c, props, reqs, idx, nidx, tc);
+  const int Kr = components_of(rest);  // components of the position buffer
+  const size_t per = slice_bytes(c, ap, 0, pl.K, Kr, any_host(props, reqs, idx, nidx));
+  const Work w = make_work(c, props, reqs, idx, nidx, chunk_slices(c, per, c->T));
   if (w.sl.empty()) return P2_OK;
-  if (rest) P2_TRY(c, c->cbuf.ensure((size_t)w.max_n * pl.K * c->V3 * 16), "position buffer alloc");
-  if (ap) P2_TRY(c, c->axes_ws.ensure(axes_ws_start(c, *ap, 0, w.max_n, pl.K)), "projection workspace");
+  P2_TRY(c, c->cbuf.ensure(scratch_start(c, ap, 0, w.max_n, pl.K, Kr)), "workspace alloc");
+  void* const s1 = (char*)c->cbuf.p + sums_offset(c, 0, w.max_n, Kr);
   Stager sg(c, props, reqs, w);
   if ((st = sg.prepare(outs)) != P2_OK) return st;
 
@@ -553,7 +565,7 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     a.g16_raw = p2::g16_raw(what) ? 1 : 0;  // the projection is followed by k_meson_gamma
     if (fused) {
       p2::ContractArgs r = a;
-      r.out = c->axes_ws.p;
+      r.out = s1;
       r.Lx = c->Ll[0];
       r.R1 = ap->R1;
       ProfScope ps(c, "contract_site");
@@ -563,6 +575,8 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
         P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), ap->rows, 1, 0, c->nsm, c->stream), "contract kernel");
     }
     if ((a.what = rest)) {
+      a.K = Kr;
+      a.k = offsets_of(rest);
       ProfScope ps(c, "contract_plain_fp64");
       P2_TRY(c, p2::launch_contract_plain(a, c->nsm, c->stream), "contract kernel");
     }
@@ -570,11 +584,11 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     if ((st = sg.issue((int)ci + 2)) != P2_OK) return st;
 
     if (ap) {
-      if (rest && (st = axes_x_blocks(c, *ap, pl, what, rest, c->cbuf.p, 0, n, c->axes_ws.p)) != P2_OK) return st;
+      if (rest && (st = axes_x_blocks(c, *ap, what, rest, c->cbuf.p, 0, n, s1)) != P2_OK) return st;
       AxesOut ao;
       ao.dsl = sg.desc((int)ci);
       ao.blocks = &pl.blocks;
-      if ((st = axes_yz(c, *ap, c->axes_ws.p, 0, n, pl.K, ao)) != P2_OK) return st;
+      if ((st = axes_yz(c, *ap, s1, 0, n, pl.K, ao)) != P2_OK) return st;
     } else if ((st = project_direct(c, pl, pl.K, n, w.max_n, sg.desc((int)ci), pl.blocks)) != P2_OK) {
       return st;
     }
@@ -607,18 +621,17 @@ p2_status ft_axes(p2_ctx* c, const AxesPlan& ap, const double* field, int dof, i
     P2_TRY(c, c->res.ensure(total * 16), "result alloc");
     dst = (double*)c->res.p;
   }
-  const size_t per = axes_ws_bytes(c, ap, 0, 1, dof);
-  const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)nt));
-  P2_TRY(c, c->axes_ws.ensure(axes_ws_bytes(c, ap, 0, tc, dof)), "projection workspace");
+  const int tc = chunk_slices(c, axes_ws_bytes(c, ap, 0, 1, dof), nt);
+  P2_TRY(c, c->cbuf.ensure(axes_ws_bytes(c, ap, 0, tc, dof)), "workspace alloc");
   for (int t0 = 0; t0 < nt; t0 += tc) {
     const int n = std::min(tc, nt - t0);
-    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, dof, c->axes_ws.p);
+    p2_status st = axes_x(c, ap, field + 2 * (size_t)t0 * c->V3, 0, c->V3, c->V3 * nt, n, dof, dof, c->cbuf.p);
     if (st != P2_OK) return st;
     AxesOut ao;
     ao.oT = (long long)dof * ap.nmom;
     ao.oK = ap.nmom;
     ao.out = dst + 2 * (size_t)t0 * ao.oT;
-    if ((st = axes_yz(c, ap, c->axes_ws.p, 0, n, dof, ao)) != P2_OK) return st;
+    if ((st = axes_yz(c, ap, c->cbuf.p, 0, n, dof, ao)) != P2_OK) return st;
   }
   if (out_location == P2_HOST) {
     P2_TRY(c, cudaMemcpyAsync(out, dst, total * 16, cudaMemcpyDeviceToHost, c->stream), "result download");
@@ -762,7 +775,7 @@ p2_status p2_ctx_destroy(p2_ctx* c) {
   }
   cudaStreamSynchronize(c->stream);
   for (DevBuf* b : {&c->cbuf, &c->part, &c->tab, &c->res, &c->moms, &c->sdesc, &c->ptab, &c->ft_kexp, &c->axes[0].tab,
-                    &c->axes[1].tab, &c->axes_ws})
+                    &c->axes[1].tab})
     b->release();
   if (c->sdesc_host) cudaFreeHost(c->sdesc_host);
   if (c->sdesc_copied) cudaEventDestroy(c->sdesc_copied);
@@ -974,7 +987,7 @@ p2_status p2_contract_position(p2_ctx* c, const p2_prop* props, int nprops, cons
   if (c->host_only) return c->fail(P2_ERR_UNSUPPORTED, "host-only context");
   const int K = components_of(r->contractions);
   const size_t slice = (size_t)K * c->V3;  // complex elements of one time slice
-  const Work w = make_work(c, props, r, nullptr, 1, chunk_slices(c, K));
+  const Work w = make_work(c, props, r, nullptr, 1, chunk_slices(c, slice * 16, c->T));
   if (w.sl.empty()) return P2_OK;
   P2_TRY(c, c->cbuf.ensure((size_t)w.max_n * slice * 16), "position buffer alloc");
   Stager sg(c, props, r, w);
@@ -1060,7 +1073,7 @@ p2_status p2_ft_apply_split(p2_ctx* c, const double* field, int dof, int nt, con
     c->ft_kexp_n = dof;
   }
   const size_t per = (size_t)dof * c->V3 * 8;
-  const int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per, 1), (size_t)nt));
+  const int tc = chunk_slices(c, per, nt);
   for (int t0 = 0; t0 < nt; t0 += tc) {
     const int n = std::min(tc, nt - t0);
     P2_TRY(c, c->cbuf.ensure((size_t)n * per), "position buffer alloc");

@@ -122,9 +122,8 @@ struct p2_ctx {
   p2host::DevBuf ptab;
   std::vector<int> plain_moms_key;
   p2_udsc_cache* udsc = nullptr;
-  // axis-by-axis projection: tables per transform sign (-1, +1), sums over x and over y
+  // axis-by-axis projection: tables per transform sign (-1, +1)
   p2host::AxesPlan axes[2];
-  p2host::DevBuf axes_ws;  // S1, then S2 (axes_ws_bytes)
   // launch-shape autotuner (shared with the context's graphs)
   std::shared_ptr<p2host::Tuner> tuner = std::make_shared<p2host::Tuner>();
 
@@ -262,18 +261,30 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
 bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int nidx);
 // Bits of a contraction set that the kernels fused with the sums over x take.
 unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what);
-// The sums over x of the blocks of `bits` from a position buffer of the whole
-// set `what` (n slices, K components of V3 sites each).
-p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
-                        int fp32, int n, void* s1);
-// Bytes of the sums over x of n slices of K components, and of the workspace
-// that holds them and the sums over y (one allocation: each costs about 0.4 ms
-// of a context's first call).
+// The sums over x of the blocks `rest` of a set `what`, from a position buffer
+// that holds the components of `rest` alone (n slices, V3 sites each).
+p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, unsigned what, unsigned rest, const void* cbuf, int fp32, int n,
+                        void* s1);
+// Bytes of the sums over x (S1) of n slices of K components, and with those
+// over y (S2) after them.
 size_t axes_s1_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
 size_t axes_ws_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
-// The workspace of a contraction: at least 64 MB where a position buffer would
-// have taken that, so that calls of different sizes share one allocation.
-size_t axes_ws_start(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K);
+// Scratch of a chunk of n slices (p2_ctx::cbuf, one allocation): the position
+// buffer of Kr of the K components, then, from sums_offset on, S1 and S2.
+size_t sums_offset(const p2_ctx* c, int fp32, size_t n, size_t Kr);
+size_t scratch_bytes(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t n, size_t K, size_t Kr);
+// What a contraction allocates: at least 64 MB where a position buffer of all K
+// would have taken that and the budget allows it, so that calls of different
+// sizes share one allocation (64 MB takes as long to allocate as 2 MB, 0.33 ms
+// on a B200 box; a second, larger one costs 0.6 ms with the release of the first).
+size_t scratch_start(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t n, size_t K, size_t Kr);
+// Bytes that a slice takes of the workspace budget.  Host propagators: at least
+// a position buffer of all K, since their staging buffers hold a chunk each and
+// a chunk's copies overlap the chunk before.
+size_t slice_bytes(const p2_ctx* c, const AxesPlan* ap, int fp32, size_t K, size_t Kr, bool host);
+// Slices per chunk: within the budget, and within the 65535 blocks that a grid
+// has in y and z.
+int chunk_slices(const p2_ctx* c, size_t per, long long slices);
 p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, long long sT, long long sK, int n, int K,
                  int Kst, void* s1);
 p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n, int K, const AxesOut& o);

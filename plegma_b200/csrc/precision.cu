@@ -342,29 +342,23 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
 
   const unsigned fused = fused_bits(c, ap, what);
   const unsigned rest = what & ~fused;
+  const int Kr = components_of(rest);  // components of the position buffer
 
-  // chunk of slices: FP32 position buffer within the workspace budget; a
-  // chunk may hold slices of many requests (a batch of sources), so up to
-  // all of the batch's slices go into one chunk
-  const size_t s1_slice = ap ? axes_s1_bytes(c, *ap, 1, 1, K) : 0;
-  const size_t cb_slice = rest ? (size_t)K * c->V3 * 8 : 0;
-  // without a position buffer (host propagators keep its chunks: their staging
-  // buffers hold a chunk each, and the copies overlap the chunk before)
-  const size_t per_slice = !any_host(props, reqs, idx, nidx) ? std::max(cb_slice, s1_slice) : (size_t)K * c->V3 * 8;
-  size_t nslices = 0;
-  for (int q = 0; q < nidx; q++) nslices += (size_t)std::max(reqs[idx[q]].totalT, 0);
-  int tc = (int)std::max<size_t>(1, std::min<size_t>(c->ws_budget / std::max<size_t>(per_slice, 1),
-                                                   std::max<size_t>(nslices, 1)));
+  // chunk of slices within the workspace budget; a chunk may hold slices of
+  // many requests (a batch of sources), so up to all of the batch's slices go
+  // into one chunk
+  const size_t per_slice = slice_bytes(c, ap, 1, K, Kr, any_host(props, reqs, idx, nidx));
+  long long nslices = 0;
+  for (int q = 0; q < nidx; q++) nslices += std::max(reqs[idx[q]].totalT, 0);
+  int tc = chunk_slices(c, per_slice, nslices);
   if (all_host64) tc = std::min(tc, 4);  // short chunks: the host conversion pipeline fills and drains faster
   const Work w = make_work(c, props, reqs, idx, nidx, tc);
   if (w.sl.empty()) return P2_OK;
   const int mx = w.max_n;
-  if (rest) P2_TRY(c, c->cbuf.ensure((size_t)mx * cb_slice), "position buffer alloc");
+  P2_TRY(c, c->cbuf.ensure(scratch_start(c, ap, 1, mx, K, Kr)), "workspace alloc");
+  void* const s1 = (char*)c->cbuf.p + sums_offset(c, 1, mx, Kr);
   P2_TRY(c, c->expb.ensure((size_t)2 * mx * sizeof(int)), "exponent alloc");
-  if (ap)
-    P2_TRY(c, c->axes_ws.ensure(axes_ws_start(c, *ap, 1, mx, K)), "projection workspace");
-  else
-    P2_TRY(c, c->cmaxb.ensure((size_t)mx * K * sizeof(int)), "maxima alloc");
+  if (!ap) P2_TRY(c, c->cmaxb.ensure((size_t)mx * K * sizeof(int)), "maxima alloc");
   Stager sg(c, props, reqs, w);
   sg.cvt32 = all_host64;
   if ((st = sg.prepare(outs)) != P2_OK) return st;
@@ -394,7 +388,7 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     a.g16_raw = g16_raw(what) ? 1 : 0;
     if (fused) {
       p2::ContractArgs r = a;
-      r.out = c->axes_ws.p;
+      r.out = s1;
       r.Lx = c->Ll[0];
       r.R1 = ap->R1;
       ProfScope ps(c, "contract_site");
@@ -404,6 +398,8 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
         P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), ap->rows, 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
     }
     if ((a.what = rest)) {
+      a.K = Kr;
+      a.k = offsets_of(rest);
       ProfScope ps(c, "contract_f32");
       P2_TRY(c, p2::launch_contract_f32(a, chunk_fp32, 2 * c->nsm, c->stream), "contract kernel");
     }
@@ -412,14 +408,14 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     const int* kexp = (const int*)c->kexp.p;
     const int* kphase = g16_phase_deferred(what) ? kexp + 2 * K : nullptr;
     if (ap) {
-      if (rest && (st = axes_x_blocks(c, *ap, pl, what, rest, c->cbuf.p, 1, n, c->axes_ws.p)) != P2_OK) return st;
+      if (rest && (st = axes_x_blocks(c, *ap, what, rest, c->cbuf.p, 1, n, s1)) != P2_OK) return st;
       AxesOut ao;
       ao.dsl = dsl;
       ao.exps = (const int*)c->expb.p;
       ao.kexp = kexp;
       ao.kphase = kphase;
       ao.blocks = &pl.blocks;
-      if ((st = axes_yz(c, *ap, c->axes_ws.p, 1, n, K, ao)) != P2_OK) return st;
+      if ((st = axes_yz(c, *ap, s1, 1, n, K, ao)) != P2_OK) return st;
     } else if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, (const int*)c->expb.p, kexp, pl.blocks, nullptr,
                                    0, 0, kphase)) != P2_OK) {
       return st;

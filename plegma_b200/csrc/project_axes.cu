@@ -665,10 +665,6 @@ size_t axes_s1_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, si
 size_t axes_ws_bytes(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K) {
   return axes_s1_bytes(c, ap, fp32, n, K) + n * c->Ll[2] * ap.NP * K * (fp32 ? 8 : 16);
 }
-size_t axes_ws_start(const p2_ctx* c, const AxesPlan& ap, int fp32, size_t n, size_t K) {
-  const size_t buf = n * K * (size_t)c->V3 * (fp32 ? 8 : 16);
-  return std::max(std::min(buf, (size_t)64 << 20), axes_ws_bytes(c, ap, fp32, n, K));
-}
 
 // Sums over x of n slices of K components of a position buffer into the
 // first K of the Kst components of s1.
@@ -705,23 +701,25 @@ unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what) {
   return (what & kDelta) | (what & ~(kPass2 | kMes) ? 0u : what & kMes);
 }
 
-p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, const Plan& pl, unsigned what, unsigned bits, const void* cbuf,
-                        int fp32, int n, void* s1) {
+p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, unsigned what, unsigned rest, const void* cbuf, int fp32, int n,
+                        void* s1) {
   const size_t esz = fp32 ? 8 : 16;
-  // runs of neighbouring blocks; pl.blocks follows kBlocks
-  int k0 = 0, k1 = 0;
+  const int K = components_of(what), Kr = components_of(rest);
+  // runs of neighbouring blocks of `rest`, [k0, k1) in `what`, from component q0 of the buffer
+  int k0 = 0, k1 = 0, q0 = 0;
   for (size_t i = 0; i <= sizeof(kBlocks) / sizeof(kBlocks[0]); i++) {
     const bool end = i == sizeof(kBlocks) / sizeof(kBlocks[0]);
     if (!end && !(what & kBlocks[i].bit)) continue;
     const int comps = end ? 0 : kBlocks[i].groups * kBlocks[i].datasets * kBlocks[i].comps;
-    if (!end && (bits & kBlocks[i].bit)) {
+    if (!end && (rest & kBlocks[i].bit)) {
       k1 += comps;
       continue;
     }
     if (k1 > k0) {
-      p2_status st = axes_x(c, ap, (const char*)cbuf + (size_t)k0 * c->V3 * esz, fp32, (long long)pl.K * c->V3, c->V3,
-                            n, k1 - k0, pl.K, (char*)s1 + (size_t)k0 * esz);
+      p2_status st = axes_x(c, ap, (const char*)cbuf + (size_t)q0 * c->V3 * esz, fp32, (long long)Kr * c->V3, c->V3, n,
+                            k1 - k0, K, (char*)s1 + (size_t)k0 * esz);
       if (st != P2_OK) return st;
+      q0 += k1 - k0;
     }
     k0 = k1 = k1 + comps;
   }

@@ -625,20 +625,12 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
   }
   if (!up.empty() && (st = upload_async(c, U.args, up.data(), up.size(), "udsc arguments")) != P2_OK) return st;
 
-  // slices of a chunk; the buffers are sized for the largest group at once
-  const size_t esz = split ? 8 : 16;
-  auto chunk_of = [&](const UdscGroup& g) {
-    const size_t fit = c->ws_budget / std::max<size_t>((size_t)g.K * (size_t)c->V3 * esz, 1);
-    return (int)std::max<size_t>(1, std::min<size_t>(fit, (size_t)T));
-  };
-  size_t cbytes = 0, wbytes = 0;
-  for (const UdscGroup& g : groups) {
-    const size_t n = std::min((size_t)chunk_of(g), g.taus.size());
-    cbytes = std::max(cbytes, n * (size_t)g.K * (size_t)c->V3 * esz);
-    if (ap) wbytes = std::max(wbytes, axes_ws_bytes(c, *ap, split, n, g.K));
-  }
-  P2_TRY(c, c->cbuf.ensure(cbytes), "position buffer alloc");
-  if (ap) P2_TRY(c, c->axes_ws.ensure(wbytes), "projection workspace");
+  // slices of a chunk; the scratch is sized for the largest group at once
+  auto chunk_of = [&](const UdscGroup& g) { return chunk_slices(c, slice_bytes(c, ap, split, g.K, g.K, false), T); };
+  size_t bytes = 0;
+  for (const UdscGroup& g : groups)
+    bytes = std::max(bytes, scratch_bytes(c, ap, split, std::min((size_t)chunk_of(g), g.taus.size()), g.K, g.K));
+  P2_TRY(c, c->cbuf.ensure(bytes), "workspace alloc");
 
   for (const UdscGroup& g : groups) {
     const int nf = (int)g.flavours.size(), K = g.K, n_all = (int)g.taus.size();
@@ -694,7 +686,8 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
         P2_TRY(c, launch_contract_udsc(a, nf, c->nsm, c->stream), "udsc contraction");
       }
       if (ap) {
-        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, K, c->axes_ws.p)) != P2_OK)
+        void* const s1 = (char*)c->cbuf.p + sums_offset(c, split, n, K);
+        if ((st = axes_x(c, *ap, c->cbuf.p, split, (long long)K * c->V3, c->V3, n, K, K, s1)) != P2_OK)
           return st;
         AxesOut ao;
         ao.dsl = dsl;
@@ -703,7 +696,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
           ao.exps = a.es;
           ao.kexp = kexp;
         }
-        if ((st = axes_yz(c, *ap, c->axes_ws.p, split, n, K, ao)) != P2_OK) return st;
+        if ((st = axes_yz(c, *ap, s1, split, n, K, ao)) != P2_OK) return st;
       } else if (split) {
         if ((st = split_project(c, pl, K, n, nmtile, nkstep, dsl, a.es, kexp, blocks)) != P2_OK) return st;
       } else if ((st = project_direct(c, pl, K, n, n, dsl, blocks)) != P2_OK) {

@@ -121,3 +121,40 @@ def test_sums_of_equal_values(what, baryons, L):
         err = np.abs(res - ref) / np.where(held, scale, np.inf)
         assert err.max() < 1e-6, err.max()
     ctx.close()
+
+
+@pytest.mark.parametrize("what,mode", [
+    (NUC | D | G16, SPLIT), (NUC | D | G16, p2.P2_PLAIN_FP64),
+    (p2.NUCLEON_NTOR | p2.NUCLEON_RTON | D | p2.MESON_ALL34, SPLIT),
+    (p2.NUCLEON_NTOR | p2.NUCLEON_RTON | D | p2.MESON_ALL34, p2.P2_PLAIN_FP64),
+    ("udsc", p2.P2_PLAIN_FP64),
+])
+def test_scratch_stays_within_the_workspace(what, mode):
+    """The position buffer and the sums over x and y share the workspace
+    budget: on a short x axis the sums take more than the buffer.  Same bits
+    with and without the limit."""
+    L, moms, T = (2, 64, 32, 24), p2.mom_list(1), 24
+    budget, slack = 80 << 20, 12 << 20  # slack: tables, descriptors and the driver's granularity
+    got = []
+    for limit in (None, budget):  # the first pass loads the kernels and fills torch's pool
+        torch.cuda.synchronize()
+        ctx = p2.Context(L)
+        bufs = device_props(ctx, [(67, 0), (67, 1)], t0=0)
+        n = 28 if what == "udsc" else p2.components(what)
+        out = torch.zeros(n * T * len(moms), dtype=torch.complex128, device="cuda")
+        if limit:
+            ctx.set_workspace(limit)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        props = [ctx.prop(b.data_ptr()) for b in bufs]
+        if what == "udsc":
+            ctx.contract_udsc(props, ctx.udsc_request((0, 0, 0, 0), T, out.data_ptr(), moms=moms, mode=mode, prop_u=0,
+                                                      prop_d=1))
+        else:
+            ctx.contract_project(props, [ctx.request((0, 0, 0, 0), T, what, out.data_ptr(), mode=mode, moms=moms)])
+        ctx.sync()
+        used = free - torch.cuda.mem_get_info()[0]
+        got.append(out.cpu().numpy())
+        ctx.close()
+    assert np.array_equal(got[0], got[1])
+    assert used <= budget + slack, used >> 20
