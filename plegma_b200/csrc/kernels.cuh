@@ -237,7 +237,7 @@ struct AxisZArgs {
   double* out;
 };
 cudaError_t launch_axis_x(const AxisXArgs& a, int fp32, cudaStream_t s);
-cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s);
+cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, int nsm, cudaStream_t s);
 cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s);
 
 cudaError_t launch_contract_plain(const ContractArgs& a, int grid, cudaStream_t s);

@@ -420,11 +420,11 @@ cudaError_t launch_x_t(const AxisXArgs& a, cudaStream_t s) {
 }
 
 template <typename R, int KPL, int W>
-cudaError_t launch_y(const AxisYArgs& a0, cudaStream_t s) {
+cudaError_t launch_y(const AxisYArgs& a0, int nsm, cudaStream_t s) {
   AxisYArgs a = a0;
   // as many z per block as leave about eight blocks per SM: a block fills the phase table first
   const long long per_z = (long long)((a.K + 32 * KPL - 1) / (32 * KPL)) * a.ntau;
-  a.zper = (int)std::max<long long>(1, std::min<long long>(a.Lz, per_z * a.Lz / (8 * 148)));
+  a.zper = (int)std::max<long long>(1, std::min<long long>(a.Lz, per_z * a.Lz / (8 * nsm)));
   const int smem = a.RY * ((a.Ly + kYUnroll - 1) / kYUnroll * kYUnroll) * (int)sizeof(R);
   if (smem > 48 << 10) {
     cudaError_t e = ensure_smem((const void*)k_axis_y<R, KPL, W>, smem);
@@ -513,11 +513,11 @@ cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
   return fp32 ? launch_x_t<float>(a, s) : launch_x_t<double>(a, s);
 }
 
-cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, cudaStream_t s) {
+cudaError_t launch_axis_y(const AxisYArgs& a, int fp32, int kpl, int nsm, cudaStream_t s) {
   constexpr int W = kAxisMaxRows;
-  if (!fp32) return kpl == 2 ? launch_y<double, 2, W>(a, s) : launch_y<double, 1, W>(a, s);
-  if (a.R1 <= 7) return kpl == 2 ? launch_y<float, 2, 7>(a, s) : launch_y<float, 1, 7>(a, s);
-  return kpl == 2 ? launch_y<float, 2, W>(a, s) : launch_y<float, 1, W>(a, s);
+  if (!fp32) return kpl == 2 ? launch_y<double, 2, W>(a, nsm, s) : launch_y<double, 1, W>(a, nsm, s);
+  if (a.R1 <= 7) return kpl == 2 ? launch_y<float, 2, 7>(a, nsm, s) : launch_y<float, 1, 7>(a, nsm, s);
+  return kpl == 2 ? launch_y<float, 2, W>(a, nsm, s) : launch_y<float, 1, W>(a, nsm, s);
 }
 
 cudaError_t launch_axis_z(const AxisZArgs& a, int fp32, cudaStream_t s) {
@@ -749,16 +749,16 @@ p2_status axes_yz(p2_ctx* c, const AxesPlan& ap, const void* s1, int fp32, int n
   std::vector<std::vector<int>> cands{{1}, {2}};
   if (fp32 && (long long)n * Lz * ((K + 63) / 64) >= 2LL * c->nsm) std::swap(cands[0], cands[1]);
   char key[160];
-  std::snprintf(key, sizeof(key), "%s axes V3=%lld K=%d nmom=%d n=%d", fp32 ? "project_split" : "project_fp64", c->V3, K,
-                ap.nmom, n);
+  std::snprintf(key, sizeof(key), "%s axes y=%d z=%d rows=%d pairs=%d K=%d n=%d",
+                fp32 ? "project_split" : "project_fp64", y.Ly, Lz, ap.R1, ap.NP, K, n);
   std::vector<int> pick;
   P2_TRY(c,
          tune_choose(c->tuner.get(), key, cands, c->stream, !c->capturing,
-                     [&](const std::vector<int>& v) { return p2::launch_axis_y(y, fp32, v[0], c->stream); }, pick),
+                     [&](const std::vector<int>& v) { return p2::launch_axis_y(y, fp32, v[0], c->nsm, c->stream); }, pick),
          "projection tuning");
   {
     ProfScope ps(c, "project_axis_y");
-    P2_TRY(c, p2::launch_axis_y(y, fp32, pick[0], c->stream), "projection over y");
+    P2_TRY(c, p2::launch_axis_y(y, fp32, pick[0], c->nsm, c->stream), "projection over y");
   }
   p2::AxisZArgs z{};
   z.s2 = s2;

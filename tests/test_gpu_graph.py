@@ -137,3 +137,23 @@ def test_tuner_caches_choices_and_stays_accurate(tmp_path, mode):
         assert torch.equal(a, b)
     ctx2.close()
     assert os.path.exists(path)
+
+
+def test_tuner_keeps_shapes_apart(tmp_path):
+    """Lattices of one volume whose y and z extents differ, and lists of one
+    length with other phase rows, have choices of their own in a shared file."""
+    path = str(tmp_path / "tune.tsv")
+    lists = [np.array([[0, 0, 0], [1, 0, 0], [-1, 0, 0]], np.int32), np.array([[0, 0, 0], [0, 1, 0], [0, -1, 0]], np.int32)]
+    count = []
+    for L in ((8, 4, 6, 4), (4, 6, 8, 4)):
+        for moms in lists:
+            ctx = p2.Context(L)
+            ctx.tune(True, path)
+            bufs = device_props(ctx, [(91, 0), (91, 1)], t0=0)
+            out = torch.zeros(p2.block_info(NUC, 4, len(moms))[1], dtype=torch.complex128, device="cuda")
+            ctx.contract_project([ctx.prop(b.data_ptr()) for b in bufs],
+                                 [ctx.request((0, 0, 0, 0), 4, NUC, out.data_ptr(), moms=moms, mode=p2.P2_SPLIT_FP16)])
+            ctx.sync()
+            count.append(ctx.tune_count())
+            ctx.close()
+    assert count == [1, 2, 3, 4]
