@@ -539,7 +539,7 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
     c->plain_moms_key = pl.moms;
   }
 
-  const unsigned fused = fused_bits(c, ap, what), rest = what & ~fused;
+  const unsigned fused = fused_bits(c, ap, what, 0), rest = what & ~fused;
   const int Kr = components_of(rest);  // components of the position buffer
   const size_t per = slice_bytes(c, ap, 0, pl.K, Kr, any_host(props, reqs, idx, nidx));
   const Work w = make_work(c, props, reqs, idx, nidx, chunk_slices(c, per, c->T));
@@ -570,9 +570,9 @@ p2_status run_plain(p2_ctx* c, const p2_prop* props, const p2_request* reqs, con
       r.R1 = ap->R1;
       ProfScope ps(c, "contract_site");
       if ((r.what = fused & (P2_NUCLEON_CG5 | P2_MESON_G16)))
-        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), ap->rows, 1, 0, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
       if ((r.what = fused & (P2_DELTA_ISO12 | P2_DELTA_ISO32)))
-        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), ap->rows, 1, 0, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), 1, 0, c->nsm, c->stream), "contract kernel");
     }
     if ((a.what = rest)) {
       a.K = Kr;

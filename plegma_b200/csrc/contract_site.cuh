@@ -16,8 +16,8 @@
 // prefetched into L2 during a tile's contraction; its u half is loaded into
 // registers before the last phase of the contraction, its d half before the
 // sums over x, so that both latencies are covered.  A row's sites are added
-// in order by one thread, in the split form by groups that depend on Lx alone
-// (RowGroups), so a row's sum does not depend on the launch shape.
+// in order by one thread, in the split form by fours that count from the
+// slice's first site, so a row's sum does not depend on the launch shape.
 // The x phases are kernel parameters: they come through the constant bank and
 // cost no shared-memory wavefronts (copied to shared memory the plain form was
 // 14 % slower).
@@ -51,49 +51,45 @@ struct Cfg {
 };
 
 // ---- sums over x -----------------------------------------------------------------
-// t: [Lx][phase_stride(RT)]; g: the groups of a row (split form)
+// [Lx][phase_stride(RT)]
 template <typename R>
 struct __align__(16) XPhases {
   R t[kRowsMaxPhases];
-  RowGroups g;
 };
 __host__ __device__ constexpr int phase_stride(int RT) { return (RT + 3) / 4 * 4; }
 
 // Sums of one output position for N units of phase rows: FP32 a unit is a
-// packed pair of rows (one paired FMA for both), FP64 one row.  FP32 sums run
-// over a group of sites (RowGroups) and fold() adds the group to the row's.
+// packed pair of rows (one paired FMA for both), FP64 one row.  FP32 sums take
+// four sites at a time, whose sum is formed first (kSumGroup in kernels.cuh
+// says why; it costs an addition per sum and four sites).
 template <typename R, int N>
 struct RowSums;
 template <int N>
 struct RowSums<float, N> {
   static constexpr int kRows = 2;  // rows per unit
-  f32x2 re[N], im[N];    // the row's groups
-  f32x2 gre[N], gim[N];  // the group
+  f32x2 re[N], im[N];
   __device__ __forceinline__ void clear() {
 #pragma unroll
     for (int i = 0; i < N; i++) re[i] = im[i] = f2pack(0.f, 0.f);
   }
-  __device__ __forceinline__ void begin() {
+  // sites v[0..4) with the phases f[j * stride]; the first m of them (the others' values are zero)
+  __device__ __forceinline__ void add4(const float* f, int stride, const Cx<float> (&v)[4], int m = 4) {
+    f32x2 a[N], b[N];
 #pragma unroll
-    for (int i = 0; i < N; i++) gre[i] = gim[i] = f2pack(0.f, 0.f);
-  }
-  __device__ __forceinline__ void add(const float* f, Cx<float> v) {
-    const f32x2 vx = f2pack(v.x, v.x), vy = f2pack(v.y, v.y);
-    const unsigned long long* q = reinterpret_cast<const unsigned long long*>(f);
+    for (int j = 0; j < 4; j++) {
+      const unsigned long long* q = reinterpret_cast<const unsigned long long*>(f + min(j, m - 1) * stride);
+      const f32x2 vx = f2pack(v[j].x, v[j].x), vy = f2pack(v[j].y, v[j].y);
+#pragma unroll
+      for (int i = 0; i < N; i++) {
+        a[i] = j ? f2fma(q[i], vx, a[i]) : f2mul(q[i], vx);
+        b[i] = j ? f2fma(q[i], vy, b[i]) : f2mul(q[i], vy);
+      }
+    }
 #pragma unroll
     for (int i = 0; i < N; i++) {
-      const unsigned long long p = q[i];
-      gre[i] = f2fma(p, vx, gre[i]);
-      gim[i] = f2fma(p, vy, gim[i]);
+      re[i] = f2add(re[i], a[i]);
+      im[i] = f2add(im[i], b[i]);
     }
-  }
-  __device__ __forceinline__ void fold() {
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-      re[i] = f2add(re[i], gre[i]);
-      im[i] = f2add(im[i], gim[i]);
-    }
-    begin();
   }
   __device__ __forceinline__ void write(Cx<float>* o, int row, int R1, long long K) {
 #pragma unroll
@@ -123,8 +119,10 @@ struct RowSums<double, N> {
       s[i].y = fma(f[i], v.y, s[i].y);
     }
   }
-  __device__ __forceinline__ void begin() {}
-  __device__ __forceinline__ void fold() {}
+  __device__ __forceinline__ void add4(const double* f, int stride, const Cx<double> (&v)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; j++) add(f + j * stride, v[j]);
+  }
   __device__ __forceinline__ void write(Cx<double>* o, int row, int R1, long long K) {
 #pragma unroll
     for (int i = 0; i < N; i++)
@@ -139,51 +137,40 @@ constexpr int row_units(int RT, int share) {
 }
 
 // A CTA's walk over units of a.unit whole rows (the last unit of a slice
-// fewer), each in tiles of up to kS consecutive sites; in the split form a tile
-// ends with a group, so that no group's sum is carried from one tile to the
-// next (both sums live through the contraction made the kernels 4 to 12 %
-// slower by spills, a place for them in shared memory as much by a smaller L1).
-// The units of all slices are numbered through and a CTA takes every
-// gridDim.x-th.
+// fewer), each in tiles of up to kS consecutive sites.  The units of all slices
+// are numbered through and a CTA takes every gridDim.x-th.
+// Split form: the sites that are added together (add_x) are the fours of the
+// slice's sites within a row, and a tile ends with one, so that their sum is
+// never carried from tile to tile: that made the kernels 4 to 12 % slower (in
+// registers by spills, in shared memory by a smaller L1, in the result by the
+// loads).  Only a unit's first tile is shorter by it, by up to three sites.
 template <typename R>
 struct Cursor {
   static constexpr int kS = Cfg<R>::kS;
   int tl, unit, x0, n;  // slice, unit, first site of the tile in the slice, sites of the tile
   int row, x;           // of the first site
-  int nrow, nx;         // split form: of the site after the last
   __device__ __forceinline__ int end(const ContractArgs& a) const { return min(a.V3, (unit + 1) * a.unit * a.Lx); }
-  __device__ __forceinline__ void fit(const ContractArgs& a, const RowGroups& g) {
-    n = min(kS, end(a) - x0);
-    if constexpr (sizeof(R) == 4) {
-      nrow = row;
-      for (nx = x + n; nx >= a.Lx; nx -= a.Lx) nrow++;
-      const int b = g.begin[nx];
-      n -= nx - b;
-      nx = b;
-    }
+  __device__ __forceinline__ void fit(const ContractArgs& a) {
+    const int left = end(a) - x0;
+    n = min(kS - (sizeof(R) == 4 ? x0 & 3 : 0), left);
   }
-  __device__ __forceinline__ void place(const ContractArgs& a, const RowGroups& g) {
+  __device__ __forceinline__ void place(const ContractArgs& a) {
     row = unit * a.unit;
     x = 0;
     x0 = row * a.Lx;
-    fit(a, g);
+    fit(a);
   }
-  __device__ __forceinline__ void first(const ContractArgs& a, const RowGroups& g) {
+  __device__ __forceinline__ void first(const ContractArgs& a) {
     tl = (int)(blockIdx.x / (unsigned)a.upt);
     unit = (int)(blockIdx.x % (unsigned)a.upt);
-    place(a, g);
+    place(a);
   }
   __device__ __forceinline__ bool valid(const ContractArgs& a) const { return tl < a.ntau; }
-  __device__ __forceinline__ void next(const ContractArgs& a, const RowGroups& g) {
-    x0 += n;
-    if (x0 < end(a)) {
-      if constexpr (sizeof(R) == 4) {
-        row = nrow;
-        x = nx;
-      } else {
-        for (x += kS; x >= a.Lx; x -= a.Lx) row++;
-      }
-      fit(a, g);
+  __device__ __forceinline__ void next(const ContractArgs& a) {
+    if (x0 + n < end(a)) {
+      x0 += n;
+      for (x += n; x >= a.Lx; x -= a.Lx) row++;
+      fit(a);
     } else {  // gridDim.x units further, without a division
       tl += a.step_slice;
       unit += a.step_unit;
@@ -191,7 +178,7 @@ struct Cursor {
         unit -= a.upt;
         tl++;
       }
-      place(a, g);
+      place(a);
     }
   }
 };
@@ -199,28 +186,46 @@ struct Cursor {
 // Adds the tile's values of one output position (val(s), sites 0..n-1) into
 // its sums for the phase rows from `first` on, writing every x row that ends.
 template <typename R, int RT, int N, typename Val>
-__device__ __forceinline__ void add_x(const ContractArgs& a, const XPhases<R>& ph, RowSums<R, N>& acc, int first,
+__device__ __forceinline__ void add_x(const ContractArgs& a, const R* ph, RowSums<R, N>& acc, int first,
                                       const Cursor<R>& c, int k, Val&& val) {
   constexpr int kStride = phase_stride(RT);
   const int rows = a.V3 / a.Lx;
   int row = c.row, x = c.x, s = 0;
-  acc.begin();
   while (s < c.n) {
-    // the sites of this group (split form) or row
-    const int end = sizeof(R) == 4 ? s + ph.g.end[x] - x : min(c.n, s + a.Lx - x);
-    const R* f = ph.t + x * kStride + first;
+    const int end = min(c.n, s + a.Lx - x);  // the sites of this row
+    const R* f = ph + x * kStride + first;
     x += end - s;
+    if constexpr (sizeof(R) == 4) {
+      // one to three sites before the first of the slice's fours, and after the last
+      auto some = [&](int m) {
+        Cx<R> v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) v[i] = i < m ? val(s + i) : czero<R>();
+        acc.add4(f, kStride, v, m);
+        s += m;
+        f += m * kStride;
+      };
+      const int head = min(end - s, -(c.x0 + s) & 3);
+      if (head) some(head);
 #pragma unroll 1
-    for (; s + 4 <= end; s += 4, f += 4 * kStride) {
-      Cx<R> v[4];
+      for (; s + 4 <= end; s += 4, f += 4 * kStride) {
+        Cx<R> v[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) v[i] = val(s + i);
+        for (int i = 0; i < 4; i++) v[i] = val(s + i);
+        acc.add4(f, kStride, v);
+      }
+      if (s < end) some(end - s);
+    } else {
+#pragma unroll 1
+      for (; s + 4 <= end; s += 4, f += 4 * kStride) {
+        Cx<R> v[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) acc.add(f + i * kStride, v[i]);
+        for (int i = 0; i < 4; i++) v[i] = val(s + i);
+        acc.add4(f, kStride, v);
+      }
+#pragma unroll 1
+      for (; s < end; s++, f += kStride) acc.add(f, val(s));
     }
-#pragma unroll 1
-    for (; s < end; s++, f += kStride) acc.add(f, val(s));
-    acc.fold();
     if (x == a.Lx) {
       acc.write((Cx<R>*)a.out + ((long long)c.tl * rows + row) * a.R1 * a.K + k, first, a.R1, a.K);
       x = 0;
@@ -421,14 +426,13 @@ __device__ __forceinline__ void diquark_add(const Cx<R> (&x)[9], const Cx<R> (&y
 
 // xt: [Lx][R1] phase rows; one CTA per SM (its shared memory and registers fill it)
 template <typename R, typename K>
-cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, const RowPlan& rp, int RT, int smem,
-                         int nsm, cudaStream_t s) {
+cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, int RT, int smem, int nsm,
+                         cudaStream_t s) {
   constexpr int kS = Cfg<R>::kS;
   ContractArgs a = a0;
   const int stride = phase_stride(RT);
   if (a.Lx * stride > kRowsMaxPhases || a.R1 > RT) return cudaErrorInvalidValue;
   XPhases<R> ph;
-  ph.g = rp.g;
   for (int i = 0; i < a.Lx; i++)
     for (int r = 0; r < stride; r++) ph.t[i * stride + r] = r < a.R1 ? (R)xt[i * a.R1 + r] : R(0);
   // rows per unit: the fewest tiles per CTA, the smaller unit on a tie (a unit
@@ -437,7 +441,8 @@ cudaError_t launch_tiles(K kernel, const ContractArgs& a0, const double* xt, con
   long long best = -1;
   for (int m = 1; m <= kS && m <= rows; m++) {
     const long long units = (long long)((rows + m - 1) / m) * a.ntau;
-    const long long cost = (units + nsm - 1) / nsm * (kS == 32 ? rp.tiles[m] : (m * a.Lx + kS - 1) / kS);
+    const int cut = sizeof(R) == 4 && m * a.Lx % 4 ? 3 : 0;  // of a unit's first tile
+    const long long cost = (units + nsm - 1) / nsm * ((m * a.Lx + cut + kS - 1) / kS);
     if (best < 0 || cost < best) {
       best = cost;
       a.unit = m;

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
   acc.clear();
 
   Cursor<R> cur, nx;
-  cur.first(a, ph.g);
+  cur.first(a);
 #pragma unroll 1
   for (int f = 0; f < 2; f++) {
     Loader<R, Tin> ld;
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
   __syncthreads();
   for (; cur.valid(a); cur = nx) {
     nx = cur;
-    nx.next(a, ph.g);
+    nx.next(a);
     prefetch<R, Tin>(a, nx, w, lane);
     // outputs of (m, r) = (w & 3, w >> 2): o[g][j], j = 0 Delta+, 1 Delta0, 2 Delta++, 3 Delta-
     Cx<R> o[3][4];
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
     {
       const int share = warp / (kOut / 32), pos = tid % kOut;
       if (share < kShare && (a.what & (pos < 96 ? 2u : 4u)))
-        add_x<R, RT>(a, ph, acc, share * NU * RowSums<R, NU>::kRows, cur, pos < 96 ? a.k.diso12 + pos : a.k.diso32 + pos - 96,
+        add_x<R, RT>(a, ph.t, acc, share * NU * decltype(acc)::kRows, cur, pos < 96 ? a.k.diso12 + pos : a.k.diso32 + pos - 96,
                         [&](int i) { return so[pos * kOutStride + i]; });
     }
     ld.store(a, nx, t, w);
@@ -266,24 +266,24 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
 }
 
 template <typename R, typename Tin, int RT>
-cudaError_t go(const ContractArgs& a, const double* xt, const RowPlan& rp, int nsm, cudaStream_t s) {
-  return launch_tiles<R>(k_site_delta<R, Tin, RT>, a, xt, rp, RT, Mem<R>::kAll, nsm, s);
+cudaError_t go(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s) {
+  return launch_tiles<R>(k_site_delta<R, Tin, RT>, a, xt, RT, Mem<R>::kAll, nsm, s);
 }
 
 template <typename R, typename Tin>
-cudaError_t go_rows(const ContractArgs& a, const double* xt, const RowPlan& rp, int nsm, cudaStream_t s) {
-  return a.R1 <= 3   ? go<R, Tin, 3>(a, xt, rp, nsm, s)
-         : a.R1 <= 7 ? go<R, Tin, 7>(a, xt, rp, nsm, s)
-                     : go<R, Tin, 9>(a, xt, rp, nsm, s);
+cudaError_t go_rows(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s) {
+  return a.R1 <= 3   ? go<R, Tin, 3>(a, xt, nsm, s)
+         : a.R1 <= 7 ? go<R, Tin, 7>(a, xt, nsm, s)
+                     : go<R, Tin, 9>(a, xt, nsm, s);
 }
 
 }  // namespace
 }  // namespace site
 
-cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, const RowPlan& rp, int plain, int fp32_in,
-                              int nsm, cudaStream_t s) {
-  if (plain) return site::go_rows<double, double>(a, xt, rp, nsm, s);
-  return fp32_in ? site::go_rows<float, float>(a, xt, rp, nsm, s) : site::go_rows<float, double>(a, xt, rp, nsm, s);
+cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                              cudaStream_t s) {
+  if (plain) return site::go_rows<double, double>(a, xt, nsm, s);
+  return fp32_in ? site::go_rows<float, float>(a, xt, nsm, s) : site::go_rows<float, double>(a, xt, nsm, s);
 }
 
 }  // namespace p2

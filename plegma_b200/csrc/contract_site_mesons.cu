@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
   const int rows = a.V3 / a.Lx;
 
   Cursor<R> cur, nx;
-  cur.first(a, ph.g);
+  cur.first(a);
 #pragma unroll 1
   for (int f = 0; f < 2; f++) {
     Loader<R, Tin> ld;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
   __syncthreads();
   for (; cur.valid(a); cur = nx) {
     nx = cur;
-    nx.next(a, ph.g);
+    nx.next(a);
     prefetch<R, Tin>(a, nx, role, site);
     // ---- A ----
     {
@@ -163,33 +163,50 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
     ld.store(a, nx, t, role);
     ld.load(a, nx, 1, role, site);
     if (mes)
-      add_x<R, RT>(a, ph, acc, warp / 8 * NU * RowSums<R, NU>::kRows, cur, a.k.g16 + tid % 256,
+      add_x<R, RT>(a, ph.t, acc, warp / 8 * NU * decltype(acc)::kRows, cur, a.k.g16 + tid % 256,
                    [&](int s) { return so[(tid % 256) * kOutStride + s]; });
     if (nuc) {
       const int lane = tid & 31, w = warp;
       int row = cur.row, x = cur.x, s = 0;
       const Cx<R>* src = so + (256 + lane) * kOutStride;
       while (s < cur.n) {
-        constexpr bool kGroups = sizeof(R) == 4;
-        const int end = kGroups ? s + ph.g.end[x] - x : min(cur.n, s + a.Lx - x);
-        Cx<R> g[kNR];
+        const int end = min(cur.n, s + a.Lx - x);
+        if constexpr (sizeof(R) == 4) {
+          // fours as in add_x
+          auto some = [&](int m) {
+            Cx<R> g = czero<R>();
 #pragma unroll
-        for (int i = 0; i < kNR; i++) g[i] = kGroups ? czero<R>() : accn[i];
+            for (int i = 0; i < 4; i++)
+              if (i < m && w < RT) {
+                const Cx<R> v = src[s + i];
+                const R f = ph.t[(x + i) * phase_stride(RT) + w];
+                g.x = fma(f, v.x, g.x);
+                g.y = fma(f, v.y, g.y);
+              }
+            accn[0] = accn[0] + g;
+            s += m;
+            x += m;
+          };
+          const int head = min(end - s, -(cur.x0 + s) & 3);
+          if (head) some(head);
+#pragma unroll 2
+          for (; s + 4 <= end;) some(4);
+          if (s < end) some(end - s);
+        } else {
 #pragma unroll 8
-        for (; s < end; s++, x++) {
-          const Cx<R> v = src[s];
+          for (; s < end; s++, x++) {
+            const Cx<R> v = src[s];
 #pragma unroll
-          for (int i = 0; i < kNR; i++) {
-            const int r = w + kWarps * i;
-            if (r < RT) {
-              const R f = ph.t[x * phase_stride(RT) + r];
-              g[i].x = fma(f, v.x, g[i].x);
-              g[i].y = fma(f, v.y, g[i].y);
+            for (int i = 0; i < kNR; i++) {
+              const int r = w + kWarps * i;
+              if (r < RT) {
+                const R f = ph.t[x * phase_stride(RT) + r];
+                accn[i].x = fma(f, v.x, accn[i].x);
+                accn[i].y = fma(f, v.y, accn[i].y);
+              }
             }
           }
         }
-#pragma unroll
-        for (int i = 0; i < kNR; i++) accn[i] = kGroups ? accn[i] + g[i] : g[i];
         if (x == a.Lx) {
           Cx<R>* o = (Cx<R>*)a.out + ((long long)cur.tl * rows + row) * a.R1 * a.K + a.k.nuc + lane;
 #pragma unroll
@@ -209,24 +226,24 @@ __global__ void __launch_bounds__(Cfg<R>::kTh, 1)
 }
 
 template <typename R, typename Tin, int RT>
-cudaError_t go(const ContractArgs& a, const double* xt, const RowPlan& rp, int nsm, cudaStream_t s) {
-  return launch_tiles<R>(k_site_mesons<R, Tin, RT>, a, xt, rp, RT, Mem<R>::kAll, nsm, s);
+cudaError_t go(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s) {
+  return launch_tiles<R>(k_site_mesons<R, Tin, RT>, a, xt, RT, Mem<R>::kAll, nsm, s);
 }
 
 template <typename R, typename Tin>
-cudaError_t go_rows(const ContractArgs& a, const double* xt, const RowPlan& rp, int nsm, cudaStream_t s) {
-  return a.R1 <= 3   ? go<R, Tin, 3>(a, xt, rp, nsm, s)
-         : a.R1 <= 7 ? go<R, Tin, 7>(a, xt, rp, nsm, s)
-                     : go<R, Tin, 9>(a, xt, rp, nsm, s);
+cudaError_t go_rows(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s) {
+  return a.R1 <= 3   ? go<R, Tin, 3>(a, xt, nsm, s)
+         : a.R1 <= 7 ? go<R, Tin, 7>(a, xt, nsm, s)
+                     : go<R, Tin, 9>(a, xt, nsm, s);
 }
 
 }  // namespace
 }  // namespace site
 
-cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, const RowPlan& rp, int plain, int fp32_in,
-                               int nsm, cudaStream_t s) {
-  if (plain) return site::go_rows<double, double>(a, xt, rp, nsm, s);
-  return fp32_in ? site::go_rows<float, float>(a, xt, rp, nsm, s) : site::go_rows<float, double>(a, xt, rp, nsm, s);
+cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                               cudaStream_t s) {
+  if (plain) return site::go_rows<double, double>(a, xt, nsm, s);
+  return fp32_in ? site::go_rows<float, float>(a, xt, nsm, s) : site::go_rows<float, double>(a, xt, nsm, s);
 }
 
 }  // namespace p2

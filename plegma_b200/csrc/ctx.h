@@ -57,7 +57,6 @@ struct AxesPlan {
   int R1 = 0, RY = 0, NP = 0, NO = 0, nmom = 0;
   DevBuf tab;  // phases, then the orbit lists
   std::vector<double> xth;  // xt on the host, for the fused contraction
-  p2::RowPlan rows;         // the same
   const double *xt = nullptr, *yt = nullptr, *zt = nullptr;
   std::vector<int> first, ylist;
   const int *orb = nullptr, *omom = nullptr;
@@ -260,7 +259,7 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
 // Some propagator of the requests is in host memory.
 bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int nidx);
 // Bits of a contraction set that the kernels fused with the sums over x take.
-unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what);
+unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what, int split);
 // The sums over x of the blocks `rest` of a set `what`, from a position buffer
 // that holds the components of `rest` alone (n slices, V3 sites each).
 p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, unsigned what, unsigned rest, const void* cbuf, int fp32, int n,

@@ -196,11 +196,13 @@ constexpr int kAxisMaxRows = 9;  // cos / sin rows per axis
 // Sites that the split form adds in one running FP32 sum.  Adding equal or
 // like-signed values rounds the same way at every step, so a sum's error
 // grows with its number of steps: one running sum over x and one over y were
-// 1.3e-6 of sum |c| off at 48 x 48 and 7e-6 at 240 x 240.  So sites are added
-// by groups of at most kSumGroup; the groups of a row again (at most 24, or in
-// FP64), those of a y sum by kSumGroups.  For equal values the two sums are
-// then off by at most 8e-7 at any admitted extents, 5e-7 at 48 x 48.
-constexpr int kSumGroup = 16, kSumGroups = 16;
+// 1.3e-6 of sum |c| off at 48 x 48 and 7e-6 at 240 x 240.  So the sums over x of
+// a position buffer add at most kSumGroup sites in FP32 and these in FP64, the
+// fused contraction four sites and these in FP32 (rows of at most kRowsMaxSplit
+// sites), the sums over y eight, then kSumGroups of those.  For equal values
+// the two sums are then off by at most 3.5e-7 at 48 x 48, 5.5e-7 at 96 x 48 and
+// 9.7e-7 at any admitted extents.
+constexpr int kSumGroup = 16, kSumGroups = 16, kRowsMaxSplit = 128;
 
 struct AxisXArgs {
   const void* c;      // complex double or complex float, element (tau, k, x) at c[tau*sT + k*sK + x]
@@ -247,20 +249,10 @@ cudaError_t launch_contract_f32(const ContractArgs& a, int fp32_in, int grid, cu
 // nucleon and the colour products of the 16 x 16 mesons; the Delta.  xt
 // [Lx][R1] the phase rows.
 constexpr int kRowsMaxPhases = 960;  // Lx x phase rows (4, 8 or 12) of the fused kernels' parameter block
-constexpr int kRowsMaxLx = kRowsMaxPhases / 4;
-// The groups of an x row, at most kSumGroup sites each: site x is in [begin[x], end[x]).
-struct RowGroups {
-  unsigned char begin[kRowsMaxLx], end[kRowsMaxLx];
-};
-struct RowPlan {
-  RowGroups g;
-  short tiles[33];  // tiles of 32 sites that a unit of m rows takes when each ends with a group
-};
-RowPlan row_plan(int Lx);  // Lx <= kRowsMaxLx
-cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, const RowPlan& rp, int plain, int fp32_in,
-                               int nsm, cudaStream_t s);
-cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, const RowPlan& rp, int plain, int fp32_in,
-                              int nsm, cudaStream_t s);
+cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                               cudaStream_t s);
+cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
+                              cudaStream_t s);
 cudaError_t launch_sample_exponents(const SampleArgs& a, cudaStream_t s);
 cudaError_t launch_project_fp64(const ProjArgs& a, cudaStream_t s);
 int project_fp64_tk(int K, int tk);  // component tile factor a launch with ProjArgs::tk uses

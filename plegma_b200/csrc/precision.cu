@@ -340,7 +340,7 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
     if ((st = split_prepare_tables(c, pl, what, nmtile, nkstep)) != P2_OK) return st;
   }
 
-  const unsigned fused = fused_bits(c, ap, what);
+  const unsigned fused = fused_bits(c, ap, what, 1);
   const unsigned rest = what & ~fused;
   const int Kr = components_of(rest);  // components of the position buffer
 
@@ -393,9 +393,9 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
       r.R1 = ap->R1;
       ProfScope ps(c, "contract_site");
       if ((r.what = fused & (P2_NUCLEON_CG5 | P2_MESON_G16)))
-        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), ap->rows, 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_mesons(r, ap->xth.data(), 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
       if ((r.what = fused & (P2_DELTA_ISO12 | P2_DELTA_ISO32)))
-        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), ap->rows, 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
+        P2_TRY(c, p2::launch_site_delta(r, ap->xth.data(), 0, chunk_fp32, c->nsm, c->stream), "contract kernel");
     }
     if ((a.what = rest)) {
       a.K = Kr;

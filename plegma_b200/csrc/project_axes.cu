@@ -466,45 +466,6 @@ struct AxisRows {
 
 }  // namespace
 
-// A row of Lx sites in equal groups.  Their number is that with the best filled
-// tiles of 32 sites: small groups leave less of a tile empty (a row of 21: two
-// groups, 30.5 sites of a tile on average; one in ten of all Lx loses more than
-// 10 %), each costs an addition per sum and a turn of the loop (0.8 % of a tile
-// per group, measured with two and four of them in a tile at Lx = 48).  It
-// depends on Lx alone, so that a row's sum does not depend on the launch.
-RowPlan row_plan(int Lx) {
-  RowPlan best{};
-  double least = 0;
-  const int n0 = (Lx + kSumGroup - 1) / kSumGroup;
-  for (int n = n0; n <= std::max(n0, std::min(24, Lx / 4)); n++) {
-    RowPlan p{};
-    auto start = [&](int i) { return i * Lx / n; };
-    for (int i = 0; i < n; i++)
-      for (int x = start(i); x < start(i + 1); x++) {
-        p.g.begin[x] = (unsigned char)start(i);
-        p.g.end[x] = (unsigned char)start(i + 1);
-      }
-    int left = 0;
-    for (int m = 1; m <= 32; m++) {
-      p.tiles[m] = p.tiles[m - 1];
-      for (int i = 0; i < n; i++) {
-        const int len = start(i + 1) - start(i);
-        if (left < len) {
-          p.tiles[m]++;
-          left = 32;
-        }
-        left -= len;
-      }
-    }
-    const double cost = p.tiles[32] + 0.008 * 32 * n;
-    if (n == n0 || cost < least) {
-      least = cost;
-      best = p;
-    }
-  }
-  return best;
-}
-
 cudaError_t launch_axis_x(const AxisXArgs& a0, int fp32, cudaStream_t s) {
   if (a0.ntau < 1 || a0.K < 1) return cudaSuccess;
   AxisXArgs a = a0;
@@ -645,7 +606,6 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
   ap.NO = (int)members.size();
   ap.nmom = nmom;
   ap.xth.assign(tab.begin(), tab.begin() + oy);
-  if (c->Ll[0] <= p2::kRowsMaxLx) ap.rows = p2::row_plan(c->Ll[0]);
   ap.xt = (const double*)ap.tab.p;
   ap.yt = ap.xt + oy;
   ap.zt = ap.xt + oz;
@@ -694,10 +654,11 @@ p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, lon
 // plain lattice 2.54 -> 2.39 ms), the nucleon would read its propagators a
 // second time.  Lists and lattices whose x phases exceed the parameters keep
 // the position buffer.
-unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what) {
+unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what, int split) {
   constexpr unsigned kDelta = P2_DELTA_ISO12 | P2_DELTA_ISO32, kMes = P2_NUCLEON_CG5 | P2_MESON_G16;
   constexpr unsigned kPass2 = kDelta | P2_NUCLEON_NTOR | P2_NUCLEON_RTON | P2_NUCLEON_RTOR;
   if (!ap || c->Ll[0] * (ap->R1 <= 3 ? 4 : ap->R1 <= 7 ? 8 : 12) > p2::kRowsMaxPhases) return 0;
+  if (split && c->Ll[0] > p2::kRowsMaxSplit) return 0;
   return (what & kDelta) | (what & ~(kPass2 | kMes) ? 0u : what & kMes);
 }
 
