@@ -260,6 +260,9 @@ p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const 
 bool any_host(const p2_prop* props, const p2_request* reqs, const int* idx, int nidx);
 // Bits of a contraction set that the kernels fused with the sums over x take.
 unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what, int split);
+// Split form: whether the axis-by-axis projection is faster than the tensor-core
+// one, which on large lattices takes at least `shortest` sites along x.
+bool axes_faster(const p2_ctx* c, int nmom, int shortest);
 // The sums over x of the blocks `rest` of a set `what`, from a position buffer
 // that holds the components of `rest` alone (n slices, V3 sites each).
 p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, unsigned what, unsigned rest, const void* cbuf, int fp32, int n,

@@ -322,11 +322,15 @@ p2_status precision_run_batch(p2_ctx* c, const p2_prop* props, const p2_request*
   }
   const int fp32_in = props[r0.prop_u].precision == P2_FP32;
   const int K = pl.K;
-  // the axis-by-axis projection when the momentum list qualifies, else the
-  // tensor-core one (which an armed p2_debug_wait_timeout asks for)
+  // the axis-by-axis projection when the momentum list qualifies and the x axis
+  // is not short (for the Delta it always is the faster one, by its fused
+  // contraction), else the tensor-core one (which an armed
+  // p2_debug_wait_timeout asks for)
   const AxesPlan* ap = nullptr;
   p2_status st;
   if (!c->wait_test && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
+  if (!(what & (P2_DELTA_ISO12 | P2_DELTA_ISO32)) && !axes_faster(c, pl.nmom, fused_bits(c, ap, what, 1) ? 8 : 16))
+    ap = nullptr;
   int nmtile = 0, nkstep = 0;
   if (ap) {
     if ((st = split_component_tables(c, what)) != P2_OK) return st;

@@ -653,13 +653,32 @@ p2_status axes_x(p2_ctx* c, const AxesPlan& ap, const void* field, int fp32, lon
 // gains from it beside such blocks (24^3 x 48 light baryons 4.77 -> 4.34 ms, odd
 // plain lattice 2.54 -> 2.39 ms), the nucleon would read its propagators a
 // second time.  Lists and lattices whose x phases exceed the parameters keep
-// the position buffer.
+// the position buffer, and so does the nucleon alone in the split form on
+// lattices of 200000 sites or more: most of a fused tile's time is spent on what
+// the mesons share (with, without the fusion, us: 48^3 x 96 1564, 1334; 24^3 x 48
+// 645, 600; 25 x 16 x 29 x 30 666, 555; but 16^3 x 32 173, 181; 8^3 x 16 60, 69).
 unsigned fused_bits(const p2_ctx* c, const AxesPlan* ap, unsigned what, int split) {
   constexpr unsigned kDelta = P2_DELTA_ISO12 | P2_DELTA_ISO32, kMes = P2_NUCLEON_CG5 | P2_MESON_G16;
   constexpr unsigned kPass2 = kDelta | P2_NUCLEON_NTOR | P2_NUCLEON_RTON | P2_NUCLEON_RTOR;
   if (!ap || c->Ll[0] * (ap->R1 <= 3 ? 4 : ap->R1 <= 7 ? 8 : 12) > p2::kRowsMaxPhases) return 0;
   if (split && c->Ll[0] > p2::kRowsMaxSplit) return 0;
-  return (what & kDelta) | (what & ~(kPass2 | kMes) ? 0u : what & kMes);
+  unsigned mes = what & ~(kPass2 | kMes) ? 0u : what & kMes;
+  if (split && mes == P2_NUCLEON_CG5 && c->V3 * c->Ll[3] >= 200000) mes = 0;
+  return (what & kDelta) | mes;
+}
+
+// On a short x axis the sums over x leave about as much as they read, and the
+// tensor-core projection is the faster one where its rows fit one tile of 128
+// and the lattice is not so small that launches decide (nucleon and 16 x 16
+// mesons, us, sums and tensor cores: 7 x 10 x 10 x 24 164 and 178, 7 x 20 x 20 x 16
+// 158 and 153, 6 x 40 x 40 x 16 365 and 320; without an x axis to sum over, 1 x 32 x
+// 32 x 16 200 and 152).  `shortest` is the first Lx where the sums win.  Measured at Lx x 48 x 40, 8 slices, 123 momenta, us, sums
+// and tensor cores: nucleon and 16 x 16 mesons, fused, Lx = 4 359 and 327, 6 429
+// and 363, 8 465 and 446, 16 737 and 774; 16 x 16 mesons alone 6 317 and 288, 8
+// 334 and 351; 34 mesons, not fused, 8 301 and 275, 16 468 and 450; nucleon, not
+// fused, 8 281 and 268, 16 449 and 446; u, d table-driven 3 425 and 409, 4 552 and 544.
+bool axes_faster(const p2_ctx* c, int nmom, int shortest) {
+  return c->V3 * c->Ll[3] < (c->Ll[0] > 1 ? 100000 : 10000) || nmom > 128 || c->Ll[0] >= shortest;
 }
 
 p2_status axes_x_blocks(p2_ctx* c, const AxesPlan& ap, unsigned what, unsigned rest, const void* cbuf, int fp32, int n,

@@ -518,6 +518,7 @@ p2_status p2_contract_udsc(p2_ctx* c, const p2_prop* props, int nprops, const p2
   const AxesPlan* ap = nullptr;  // the axis-by-axis projection, when the list qualifies
   // (an armed p2_debug_wait_timeout asks for the tensor-core projection)
   if (!(split && c->wait_test) && (st = axes_prepare(c, pl.moms, -1, &ap)) != P2_OK) return st;
+  if (split && !axes_faster(c, pl.nmom, 4)) ap = nullptr;
   int nmtile = 0, nkstep = 0;
   if (split && !ap) {
     if (c->project_split_smem_max < project_split_smem_bytes(project_split_max_nt()))

@@ -158,3 +158,49 @@ def test_scratch_stays_within_the_workspace(what, mode):
         ctx.close()
     assert np.array_equal(got[0], got[1])
     assert used <= budget + slack, used >> 20
+
+
+@pytest.mark.parametrize("L,what,q2,ran", [
+    ((7, 40, 40, 9), NUC | G16, 2, "project_split_tc"),   # short x axis
+    ((8, 40, 40, 9), NUC | G16, 2, "contract_site"),
+    ((7, 40, 40, 8), NUC | G16, 2, "contract_site"),      # 89600 sites
+    ((7, 40, 40, 9), NUC | G16, 10, "contract_site"),     # more than 128 momenta
+    ((7, 40, 40, 9), G16 | p2.DELTA_ISO12, 2, "contract_site"),
+    ((1, 50, 50, 4), G16, 2, "project_split_tc"),
+    ((1, 50, 50, 3), G16, 2, "contract_site"),
+    ((15, 30, 30, 8), p2.MESON_ALL34, 2, "project_split_tc"),
+    ((16, 30, 30, 8), p2.MESON_ALL34, 2, "project_axis_x"),
+    ((24, 25, 30, 12), NUC, 2, "project_axis_x"),         # the nucleon alone on a large lattice
+    ((24, 25, 30, 11), NUC, 2, "contract_site"),
+])
+def test_split_dispatch_by_size(L, what, q2, ran):
+    """Both sides of each line between the split form's paths: the kernel that runs and its result."""
+    ctx = p2.Context(L)
+    bufs = device_props(ctx, [(68, 0), (68, 1)], t0=0)
+    ctx.profile()
+    src = (L[0] - 1, 2, 3, 0)
+    out, moms = run(ctx, bufs, src, 2, what, q2max=q2, mode=SPLIT)
+    names = set(ctx.profile_read())
+    assert ran in names and ("project_split_tc" in names) != ("project_axis_y" in names), names
+    ref = oracle_blocks(ctx.L, bufs, src, moms, what, [1])
+    assert per_t_error(out, what, 2, moms, ref, [1]).max() < 1e-6
+    ctx.close()
+
+
+@pytest.mark.parametrize("Lx,ran", [(3, "project_split_tc"), (4, "project_axis_x")])
+def test_split_udsc_dispatch(Lx, ran):
+    ctx = p2.Context((Lx, 60, 60, 10))
+    bufs = device_props(ctx, [(69, 0), (69, 1)], t0=0)
+    moms = p2.mom_list(2)
+    got = []
+    for mode in (p2.P2_PLAIN_FP64, SPLIT):
+        out = torch.zeros(28 * len(moms), dtype=torch.complex128, device="cuda")
+        ctx.profile()
+        ctx.contract_udsc([ctx.prop(b.data_ptr()) for b in bufs],
+                          ctx.udsc_request((0, 0, 0, 0), 1, out.data_ptr(), moms=moms, mode=mode, prop_u=0, prop_d=1))
+        ctx.sync()
+        got.append(out.cpu().numpy().reshape(28, len(moms)))
+    assert ran in ctx.profile_read()
+    # random signs: the values are about 1e-2 of sum_x |c|, which the form's 1e-6 is relative to
+    assert np.abs(got[1] - got[0]).max() < 1e-4 * np.abs(got[0]).max()
+    ctx.close()
