@@ -30,6 +30,14 @@ def device_props(ctx, seeds, t0, decay=0.5, precision=p2.P2_FP64, t_first=0, nt=
     return out
 
 
+def long_list(q2max):
+    """|n|^2 <= q2max and (1..5, 0, 0): eleven phase rows on an x axis of eleven
+    or more sites, so that the list is projected directly (split form: on the
+    tensor cores) and not axis by axis."""
+    extra = [[n, 0, 0] for n in range(1, 6) if n * n > q2max]
+    return np.concatenate([p2.mom_list(q2max), np.array(extra, dtype=np.int32).reshape(-1, 3)])
+
+
 def run(ctx, bufs, source, totalT, what, q2max=None, moms=None, mode=p2.P2_PLAIN_FP64, precision=p2.P2_FP64,
         t_first=0, nt=None, pu=0, pd=1, host_props=False, host_out=False):
     nt = ctx.Ll[3] if nt is None else nt

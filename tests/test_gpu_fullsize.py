@@ -20,7 +20,7 @@ import torch
 
 from plegma_b200 import lib as p2
 
-import p2test  # noqa: F401  (puts the oracle on the path)
+import p2test  # (puts the oracle on the path)
 import oracle_py as orc  # noqa: E402
 
 pytestmark = pytest.mark.gpu
@@ -176,10 +176,12 @@ def test_split_error_large_configuration_64():
     assert max(e for _, e in errs) < TOL_SPLIT, errs
 
 
-def test_split_error_mean_dominated_sums():
+@pytest.mark.parametrize("long", [False, True])
+def test_split_error_mean_dominated_sums(long):
     """Correlators whose site values all share a sign (the pion Tr[S S^+] >= 0
     of u = d, and a generic field of mean 1) are the worst case for the
-    tensor-core accumulation, whose rounding loses ~2^-27 of the running sum
+    accumulation in FP32: that of the sums over x and y, and with the long list
+    that of the tensor cores, whose rounding loses ~2^-27 of the running sum
     per step with a consistent sign: a whole slice summed in one TMEM tile
     was 3e-5 off at 48^3.  The accumulator tiles are added into an FP32 sum
     every few k-steps, so the error stays well inside the bound at any
@@ -189,7 +191,8 @@ def test_split_error_mean_dominated_sums():
     ctx = p2.Context(L)
     # generic transform of a mean-1 field, all 16 slices in one launch (long site ranges per CTA)
     rng = np.random.default_rng(11)
-    moms = p2.mom_list(2)
+    ctx.profile()
+    moms = p2test.long_list(2) if long else p2.mom_list(2)
     dof, nt = 8, L[3]
     f = 1.0 + 0.1 * (rng.standard_normal((dof, nt, V3)) + 1j * rng.standard_normal((dof, nt, V3)))
     fd = torch.from_numpy(f.reshape(-1)).cuda()
@@ -210,7 +213,7 @@ def test_split_error_mean_dominated_sums():
     (u,) = [torch.empty(144 * V3 * L[3], dtype=torch.complex128, device="cuda")]
     ctx.synth(u.data_ptr(), True, p2.P2_FP64, 1107, 0, src[3], 0.5)
     what = p2.NUCLEON_CG5 | p2.MESON_G16
-    mq = p2.mom_list(9)
+    mq = p2test.long_list(9) if long else p2.mom_list(9)
     _, total = p2.block_info(what, L[3], len(mq))
     o = torch.zeros(total, dtype=torch.complex128, device="cuda")
     props = [ctx.prop(u.data_ptr()), ctx.prop(u.data_ptr())]
@@ -222,6 +225,8 @@ def test_split_error_mean_dominated_sums():
         t = (src[3] + tau) % L[3]
         us = _slice(u, V3, t)
         perr.append(_slice_error(L, res, us, us, src, mq, what, tau, t))
+    names = ctx.profile_read()
+    assert ("project_split_tc" in names) == long and ("field_to_f32" in names) == long
     ctx.close()
     print("mean-dominated: field err", ferr, "pion (u = d) err(t)", perr)
     assert ferr < TOL_SPLIT, ferr

@@ -10,7 +10,7 @@ import torch
 
 from plegma_b200 import lib as p2
 
-from p2test import device_props, oracle_blocks, per_t_error
+from p2test import device_props, long_list, oracle_blocks, per_t_error
 
 pytestmark = pytest.mark.gpu
 
@@ -19,9 +19,9 @@ WHAT = NUC | p2.DELTA_ISO12 | p2.DELTA_ISO32 | p2.MESON_G16
 TOL = {p2.P2_PLAIN_FP64: 1e-12, p2.P2_SPLIT_FP16: 1e-6}
 
 
-def _setup(ctx, mode, nsrc=4, seed=40, q2max=2, what=WHAT):
+def _setup(ctx, mode, nsrc=4, seed=40, what=WHAT, long=False):
     rng = np.random.default_rng(seed)
-    moms = p2.mom_list(q2max)
+    moms = long_list(2) if long else p2.mom_list(2)
     srcs, bufs, props, outs, reqs = [], [], [], [], []
     for i in range(nsrc):
         src = tuple(int(rng.integers(0, ctx.L[d])) for d in range(4))
@@ -37,12 +37,20 @@ def _setup(ctx, mode, nsrc=4, seed=40, q2max=2, what=WHAT):
     return srcs, bufs, props, outs, reqs, moms
 
 
+#: the projection kernel of a list that is not projected axis by axis
+DIRECT = {p2.P2_PLAIN_FP64: "project_fp64", p2.P2_SPLIT_FP16: "project_split_tc"}
+
+
 @pytest.mark.parametrize("mode", [p2.P2_PLAIN_FP64, p2.P2_SPLIT_FP16])
-def test_graph_replay_matches_eager_and_follows_refills(mode):
-    ctx = p2.Context((5, 4, 6, 10))
-    srcs, bufs, props, outs, reqs, moms = _setup(ctx, mode)
+@pytest.mark.parametrize("L,long", [((5, 4, 6, 10), False), ((11, 4, 6, 10), True)])
+def test_graph_replay_matches_eager_and_follows_refills(L, long, mode):
+    ctx = p2.Context(L)
+    srcs, bufs, props, outs, reqs, moms = _setup(ctx, mode, long=long)
+    ctx.profile()
     ctx.contract_project(props, reqs)
     ctx.sync()
+    assert (DIRECT[mode] in ctx.profile_read()) == long
+    ctx.profile(False)
     eager = [o.clone() for o in outs]
     for o in outs:
         o.zero_()
@@ -105,11 +113,12 @@ def test_graph_rejects_two_batches():
 
 
 @pytest.mark.parametrize("mode", [p2.P2_PLAIN_FP64, p2.P2_SPLIT_FP16])
-def test_tuner_caches_choices_and_stays_accurate(tmp_path, mode):
+@pytest.mark.parametrize("L,long", [((6, 6, 4, 8), False), ((12, 6, 4, 8), True)])  # y stage; direct projections
+def test_tuner_caches_choices_and_stays_accurate(tmp_path, L, long, mode):
     path = str(tmp_path / "tune.tsv")
-    ctx = p2.Context((6, 6, 4, 8))
+    ctx = p2.Context(L)
     ctx.tune(True, path)
-    srcs, bufs, props, outs, reqs, moms = _setup(ctx, mode, nsrc=2, seed=90, what=NUC | p2.MESON_G16)
+    srcs, bufs, props, outs, reqs, moms = _setup(ctx, mode, nsrc=2, seed=90, what=NUC | p2.MESON_G16, long=long)
     ctx.contract_project(props, reqs)
     ctx.sync()
     n = ctx.tune_count()
@@ -118,6 +127,7 @@ def test_tuner_caches_choices_and_stays_accurate(tmp_path, mode):
     assert len(lines) == n
     kernel = "project_split" if mode == p2.P2_SPLIT_FP16 else "project_fp64"
     assert all(line.startswith(kernel) and len(line.split("\t")) == 3 for line in lines)
+    assert all((" axes " in line) != long for line in lines)
     for (src, W), b, o in zip(srcs, bufs, outs):
         taus = list(range(W))
         ref = oracle_blocks(ctx.L, b, src, moms, NUC | p2.MESON_G16, taus)
@@ -126,10 +136,10 @@ def test_tuner_caches_choices_and_stays_accurate(tmp_path, mode):
     first = [o.clone() for o in outs]
     ctx.close()
     # a new context reads the file: same choices, same bits, no new entries
-    ctx2 = p2.Context((6, 6, 4, 8))
+    ctx2 = p2.Context(L)
     ctx2.tune(True, path)
     assert ctx2.tune_count() == n
-    srcs2, bufs2, props2, outs2, reqs2, _ = _setup(ctx2, mode, nsrc=2, seed=90, what=NUC | p2.MESON_G16)
+    srcs2, bufs2, props2, outs2, reqs2, _ = _setup(ctx2, mode, nsrc=2, seed=90, what=NUC | p2.MESON_G16, long=long)
     ctx2.contract_project(props2, reqs2)
     ctx2.sync()
     assert ctx2.tune_count() == n

@@ -7,7 +7,7 @@ import torch
 
 from plegma_b200 import lib as p2
 
-from p2test import device_props, oracle_blocks, per_t_error, run
+from p2test import device_props, long_list, oracle_blocks, per_t_error, run
 
 pytestmark = pytest.mark.gpu
 
@@ -198,21 +198,23 @@ def test_second_nucleon_interpolator(what, mode):
 
 
 @pytest.mark.parametrize("decay", [0.0, 40.0])
-def test_ft_apply_split_matches_oracle(decay):
-    """p2_ft_apply_split (tensor-core projection): error per (t, component,
-    momentum) <= 1e-6 of sum_x |f(x, t)| of the component, both signs, host
+@pytest.mark.parametrize("L,long", [((4, 6, 5, 3), False), ((11, 6, 5, 3), True)])
+def test_ft_apply_split_matches_oracle(L, long, decay):
+    """p2_ft_apply_split (axis by axis in FP64, or on the tensor cores for the
+    long list): error per (t, component, momentum) <= 1e-6 of sum_x |f(x, t)| of the component, both signs, host
     and device output; with decay 40 the slices span 1e-35 .. 1, which the
     per-slice power-of-two scale keeps inside FP32's range.  The known answer
     of the reference's FT test (plegma/FT.cpp:18-34): a unit field gives
     V3 at p = 0 and 0 elsewhere."""
     import oracle_py as orc
-    ctx = p2.Context((4, 6, 5, 3))
+    ctx = p2.Context(L)
     dof, nt = 21, 3
+    ctx.profile()
     rng = np.random.default_rng(6)
     f = rng.standard_normal((dof, ctx.V3 * nt)) + 1j * rng.standard_normal((dof, ctx.V3 * nt))
     f *= np.exp(-decay * np.repeat(np.arange(nt), ctx.V3))[None, :]
     fd = torch.from_numpy(f.reshape(-1)).cuda()
-    moms = p2.mom_list(5)
+    moms = long_list(5) if long else p2.mom_list(5)
     asum = np.abs(f).reshape(dof, nt, ctx.V3).sum(axis=2).T  # [t][dof]
     for sign in (-1, 1):
         ref = orc.ft(ctx.L, f, dof, nt, moms, sign)
@@ -229,17 +231,19 @@ def test_ft_apply_split_matches_oracle(decay):
     ctx.ft_apply(one.data_ptr(), 1, nt, moms, -1, out.ctypes.data, p2.P2_HOST, mode=p2.P2_SPLIT_FP16)
     out = out.reshape(nt, len(moms))
     assert np.abs(out[:, 0] - ctx.V3).max() < 1e-6 * ctx.V3 and np.abs(out[:, 1:]).max() < 1e-6 * ctx.V3
+    assert ("project_split_tc" in ctx.profile_read()) == long
     ctx.close()
 
 
-def test_ft_apply_split_odd_volume():
+@pytest.mark.parametrize("L,long", [((3, 5, 3, 2), False), ((11, 5, 3, 2), True)])  # V3 = 45, 165
+def test_ft_apply_split_odd_volume(L, long):
     import oracle_py as orc
-    ctx = p2.Context((3, 5, 3, 2))  # V3 = 45
+    ctx = p2.Context(L)
     dof, nt = 5, 2
     rng = np.random.default_rng(8)
     f = rng.standard_normal((dof, ctx.V3 * nt)) + 1j * rng.standard_normal((dof, ctx.V3 * nt))
     fd = torch.from_numpy(f.reshape(-1)).cuda()
-    moms = p2.mom_list(3)
+    moms = long_list(3) if long else p2.mom_list(3)
     ref = orc.ft(ctx.L, f, dof, nt, moms, -1)
     out = np.zeros(nt * dof * len(moms), dtype=np.complex128)
     ctx.ft_apply(fd.data_ptr(), dof, nt, moms, -1, out.ctypes.data, p2.P2_HOST, mode=p2.P2_SPLIT_FP16)

@@ -1,13 +1,14 @@
-"""Parity of the split-FP16 form (FP32 contraction, hi+lo FP16 tensor-core
-projection with FP32 accumulation, FP64 cross-block sums) with the FP64
-oracle.  Tolerance: err(t) <= 1e-6 relative to sum_x |c_k(x,t)|, per time
-slice, over all momenta and components."""
+"""Parity of the split form (FP32 contraction, projection axis by axis or, for
+long momentum lists, on the tensor cores with hi+lo FP16 operands, FP32
+accumulation and FP64 cross-block sums) with the FP64 oracle.  Tolerance:
+err(t) <= 1e-6 relative to sum_x |c_k(x,t)|, per time slice, over all momenta
+and components."""
 import numpy as np
 import pytest
 
 from plegma_b200 import lib as p2
 
-from p2test import device_props, oracle_blocks, per_t_error, run
+from p2test import device_props, long_list, oracle_blocks, per_t_error, run
 
 pytestmark = pytest.mark.gpu
 
@@ -91,13 +92,16 @@ def test_split_matches_plain_to_tolerance():
     ctx.close()
 
 
-def test_split_delta_batched_set():
-    """Nucleon + Delta (both isospins, k = 1..3) + 16x16 mesons, K = 480:
-    four N-tiles of the tensor-core projection."""
-    ctx = p2.Context((8, 6, 4, 8))
+@pytest.mark.parametrize("L,long", [((8, 6, 4, 8), False), ((11, 6, 4, 8), True)])
+def test_split_delta_batched_set(L, long):
+    """Nucleon + Delta (both isospins, k = 1..3) + 16x16 mesons, K = 480: six
+    N-tiles of the tensor-core projection with the long list."""
+    ctx = p2.Context(L)
     bufs = device_props(ctx, [(1004, 0), (1004, 1)], t0=6)
     what = NUC | p2.DELTA_ISO12 | p2.DELTA_ISO32 | p2.MESON_G16
-    out, moms = run(ctx, bufs, (3, 1, 2, 6), 7, what, q2max=5, mode=SPLIT)
+    ctx.profile()
+    out, moms = run(ctx, bufs, (3, 1, 2, 6), 7, what, moms=long_list(5) if long else p2.mom_list(5), mode=SPLIT)
+    assert ("project_split_tc" in ctx.profile_read()) == long
     taus = list(range(7))
     ref = oracle_blocks(ctx.L, bufs, (3, 1, 2, 6), moms, what, taus)
     err = per_t_error(out, what, 7, moms, ref, taus)
@@ -168,18 +172,23 @@ def test_every_contraction_block_in_one_request(mode):
     ctx.close()
 
 
-@pytest.mark.parametrize("q2max", [0, 16])
-def test_split_momentum_list_extremes(q2max):
-    """One momentum (a single cos row) and |n|^2 <= 16 (257 momenta: 257 phase
-    rows in three 128-row tiles, the batched 64^3 x 128 configuration's
-    list) against the oracle."""
-    ctx = p2.Context((6, 5, 4, 4))
+@pytest.mark.parametrize("L,q2max,n", [
+    ((6, 5, 4, 4), 0, 1), ((6, 5, 4, 4), 16, 257),
+    ((12, 5, 4, 4), 25, 515),  # eleven rows along x: 515 phase rows in five 128-row tiles of the tensor cores
+])
+def test_split_momentum_list_extremes(L, q2max, n):
+    """One momentum (a single cos row), |n|^2 <= 16 (the batched 64^3 x 128
+    configuration's list, axis by axis) and |n|^2 <= 25 on a long x axis
+    (tensor cores) against the oracle."""
+    ctx = p2.Context(L)
     src = (3, 1, 2, 1)
     bufs = device_props(ctx, [(61, 0), (61, 1)], t0=src[3])
     what = p2.NUCLEON_CG5 | p2.MESON_G16
     moms = p2.mom_list(q2max)
-    assert len(moms) == (1 if q2max == 0 else 257)
+    assert len(moms) == n
+    ctx.profile()
     out, _ = run(ctx, bufs, src, 4, what, moms=moms, mode=p2.P2_SPLIT_FP16)
+    assert ("project_split_tc" in ctx.profile_read()) == (q2max == 25)
     taus = list(range(4))
     ref = oracle_blocks(ctx.L, bufs, src, moms, what, taus)
     err = per_t_error(out, what, 4, moms, ref, taus)

@@ -10,7 +10,7 @@ import torch
 from plegma_b200 import lib as p2
 from plegma_b200 import udsc
 
-from p2test import device_props
+from p2test import device_props, long_list
 
 import oracle_py as orc
 
@@ -124,8 +124,7 @@ SPLIT_TOL = 1e-6
 
 
 def test_split_light_baryons_u_d():
-    """Split form (FP32 contraction, hi+lo FP16 tensor-core projection): u and
-    d, 28 datasets, window wrapping through t = 0."""
+    """Split form (FP32 contraction): u and d, 28 datasets, window wrapping through t = 0."""
     ctx = p2.Context((4, 4, 2, 6))
     src = (1, 2, 0, 4)
     u, d = device_props(ctx, [(73, 0), (73, 1)], t0=src[3])
@@ -200,4 +199,29 @@ def test_odd_spatial_volume(mode):
     ctx.sync()
     err = _check(ctx, {"u": u, "d": d}, src, W, moms, out.cpu().numpy(), req)
     assert err < (TOL if mode == p2.P2_PLAIN_FP64 else SPLIT_TOL), err
+    ctx.close()
+
+
+@pytest.mark.parametrize("mode,kernel,tol", [(p2.P2_PLAIN_FP64, "project_fp64", TOL),
+                                             (p2.P2_SPLIT_FP16, "project_split_tc", SPLIT_TOL)])
+def test_list_that_is_projected_directly(mode, kernel, tol):
+    """Eleven phase rows along x: the direct FP64 sum, the tensor cores; u, d and
+    s (one to three flavours per product), two chunks of the largest group."""
+    ctx = p2.Context((11, 4, 3, 5))
+    src = (7, 2, 1, 3)
+    bufs = device_props(ctx, [(78, 0), (78, 1), (79, 0)], t0=src[3])
+    moms = long_list(3)
+    W = 5
+    req = ctx.udsc_request(src, W, 0, moms=moms, prop_u=0, prop_d=1, prop_s=2, mode=mode)
+    n = len(p2.udsc_datasets(req))
+    ctx.set_workspace(4 * 32 * ctx.V3 * 8)
+    out = torch.zeros(n * W * len(moms), dtype=torch.complex128, device="cuda")
+    req.out = out.data_ptr()
+    ctx.profile()
+    ctx.contract_udsc([ctx.prop(b.data_ptr()) for b in bufs], req)
+    ctx.sync()
+    names = ctx.profile_read()
+    assert kernel in names and "project_axis_y" not in names
+    err = _check(ctx, dict(zip("uds", bufs)), src, W, moms, out.cpu().numpy(), req)
+    assert err < tol, err
     ctx.close()
