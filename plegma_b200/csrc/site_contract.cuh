@@ -263,27 +263,6 @@ __device__ __forceinline__ void dq_fin_f32(const f32x2 px[9], const f32x2 py[9],
   }
 }
 
-// q = s1 P^{XY}_{(nu1, lam1)} + s2 P^{XY}_{(nu2, lam2)} (the Delta's shared
-// diagonal pairs), paired FMAs on the FP32 tile
-template <int nu1, int lam1, int s1, int nu2, int lam2, int s2, typename Row>
-__device__ __forceinline__ void diquark_pair_ct(const Row& row, int X, int Y, int xp, int yp,
-                                                Cx<typename Row::R> q[9]) {
-  typedef typename Row::R R;
-  if constexpr (sizeof(R) == 4) {
-    f32x2 px[9], py[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) px[i] = py[i] = f2pack(0.f, 0.f);
-    dq_acc_f32<nu1, lam1, s1>(row, X, Y, xp, yp, px, py);
-    dq_acc_f32<nu2, lam2, s2>(row, X, Y, xp, yp, px, py);
-    dq_fin_f32(px, py, q);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 9; i++) q[i] = czero<R>();
-    diquark_acc(row, X, Y, nu1, lam1, R(s1), xp, yp, q);
-    diquark_acc(row, X, Y, nu2, lam2, R(s2), xp, yp, q);
-  }
-}
-
 template <int S, typename Row>
 __device__ __forceinline__ void diquark_G_ct(const Row& row, int X, int Y, int xp, int yp, Cx<typename Row::R> q[9]) {
   typedef typename Row::R R;
@@ -387,88 +366,51 @@ __device__ __forceinline__ void diquark_transpose(Cx<R> q[9], int l, unsigned ma
   for (int i = 0; i < 9; i++) q[i] = cscale(shfl_idx16(q[i], src, mask), sign);
 }
 
-// Slot terms of one group of Wick terms sharing G and the third line Z (block
-// offset in the site row); returns the lane's share of T[mu = l >> 2][mu' = l & 3].
-//   slot 2: T[mu][mu'] = sum_{x'} f2 sum_ce G(x', mu')[c][e] Z[mu][z2][c][e]
-//   slot 1: T[mu][mu'] = sum_{y'} f1 sum_ce G(mu', y')[c][e] Z[mu][z1][c][e]
-template <bool S1, bool S2, typename Row>
-__device__ __forceinline__ Cx<typename Row::R> diquark_slots(const Cx<typename Row::R> g[9], const Row& row, int Z,
-                                                             const DiquarkLane& dl, int l, unsigned mask, int c1A,
-                                                             int c1B, int c2A, int c2B) {
+// Slot-1 terms of one group of Wick terms sharing G and the third line Z (block
+// offset in the site row), with the Wick coefficient -1; returns the lane's
+// share of T[mu = l >> 2][mu' = l & 3]:
+//   T[mu][mu'] = sum_{y'} sA1 sum_ce G(mu', y')[c][e] Z[mu][z1][c][e]
+template <typename Row>
+__device__ __forceinline__ Cx<typename Row::R> diquark_slot1(const Cx<typename Row::R> g[9], const Row& row, int Z,
+                                                             const DiquarkLane& dl, int l, unsigned mask) {
   typedef typename Row::R R;
+  const R f1 = R(dl.sA1);
   Cx<R> r = czero<R>();
-  // the four m of a slot reduced over four lanes as a reduce-scatter: the lane
-  // of bit b1 = bit hb of the lane index keeps m in {2 b1, 2 b1 + 1}, then the
-  // lane of bit b0 = bit lb keeps m = 2 b1 + b0
-  auto scatter = [&](Cx<R> (&P)[4], int hb, int lb) {
-    const bool b1 = (l >> hb) & 1, b0 = (l >> lb) & 1;
-    const Cx<R> s0 = b1 ? P[0] : P[2], s1 = b1 ? P[1] : P[3];
-    Cx<R> k0 = b1 ? P[2] : P[0], k1 = b1 ? P[3] : P[1];
-    k0 = k0 + shfl_xor16(s0, 1 << hb, mask);
-    k1 = k1 + shfl_xor16(s1, 1 << hb, mask);
-    const Cx<R> s = b0 ? k0 : k1;
-    const Cx<R> k = b0 ? k1 : k0;
-    return k + shfl_xor16(s, 1 << lb, mask);
-  };
   if constexpr (sizeof(R) == 8) {
     // FP64: one m at a time (four m of FP64 sums held at once spill)
-    const int mu = l >> 2, mup = l & 3;
-    if (S2) {
-      const R f2 = R(c2A * dl.sA2 - c2B * dl.sB2);
+    const int mu = l >> 2, src = (l & 3) << 2;
 #pragma unroll 1
-      for (int m = 0; m < 4; m++) {
-        Cx<R> z[9];
-        row.load9(Z + m * 4 + dl.z2, z);
-        Cx<R> p2 = cscale(cdot9(g, z), f2);
-        p2 = p2 + shfl_xor16(p2, 4, mask);
-        p2 = p2 + shfl_xor16(p2, 8, mask);
-        if (m == mu) r = r + p2;
-      }
-    }
-    if (S1) {
-      const R f1 = R(-(c1A * dl.sA1 - c1B * dl.sB1));
-      const int src = mup << 2;
-#pragma unroll 1
-      for (int m = 0; m < 4; m++) {
-        Cx<R> z[9];
-        row.load9(Z + m * 4 + dl.z1, z);
-        Cx<R> p1 = cscale(cdot9(g, z), f1);
-        p1 = p1 + shfl_xor16(p1, 1, mask);
-        p1 = p1 + shfl_xor16(p1, 2, mask);
-        const Cx<R> v = shfl_idx16(p1, src, mask);
-        if (m == mu) r = r + v;
-      }
-    }
-    return r;
-  }
-  if (S2) {
-    // slot 2 (sum over x'): lane (x', y' = mu') forms P[m] for T[m][mu'];
-    // after the scatter over x' (lane bits 3, 2) lane (x', mu') holds T[x'][mu']
-    const R f2 = R(c2A * dl.sA2 - c2B * dl.sB2);
-    Cx<R> P[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-      Cx<R> z[9];
-      row.load9(Z + m * 4 + dl.z2, z);
-      P[m] = cscale(cdot9(g, z), f2);
-    }
-    r = r + scatter(P, 3, 2);
-  }
-  if (S1) {
-    // slot 1 (sum over y'): lane (x' = mu', y') forms P[m] for T[m][mu'];
-    // after the scatter over y' (lane bits 1, 0) lane (mu', y') holds
-    // T[y'][mu'], which lane (mu, mu') takes from the transposed lane
-    const R f1 = R(-(c1A * dl.sA1 - c1B * dl.sB1));
-    Cx<R> P[4];
-#pragma unroll
     for (int m = 0; m < 4; m++) {
       Cx<R> z[9];
       row.load9(Z + m * 4 + dl.z1, z);
-      P[m] = cscale(cdot9(g, z), f1);
+      Cx<R> p1 = cscale(cdot9(g, z), f1);
+      p1 = p1 + shfl_xor16(p1, 1, mask);
+      p1 = p1 + shfl_xor16(p1, 2, mask);
+      const Cx<R> v = shfl_idx16(p1, src, mask);
+      if (m == mu) r = r + v;
     }
-    r = r + shfl_idx16(scatter(P, 1, 0), ((l & 3) << 2) | (l >> 2), mask);
+    return r;
   }
-  return r;
+  // lane (x' = mu', y') forms P[m] for T[m][mu']; the four m are reduced over
+  // the four lanes y' (lane bits 1, 0) as a reduce-scatter: the lane of bit b1
+  // keeps m in {2 b1, 2 b1 + 1}, then that of bit b0 m = 2 b1 + b0.  Lane
+  // (mu', y') then holds T[y'][mu'], which lane (mu, mu') takes from the
+  // transposed lane.
+  Cx<R> P[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    Cx<R> z[9];
+    row.load9(Z + m * 4 + dl.z1, z);
+    P[m] = cscale(cdot9(g, z), f1);
+  }
+  const bool b1 = (l >> 1) & 1, b0 = l & 1;
+  const Cx<R> s0 = b1 ? P[0] : P[2], s1 = b1 ? P[1] : P[3];
+  Cx<R> k0 = b1 ? P[2] : P[0], k1 = b1 ? P[3] : P[1];
+  k0 = k0 + shfl_xor16(s0, 2, mask);
+  k1 = k1 + shfl_xor16(s1, 2, mask);
+  const Cx<R> s = b0 ? k0 : k1;
+  const Cx<R> k = b0 ? k1 : k0;
+  return r + shfl_idx16(k + shfl_xor16(s, 1, mask), ((l & 3) << 2) | (l >> 2), mask);
 }
 
 // Slot-1 terms of the Wick-transposed diquark G^{YX}(x', y') = sign G^{XY}(y', x')
@@ -539,13 +481,12 @@ __device__ __forceinline__ Cx<typename Row::R> diquark_typea(const Cx<typename R
   return cdot9(D, z);
 }
 
-// All Wick terms of one group: slot terms with the Wick coefficients
-// (c1A, c1B, c2A, c2B) plus the type-a terms of the sum D.
-template <bool S1, bool S2, typename Row>
+// All Wick terms of one group: slot terms plus the type-a terms of the sum D.
+template <typename Row>
 __device__ __forceinline__ Cx<typename Row::R> diquark_eval(const Cx<typename Row::R> g[9], const Row& row, int Z,
-                                                            const DiquarkLane& dl, int l, unsigned mask, int c1A,
-                                                            int c1B, int c2A, int c2B, const Cx<typename Row::R> D[9]) {
-  return diquark_slots<S1, S2>(g, row, Z, dl, l, mask, c1A, c1B, c2A, c2B) + diquark_typea(D, row, Z, l);
+                                                            const DiquarkLane& dl, int l, unsigned mask,
+                                                            const Cx<typename Row::R> D[9]) {
+  return diquark_slot1(g, row, Z, dl, l, mask) + diquark_typea(D, row, Z, l);
 }
 
 // Nucleon C g5, both datasets: out[0] = proton (u u d), out[1] = neutron (d d u),
@@ -559,7 +500,7 @@ __device__ __forceinline__ void nucleon_site(const Row& row, const LaneTables& l
   const DiquarkLane dl = unpack_diquark_lane(lt.nuc);
   constexpr int l0 = typea_lane(kNucLane);
   diquark_D(g, R(dl.sN), mask, l0, D);  // cN = 1, cL = 0
-  out[0] = diquark_eval<true, false>(g, row, kU, dl, l, mask, -1, 0, 0, 0, D);
+  out[0] = diquark_eval(g, row, kU, dl, l, mask, D);
   // G^{du}(x', y') = -G^{ud}(y', x'); its type-a sum is (-1)(tau = -1) D
   out[1] = diquark_slot1_transposed(g, row, kD, unpack_diquark_lane(lt.nucT), l, mask, -1, 0, R(-1)) +
            diquark_typea(D, row, kD, l);
@@ -910,9 +851,9 @@ __device__ __forceinline__ void light_nucleon_site(const Row& row, const LaneTab
     const DiquarkLane dl = unpack_diquark_lane(lt.light[0]);
     constexpr int l0 = typea_lane(kLightLane[0]);
     diquark_D(g, R(dl.sN), mask, l0, D);
-    const Cx<R> p = diquark_eval<true, false>(g, row, kU, dl, l, mask, -1, 0, 0, 0, D);
+    const Cx<R> p = diquark_eval(g, row, kU, dl, l, mask, D);
     diquark_transpose<R>(g, l, mask, R(-1));
-    const Cx<R> n = diquark_eval<true, false>(g, row, kD, dl, l, mask, -1, 0, 0, 0, D);
+    const Cx<R> n = diquark_eval(g, row, kD, dl, l, mask, D);
     out(0, 0, cscale(shfl_xor16(p, 2, mask), s_nr));
     out(0, 1, cscale(shfl_xor16(n, 2, mask), s_nr));
   }
@@ -926,25 +867,25 @@ __device__ __forceinline__ void light_nucleon_site(const Row& row, const LaneTab
       Cx<R> D[9];
       if (rton) {
         diquark_D(g, R(drn.sN), mask, l0rn, D);
-        prn = diquark_eval<true, false>(g, row, kU, drn, l, mask, -1, 0, 0, 0, D);
+        prn = diquark_eval(g, row, kU, drn, l, mask, D);
       }
       if (rtor) {
         diquark_D(g, R(drr.sN), mask, l0rr, D);
-        prr = diquark_eval<true, false>(g, row, kU, drr, l, mask, -1, 0, 0, 0, D);
+        prr = diquark_eval(g, row, kU, drr, l, mask, D);
       }
     }
     diquark_transpose<R>(g, l, mask, R(kCT[0]));
     if (rton) {
       Cx<R> D[9];
       diquark_D(g, R(drn.sN), mask, l0rn, D);
-      const Cx<R> n = diquark_eval<true, false>(g, row, kD, drn, l, mask, -1, 0, 0, 0, D);
+      const Cx<R> n = diquark_eval(g, row, kD, drn, l, mask, D);
       out(1, 0, cscale(shfl_xor16(prn, 8, mask), s_rn));
       out(1, 1, cscale(shfl_xor16(n, 8, mask), s_rn));
     }
     if (rtor) {
       Cx<R> D[9];
       diquark_D(g, R(drr.sN), mask, l0rr, D);
-      const Cx<R> n = diquark_eval<true, false>(g, row, kD, drr, l, mask, -1, 0, 0, 0, D);
+      const Cx<R> n = diquark_eval(g, row, kD, drr, l, mask, D);
       out(2, 0, cscale(shfl_xor16(prr, 10, mask), s_rr));
       out(2, 1, cscale(shfl_xor16(n, 10, mask), s_rr));
     }

@@ -388,32 +388,17 @@ def encode_programs(prods):
 def emit_header(path: str) -> bool:
     """C header with the tables (generated at build time); True if the file changed."""
     prods = products()
-    names, ds_begin, ent_begin, idx, val, pflav = [], [0], [0], [], [], []
+    names, ds_begin, pflav = [], [0], []
     for key, dss in prods:
         pflav.append(key)
-        for name, tups, ws in dss:
-            names.append(name)
-            for t, w in zip(tups, ws):
-                idx.append(t)
-                val.append((float(np.real(w)), float(np.imag(w))))
-            ent_begin.append(len(idx))
+        names += [name for name, _, _ in dss]
         ds_begin.append(len(names))
     L = ["// Generated by plegma_b200/udsc.py: table-driven baryon spin tables.", "#pragma once", "",
          f"constexpr int kUdscProducts = {len(prods)};",
          f"constexpr int kUdscDatasets = {len(names)};",
-         f"constexpr int kUdscEntries = {len(idx)};",
          "static const char kUdscProduct[kUdscProducts][4] = {" + ", ".join(f'"{k}"' for k in pflav) + "};",
          "static const int kUdscDsBegin[kUdscProducts + 1] = {" + ", ".join(map(str, ds_begin)) + "};",
-         "static const char* const kUdscName[kUdscDatasets] = {" + ", ".join(f'"{n}"' for n in names) + "};",
-         "static const int kUdscEntBegin[kUdscDatasets + 1] = {" + ", ".join(map(str, ent_begin)) + "};",
-         "static const signed char kUdscIdx[kUdscEntries][6] = {"]
-    for i in range(0, len(idx), 12):
-        L.append("  " + " ".join("{%d,%d,%d,%d,%d,%d}," % t for t in idx[i:i + 12]))
-    L.append("};")
-    L.append("static const float kUdscVal[kUdscEntries][2] = {")
-    for i in range(0, len(val), 8):
-        L.append("  " + " ".join("{%.9ef,%.9ef}," % v for v in val[i:i + 8]))
-    L.append("};")
+         "static const char* const kUdscName[kUdscDatasets] = {" + ", ".join(f'"{n}"' for n in names) + "};"]
     code, values, which, programs, cases = encode_programs(prods)
     L += ["", f"constexpr int kUdscWarps = {PROGRAM_WARPS};",
           "static const int kUdscProgram[kUdscProducts] = {" + ", ".join(map(str, which)) + "};",
