@@ -51,12 +51,12 @@ typedef enum { P2_FP64 = 0, P2_FP32 = 1 } p2_precision;
 /* Arithmetic of a request.
  * P2_PLAIN_FP64: FP64 site contraction, FP64 projection.
  * P2_SPLIT_FP16: FP32 site contraction with power-of-two scaling per time
- *   slice; FP32 projection sums within a row and a column of sites, FP64
- *   beyond and normalisation.
+ *   slice; projection sums over x and y in FP32 by groups of a few sites, over
+ *   z in FP64; error <= 1e-6 of sum_x |c_k(x, t)|.
  * The projection runs one axis at a time when the momenta need at most nine
  * cosine and sine rows per axis (|n_d| <= 4); other lists take a direct FP64
  * phase sum, or, split form, the tensor cores with hi+lo FP16 products and FP32
- * accumulation. */
+ * accumulation, and so do, split form, large lattices with a short x axis. */
 typedef enum { P2_PLAIN_FP64 = 0, P2_SPLIT_FP16 = 1 } p2_mode;
 
 typedef enum { P2_DEVICE = 0, P2_HOST = 1 } p2_location;
@@ -210,10 +210,11 @@ p2_status p2_ft_apply(p2_ctx* ctx, const double* field, int dof, int nt, const i
 
 /* The same transform; momentum lists that need more than nine phase rows on an
  * axis run on the tensor cores (the split projection of the contractions), the
- * others in FP64 one axis at a time.  On the tensor cores each time slice of the field is scaled by 2^-e (e the binary
- * exponent of its largest entry, exact), converted to FP32 and projected with
- * hi+lo FP16 operands and FP32 accumulation; per (t, component, momentum) the
- * error is <= 1e-6 of sum_x |field(x, t)| of that component. */
+ * others in FP64 one axis at a time.  On the tensor cores each time slice of
+ * the field is scaled by 2^-e (e the binary exponent of its largest entry,
+ * exact), converted to FP32 and projected with hi+lo FP16 operands and FP32
+ * accumulation; per (t, component, momentum) the error is <= 1e-6 of
+ * sum_x |field(x, t)| of that component. */
 p2_status p2_ft_apply_split(p2_ctx* ctx, const double* field, int dof, int nt, const int* moms, int nmom, int sign,
                             double* out, int out_location);
 
@@ -356,8 +357,7 @@ int p2_profile_read(p2_ctx* ctx, p2_kernel_time* out, int max, int reset);
 
 /* Test hook for the device-side failure path: the next tensor-core
  * projection launched on this context (the next split request or
- * p2_ft_apply_split takes it, whatever its momenta)
- * withholds its converters' operand-ready signals and gives every mbarrier
+ * p2_ft_apply_split takes it, whatever its momenta) withholds its converters' operand-ready signals and gives every mbarrier
  * wait a short limit, so its waits run out; the kernel records the timeout,
  * waits for its own bulk copies, frees its TMEM and returns, and the next
  * p2_sync (or the synchronising call itself) reports P2_ERR_DEVICE_TIMEOUT.

@@ -7,24 +7,28 @@
 // contract_mesons_{all,new,}_device (PLEGMA_mesonsAll.cuh:7-95,
 // PLEGMA_mesonsNew.cuh:5-56, PLEGMA_mesons.cuh:10-65).
 //
-// Two instantiations:
+// Two forms:
 //  - plain:  FP64 propagators, FP64 arithmetic, complex-double output;
 //  - split:  FP64 or FP32 propagators multiplied by 2^-E(slice, flavour)
 //            (exact power-of-two scaling, so correlators that fall over ten
 //            decades in t stay inside FP32's range), FP32 arithmetic,
 //            complex-float output, plus max(|Re|,|Im|) per (slice, component)
-//            for the FP16 split of the projection.
+//            for the FP16 split of the tensor-core projection.
+// Each in two instantiations, the Delta with the second nucleon interpolator
+// and the rest; what the kernels fused with the sums over x (contract_site.cuh)
+// take does not come here.
 //
 // Layout and schedule
-//  - a CTA of 256 threads is persistent over tiles of 16 consecutive sites of
-//    one time slice (tile = (tau, x0));
-//  - each tile's 2 x 144 complex per site are copied with cp.async, coalesced
-//    along the site axis of the SoA propagator, into shared memory as
-//    [site][flavour*144 + component] (row padded to 289 complex);
-//  - two stages: tile i+1's copies are in flight while tile i is contracted;
+//  - a CTA is persistent over tiles of consecutive sites of one time slice
+//    (tile = (tau, x0)): plain 128 threads and 8 sites, split 256 and 16;
 //  - half-warp h contracts site h of the tile (site_contract.cuh);
-//  - split form: the tile is converted once into padded FP32 rows (component-
-//    major staging, one buffer), and the 16 x 16 meson outputs go back through
+//  - plain: the 2 x 144 complex of a site are copied with cp.async, coalesced
+//    along the site axis of the SoA propagator, into shared memory as
+//    [site][flavour*144 + component] (row padded to 289 complex), in two stages
+//    (tile i+1's copies are in flight while tile i is contracted); the colour
+//    products of the 16 x 16 mesons leave as 128-byte component rows;
+//  - split: the copies are component-major in one buffer, the tile is converted
+//    once into padded FP32 rows, and the 16 x 16 meson outputs go back through
 //    the sites' rows to a tile-wide flush that writes 128-byte component rows;
 //    when nothing else needs the lanes' Gamma stages (g16_raw) the outputs are
 //    the colour-traced products M themselves and the Gamma sums run after the

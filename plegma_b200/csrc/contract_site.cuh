@@ -28,10 +28,10 @@
 // slice without a rotation converts whole spin blocks; the groups of four
 // blocks that a rotation mixes cost 680 instructions per site against 70, which
 // was 8 % of the mesons' time.
-// Measured on B200 against the position buffer and the sums over x from it:
-// 48^3 x 96 (22 slices), nucleon + 16 x 16 mesons, 7.52 -> 6.46 ms; 24^3 x 48
-// plain 3.78 -> 3.12 ms; 32^3 x 64 batch with both Deltas 20.6 -> 16.7 ms;
-// 64^3 x 128 FP32 with Deltas 22.3 -> 17.2 ms.
+// Measured on B200 against the position buffer and the sums over x from it, 123
+// momenta: nucleon + 16 x 16 mesons, split, 48^3 x 8 slices 2.48 -> 2.24 ms; plain,
+// 24^3 x 24 1.90 -> 1.59 ms; with both Deltas, split, 32^3 x 12 4.36 -> 3.59 ms, 48^3
+// x 8 9.50 -> 7.86 ms.
 #pragma once
 #include "kernels.cuh"
 #include "launch_util.h"

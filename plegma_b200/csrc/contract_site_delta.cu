@@ -19,9 +19,11 @@
 // and after the three pairs the outputs to the output tile and, X, the sums
 // over x.
 // Bound: FMA issue and, in A, the shared-memory loads (18 wavefronts of a
-// block against 36 issue slots of the dots it feeds): split form 1780 clk/site
-// with 3874 warp instructions and 1024 wavefronts; plain form 3361 clk/site,
-// FP64 pipe 47 %.
+// block against 36 issue slots of the dots it feeds): split form 1791 clk/site
+// with 3897 warp instructions and 1024 wavefronts; plain form 3357 clk/site,
+// FP64 pipe 47 %.  At 128 registers the split form with FP64 propagators and
+// seven rows spills 332 bytes a thread, with FP32 propagators 104, the plain form at
+// 255 registers 368 (the outputs o, the row sums and the next tile's nine values live through a flavour pair).
 #include "contract_site.cuh"
 
 namespace p2 {

@@ -15,9 +15,9 @@
 // of the class itself: z(s) = r in T[m][r] exactly for the class role (r,
 // r ^ 1), so that role adds s D to its Q before its slot terms.  The four
 // roles of the class form D among themselves, the others do not wait.
-// Bound, split form: issue with four warps per scheduler, 662 clk/site (52 %
-// of the slots, 1383 warp instructions, 296 shared-memory wavefronts); half of
-// it is A.  Plain form: FP64 latency at 8 warps per SM, 1176 clk/site (FP64
+// Bound, split form: issue with four warps per scheduler, 668 clk/site (54 %
+// of the slots, 1439 warp instructions, 296 shared-memory wavefronts); half of
+// it is A.  Plain form: FP64 latency at 8 warps per SM, 1175 clk/site (FP64
 // pipe 41 %).  The HBM floor is 196 clk/site.
 #include "contract_site.cuh"
 
@@ -230,6 +230,9 @@ cudaError_t go(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s)
   return launch_tiles<R>(k_site_mesons<R, Tin, RT>, a, xt, RT, Mem<R>::kAll, nsm, s);
 }
 
+// Instantiated for three, seven and nine phase rows: five run as seven, which
+// takes no longer (48^3 x 12 slices, split, this kernel's us: three rows 3021, five
+// 3127, seven 3126), one as three.
 template <typename R, typename Tin>
 cudaError_t go_rows(const ContractArgs& a, const double* xt, int nsm, cudaStream_t s) {
   return a.R1 <= 3   ? go<R, Tin, 3>(a, xt, nsm, s)

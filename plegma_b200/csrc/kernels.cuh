@@ -248,7 +248,12 @@ cudaError_t launch_contract_f32(const ContractArgs& a, int fp32_in, int grid, cu
 // Fused with the sums over x (contract_site.cuh), split or plain form: the
 // nucleon and the colour products of the 16 x 16 mesons; the Delta.  xt
 // [Lx][R1] the phase rows.
-constexpr int kRowsMaxPhases = 960;  // Lx x phase rows (4, 8 or 12) of the fused kernels' parameter block
+// Lx x phase rows (4, 8 or 12) of the fused kernels' parameter block: 240, 120 or
+// 80 sites of a row.  The parameters would hold four times as many, and the
+// fusion is still the faster path there (us, fused and not, 32^2 x 8 slices with Lx
+// = 96 and nine rows: nucleon and 16 x 16 mesons split 2187 and 2238, plain 3843 and
+// 4102, with both Deltas 7310 and 8493; Lx = 128, seven rows: 2562 and 2796).
+constexpr int kRowsMaxPhases = 960;
 cudaError_t launch_site_mesons(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,
                                cudaStream_t s);
 cudaError_t launch_site_delta(const ContractArgs& a, const double* xt, int plain, int fp32_in, int nsm,

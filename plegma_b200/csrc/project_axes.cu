@@ -21,16 +21,18 @@
 //
 // Measured on B200, FP64, against the direct sum of project_fp64.cu (which
 // larger lists keep): the plain form at 24^3 x 48 with 288 components and 123
-// momenta 4.17 ms instead of 14.12 ms (the projection was 10.8 ms of it), the
-// transform of a 32-component field there 0.14 ms instead of 2.18 ms.  Error
-// against 64 bits 1.7e-15 instead of 4.0e-15 (fewer terms per sum).
-// Split form, against the tensor-core projection (which larger lists keep):
-// 8^3 x 16 with 288 components 96 us instead of 101, 24^3 x 48 light baryons
-// 4.77 ms instead of 5.34, 64^3 x 128 with K = 480 and 123 momenta 22.3 ms
-// instead of 29.4 (with the Delta); error against 64 bits 2e-7 instead of 1e-6
-// (an FP32 sum over one row at a time, no split of the data into FP16 parts).
-// Without the fused contraction (contract_site.cuh) 48^3 slices gain only 2 %:
-// the position buffer's write and read bound both.
+// momenta 3.13 ms instead of 14.12 ms, with the sums over x inside the
+// contraction (the projection was 10.8 ms of it), the transform of a 32-component
+// field there 0.136 ms instead of 2.18 ms.  Error against 64 bits 1.7e-15
+// instead of 4.0e-15 (fewer terms per sum).
+// Split form, against the tensor-core projection (which larger lists, and
+// short x axes of large lattices, keep): 8^3 x 16 with 288 components 84 us
+// instead of 120, 24^3 x 48 light baryons 4.36 ms instead of 5.34, 64^3 x 128
+// with K = 480 and 257 momenta 17.0 ms instead of 29.1 (both with the Delta's new
+// contraction); error against 64 bits 1.7e-7 instead of 1e-6 (no split of the
+// data into FP16 parts).  Without the fused contraction (contract_site.cuh) 48^3
+// slices take what the tensor cores do (8 of them, nucleon and 16 x 16 mesons
+// 2.48 and 2.49 ms): the position buffer's write and read bound both.
 //
 // Sums over x: FP64 for FP64 input; FP32 input in FP32 over groups of at most
 // kSumGroup sites and in FP64 over these, one row of Lx sites by one thread, so
@@ -497,8 +499,11 @@ namespace p2host {
 // Whether a momentum list takes the axis-by-axis projection, and its tables
 // on the device (kept per transform sign until the list changes).
 // The list qualifies when no axis has more than kAxisMaxRows rows (|n| <= 4,
-// every list up to |n|^2 <= 24): a row costs the sum over x a register pair
-// per thread, and larger lists keep the direct projections.
+// every list up to |n|^2 <= 24).  The line is where the instantiations end, not
+// where the direct projections win: with eleven rows (|n|^2 <= 25, 515 momenta) a
+// build of these kernels took 2.4 ms at 24^3 x 24 slices in FP64, 288 components,
+// where the direct sum takes 28.7, 4.3 ms against 7.1 of the tensor cores at 48^3 x
+// 12, and 0.22 ms against 8.8 (FP64) and 0.71 for a field of 32 components.
 p2_status axes_prepare(p2_ctx* c, const std::vector<int>& moms, int sign, const AxesPlan** out) {
   *out = nullptr;
   AxesPlan& ap = c->axes[sign > 0 ? 1 : 0];

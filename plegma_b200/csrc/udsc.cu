@@ -5,8 +5,9 @@
 // A flavour product (e.g. "uud") has up to 16 datasets (interpolator and
 // projector variants); dataset d of a site is
 //   sum_entries w * sum_{eps eps'} P1[s0 s1][a a'] P2[s2 s3][b b'] P3[s4 s5][c c']
-// over the spin tables of plegma_b200/udsc.py (real weights in single
-// precision like the reference's; the reference spends 108 complex products
+// over the spin tables of plegma_b200/udsc.py (real weights, each rounded to
+// single precision like the reference's, the sums of merged ones in double,
+// in the split form rounded again; the reference spends 108 complex products
 // per entry).  udsc.site_program turns a product's entries into a program:
 // entries that differ by an exchange of equal flavours are merged, every
 // distinct triple of spin blocks is evaluated once for all datasets, as a
@@ -25,10 +26,11 @@
 // projection consumes.
 // Measured on B200 against one instruction stream per lane over the unmerged
 // entries (16 lanes of a site in divergent loops): split form, 32^3 x 16, u and
-// d (28 datasets), 123 momenta 20.6 -> 6.2 ms; plain form, 16^3 x 16, all 200
-// datasets, 33 momenta 33.9 -> 9.4 ms.
+// d (28 datasets), 123 momenta 20.6 -> 3.8 ms; plain form, 16^3 x 16, all 200
+// datasets, 33 momenta 33.9 -> 7.4 ms.
 // Bound: the latency of a warp's chain program word -> block -> products, with
-// 16 (split) or 8 (plain) warps per SM; the FMAs alone would take a quarter.
+// 16 (split) or 8 (plain) warps per SM: 65 % of the issue slots, FMA pipe 40 %
+// (split, 2029 clk/site), 35 % and FP64 pipe 42 % (plain, 3736 clk/site).
 #include <algorithm>
 #include <cstring>
 #include <map>
